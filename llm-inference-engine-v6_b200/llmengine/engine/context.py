@@ -16,24 +16,34 @@ class Workspace:
     """Scratch tensors by tag. A tag's buffer grows to the largest size asked for and is then
     reused by every step (and every layer that uses the tag), so steady-state steps allocate
     nothing and addresses stay fixed for CUDA-graph replays."""
+    MAX_VIEWS = 4096
 
     def __init__(self, device: torch.device):
         self.device = device
         self._buffers: Dict[str, torch.Tensor] = {}
+        self._views: Dict[tuple, torch.Tensor] = {}  # what get() made of the buffers: making a view costs more than a launch
         self.frozen = False  # set while a CUDA graph is being captured or replayed
 
     def get(self, tag: str, shape: Tuple[int, ...], dtype: torch.dtype) -> torch.Tensor:
+        key = (tag, tuple(shape), dtype)
+        view = self._views.get(key)
+        if view is not None:
+            return view
         numel = 1
         for d in shape:
             numel *= int(d)
-        nbytes = numel * torch.empty((), dtype=dtype).element_size()
+        nbytes = numel * dtype.itemsize
         buf = self._buffers.get(tag)
         if buf is None or buf.numel() < nbytes:
             if self.frozen:
                 raise RuntimeError(f"workspace '{tag}' would have to grow while a CUDA graph depends on it")
             buf = torch.empty(max(nbytes, 256), dtype=torch.uint8, device=self.device)
             self._buffers[tag] = buf
-        return buf[:nbytes].view(dtype).view(shape)
+            self._views.clear()  # (views of the smaller buffer would keep it alive)
+        elif len(self._views) >= self.MAX_VIEWS:
+            self._views.clear()  # steps of ever new sizes: a step's worth of views is made again
+        view = self._views[key] = buf[:nbytes].view(dtype).view(shape)
+        return view
 
     def get_zeroed(self, tag: str, shape: Tuple[int, ...], dtype: torch.dtype) -> torch.Tensor:
         """As get, for memory that must read zero the first time: the buffer is cleared when it is

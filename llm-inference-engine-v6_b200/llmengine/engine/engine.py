@@ -85,8 +85,8 @@ class Engine:
         self.buffers: Optional[StepBuffers] = None
         self.sampler = Sampler(self.ops, self.device)
         self._next_private_id = -1
-        # decode-only steps replay CUDA graphs (bfloat16 serving path; the 32-bit path stays eager)
-        self.cuda_graphs = (self.torch_dtype == torch.bfloat16 and self.device.type == "cuda") if cuda_graphs is None else cuda_graphs
+        # decode-only steps replay CUDA graphs
+        self.cuda_graphs = self.device.type == "cuda" if cuda_graphs is None else cuda_graphs
         self.graphs = None
         self._id_bases = 0
         self._ckpt_names: Optional[List[str]] = None

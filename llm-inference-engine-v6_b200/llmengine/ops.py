@@ -57,7 +57,9 @@ def _row_scale_args(rs: Optional["RowScale"]):
 
 
 def _stream():
-    return c_void_p(torch.cuda.current_stream().cuda_stream)
+    """The calling thread's current stream on its current device (as torch.cuda.current_stream().cuda_stream, which makes a stream
+    object each time: 7 us of host time a launch, this 0.3)."""
+    return c_void_p(torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()))
 
 
 def _need(t: torch.Tensor, name: str, dtype=None, rows_contiguous: bool = True) -> None:
@@ -67,6 +69,29 @@ def _need(t: torch.Tensor, name: str, dtype=None, rows_contiguous: bool = True) 
         raise KernelError(f"{name}: expected {dtype}, got {t.dtype}")
     if rows_contiguous and t.dim() >= 1 and t.stride(-1) != 1 and t.shape[-1] != 1:
         raise KernelError(f"{name}: last dimension must be contiguous")
+
+
+# Argument types of the launchers that a prompt step calls over and over: with them ctypes takes plain numbers, which costs a
+# third of wrapping every argument (p pointer, i int, q long long, f float).
+_TYPES = {"p": c_void_p, "i": c_int, "q": c_longlong, "f": c_float}
+_SIGNATURES = {
+    "core": {
+        "llm_rmsnorm": "ppiqpppiiifiip",
+        "llm_rope_kv_write": "pqipiqpppipppp" + "iiiii" + "piffp",
+        "llm_gemm_simt": "pppiiiqqqiip",
+        "llm_silu_mul": "ppiiiiiffp",
+    },
+    "tensorcore": {
+        "llm_gemm_tc": "pppiiiqqqiiiqip",
+        "llm_gemm_tc_swiglu": "pppiiiqqqiffp",
+        "llm_paged_attention_tc": "pqppqppppipqiiiiiifiipp",
+    },
+}
+
+
+def _at(t: Optional[torch.Tensor]):
+    """A tensor's address for a launcher with argument types."""
+    return None if t is None else t.data_ptr()
 
 
 class CudaOps:
@@ -107,6 +132,7 @@ class CudaOps:
         # round alike.
         self.meet_products = False
         self._few_cache = {}
+        self._known = {}  # what the libraries answered about a geometry (their answers depend on nothing else)
         self._err_host: Optional[torch.Tensor] = None  # pinned word that queue_error_check copies the kernels' error code into
 
     # ------------------------------------------------------------------ loading
@@ -118,6 +144,8 @@ class CudaOps:
             path = _build.kernel_library_path(name)
             lib = ctypes.CDLL(path)
             lib.llm_last_error.restype = ctypes.c_char_p
+            for fn, kinds in _SIGNATURES[name].items():
+                getattr(lib, fn).argtypes = [_TYPES[k] for k in kinds]
             if name == "tensorcore":
                 lib.llm_attention_mma_scratch_floats.restype = ctypes.c_longlong
                 lib.llm_latent_attention_scratch_floats.restype = ctypes.c_longlong
@@ -152,6 +180,15 @@ class CudaOps:
         default), or write them to global memory where the last CTA to arrive adds them (off; more
         than eight splits always end that way, cluster by cluster)."""
         self.lib("tensorcore").llm_attention_decode_cluster_merge(c_int(1 if on else 0))
+
+    def _answer(self, lib, fn: str, nq: int, nkv: int, hd: int, page: int, ld_q: int, ld_out: int) -> bool:
+        """What a library says about an attention geometry, asked once."""
+        key = (fn, nq, nkv, hd, page, ld_q, ld_out)
+        hit = self._known.get(key)
+        if hit is None:
+            hit = bool(getattr(lib, fn)(c_int(nq), c_int(nkv), c_int(hd), c_int(page), c_longlong(ld_q), c_longlong(ld_out)))
+            self._known[key] = hit
+        return hit
 
     def _check(self, rc: int, lib) -> None:
         self.launches += 1
@@ -218,10 +255,8 @@ class CudaOps:
         if rows is not None:
             _need(rows, "rmsnorm.rows", torch.int32)
             write_back = False
-        self._check(lib.llm_rmsnorm(_ptr(h), _ptr(delta), c_int(n_part), c_longlong(pstride), _ptr(weight),
-                                    _ptr(rows), _ptr(out), c_int(dtype_code(out.dtype)), c_int(n_out), c_int(dim),
-                                    c_float(eps), c_int(1 if (write_back and delta is not None) else 0),
-                                    c_int(1 if center else 0), _stream()), lib)
+        self._check(lib.llm_rmsnorm(_at(h), _at(delta), n_part, pstride, _at(weight), _at(rows), _at(out), dtype_code(out.dtype), n_out, dim,
+                                    eps, 1 if (write_back and delta is not None) else 0, 1 if center else 0, _stream()), lib)
         return out
 
     def residual_add(self, h: torch.Tensor, delta: torch.Tensor, n_rows: Optional[int] = None) -> torch.Tensor:
@@ -246,11 +281,13 @@ class CudaOps:
     # g <- min(g, limit), u <- clamp(u, -limit, limit), g * sigmoid(slope * g) * (u + 1)
     ACTIVATIONS = {"silu": 0, "gelu_tanh": 1, "clamped_swish": 2}
 
+    _PLAIN_ACT = {name: (c_int(code), c_float(0.0), c_float(1.0)) for name, code in ACTIVATIONS.items()}
+
     @classmethod
     def _act_args(cls, act):
         if isinstance(act, tuple):
             return c_int(cls.ACTIVATIONS[act[0]]), c_float(act[1]), c_float(act[2])
-        return c_int(cls.ACTIVATIONS[act]), c_float(0.0), c_float(1.0)
+        return cls._PLAIN_ACT[act]
 
     def silu_mul(self, gate_up: torch.Tensor, out: torch.Tensor, block: int = 0, act: str = "silu") -> torch.Tensor:
         """gate_up [n, 2*ff] -> out [n, ff] = act(gate)*up. block 0: gate columns first, then up;
@@ -259,8 +296,7 @@ class CudaOps:
         lib = self.lib()
         n, ff = out.shape
         assert gate_up.is_contiguous() and out.is_contiguous() and gate_up.shape == (n, 2 * ff)
-        self._check(lib.llm_silu_mul(_ptr(gate_up), _ptr(out), c_int(dtype_code(out.dtype)), c_int(n), c_int(ff),
-                                     c_int(block), *self._act_args(act), _stream()), lib)
+        self._check(lib.llm_silu_mul(_at(gate_up), _at(out), dtype_code(out.dtype), n, ff, block, *self._act_args(act), _stream()), lib)
         return out
 
     EPILOGUE_ACTIVATIONS = ("silu", "gelu_tanh", "clamped_swish")  # what the gate|up product applies in its own epilogue (gemm_swiglu)
@@ -278,9 +314,8 @@ class CudaOps:
         if m > self.SWAP_MAX_TOKENS and (act[0] if isinstance(act, tuple) else act) in self.EPILOGUE_ACTIVATIONS and self._tc_usable(a, w_blocked):
             assert row_scale is None, "a row scale is applied where partial sums are consumed (few tokens)"
             lib = self.lib("tensorcore")
-            self._check(lib.llm_gemm_tc_swiglu(_ptr(a), _ptr(w_blocked), _ptr(out), c_int(m), c_int(ff), c_int(k),
-                                               c_longlong(a.stride(0)), c_longlong(w_blocked.stride(0)),
-                                               c_longlong(out.stride(0)), *self._act_args(act), _stream()), lib)
+            self._check(lib.llm_gemm_tc_swiglu(_at(a), _at(w_blocked), _at(out), m, ff, k, a.stride(0), w_blocked.stride(0), out.stride(0),
+                                               *self._act_args(act), _stream()), lib)
             return out
         assert ws is not None, "gemm_swiglu needs a workspace when it cannot fuse"
         if m <= self.SWAP_MAX_TOKENS:
@@ -302,9 +337,12 @@ class CudaOps:
         """bfloat16 operands that the tensor-core kernel takes (16-byte aligned rows of K % 8 == 0)."""
         if a.dtype != torch.bfloat16 or not self.tensor_cores:
             return False
-        lib = self.lib("tensorcore")
-        return bool(lib.llm_gemm_tc_supported(_ptr(a), _ptr(w), c_int(a.shape[0]), c_int(w.shape[0]), c_int(a.shape[1]),
-                                              c_longlong(a.stride(0)), c_longlong(w.stride(0))))
+        if "tma" not in self._known:  # (whether the driver encodes tensor maps: asked of the library once, about operands it takes)
+            self._known["tma"] = bool(self.lib("tensorcore").llm_gemm_tc_supported(c_void_p(16), c_void_p(16), c_int(1), c_int(1), c_int(8),
+                                                                                   c_longlong(8), c_longlong(8)))
+        m, k = a.shape
+        return (self._known["tma"] and m > 0 and k > 0 and w.shape[0] > 0 and
+                (k | a.stride(0) | w.stride(0)) % 8 == 0 and (a.data_ptr() | w.data_ptr()) % 16 == 0)
 
     def _splits_for(self, M: int, N: int, K: int) -> int:
         tiles, k_tiles = (N + 127) // 128, (K + 63) // 64
@@ -312,7 +350,8 @@ class CudaOps:
             return 1
         target = self.SPLIT_TARGET_CTAS if M <= 32 else self.SPLIT_TARGET_CTAS // 2
         want = min(max(1, -(-target // tiles)), max(1, k_tiles // 2))
-        return int(self.lib("tensorcore").llm_gemm_tc_splits(c_int(K), c_int(want)))
+        per_split = -(-k_tiles // want)  # (as llm_gemm_tc_splits)
+        return -(-k_tiles // per_split)
 
     SWAP_MAX_TOKENS = 64  # up to here weights fill the accumulator lanes and tokens the columns
 
@@ -322,9 +361,8 @@ class CudaOps:
         swap = 1 if M <= self.SWAP_MAX_TOKENS else 0
         lib = self.lib("tensorcore")
         ldo = out.stride(-2)
-        self._check(lib.llm_gemm_tc(_ptr(a), _ptr(w), _ptr(out), c_int(M), c_int(N), c_int(K), c_longlong(a.stride(0)),
-                                    c_longlong(w.stride(0)), c_longlong(ldo), c_int(dtype_code(out.dtype)), c_int(swap),
-                                    c_int(splits), c_longlong(split_stride), c_int(3 if swap else 8), _stream()), lib)
+        self._check(lib.llm_gemm_tc(_at(a), _at(w), _at(out), M, N, K, a.stride(0), w.stride(0), ldo, dtype_code(out.dtype), swap, splits,
+                                    split_stride, 3 if swap else 8, _stream()), lib)
 
     def gemm(self, a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, ws=None) -> torch.Tensor:
         """out[m,n] = sum_k a[m,k]*w[n,k]; float32 accumulation; a and w of one dtype; out float32
@@ -346,9 +384,8 @@ class CudaOps:
                 self.reduce_partials(parts, out)
             return out
         lib = self.lib()
-        self._check(lib.llm_gemm_simt(_ptr(a), _ptr(w), _ptr(out), c_int(M), c_int(N), c_int(K),
-                                      c_longlong(a.stride(0)), c_longlong(w.stride(0)), c_longlong(out.stride(0)),
-                                      c_int(dtype_code(a.dtype)), c_int(dtype_code(out.dtype)), _stream()), lib)
+        self._check(lib.llm_gemm_simt(_at(a), _at(w), _at(out), M, N, K, a.stride(0), w.stride(0), out.stride(0), dtype_code(a.dtype),
+                                      dtype_code(out.dtype), _stream()), lib)
         return out
 
     def gemm_heads(self, a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, gate: Optional[torch.Tensor] = None,
@@ -639,11 +676,9 @@ class CudaOps:
             _need(parts, "rope.parts", torch.float32)
             assert parts.is_contiguous() and parts.dim() == 3 and parts.shape[2] == qkv.shape[1] and parts.shape[1] >= n_tokens
             n_parts, pstride = parts.shape[0], parts.stride(0)
-        self._check(lib.llm_rope_kv_write(_ptr(qkv), c_longlong(qkv.stride(0)), c_int(dtype_code(qkv.dtype)),
-                                          _ptr(parts), c_int(n_parts), c_longlong(pstride), _ptr(positions), _ptr(token_seq), _ptr(block_table),
-                                          c_int(block_table.shape[1]), _ptr(cos), _ptr(sin), _ptr(kcache),
-                                          _ptr(vcache), c_int(n_tokens), c_int(nq), c_int(nkv), c_int(hd),
-                                          c_int(page_size), *_row_scale_args(row_scale), _stream()), lib)
+        self._check(lib.llm_rope_kv_write(_at(qkv), qkv.stride(0), dtype_code(qkv.dtype), _at(parts), n_parts, pstride, _at(positions),
+                                          _at(token_seq), _at(block_table), block_table.shape[1], _at(cos), _at(sin), _at(kcache), _at(vcache),
+                                          n_tokens, nq, nkv, hd, page_size, *_row_scale_args(row_scale), _stream()), lib)
 
     # decoding: the key range is cut at absolute multiples of `split_keys` (a multiple of 64); see _split_policy
     ATTENTION_TARGET_CTAS = 592
@@ -739,16 +774,13 @@ class CudaOps:
             lib = self.lib("tensorcore")
             if (self.tcgen05_attention and batch.max_new_tokens >= self.TC_ATTENTION_MIN_TOKENS and
                     block_table.shape[1] <= self.TC_ATTENTION_MAX_BLOCKS and
-                    lib.llm_attention_tc_supported(c_int(nq), c_int(nkv), c_int(hd), c_int(page), c_longlong(q.stride(0)),
-                                                   c_longlong(out.stride(0)))):
+                    self._answer(lib, "llm_attention_tc_supported", nq, nkv, hd, page, q.stride(0), out.stride(0))):
                 # prompt portions: tcgen05 kernel (128 rows per CTA, scores and output in tensor memory)
                 work = batch.ws.get_zeroed("attention.work_counters", (2,), torch.int32)  # left at zero by the kernel
                 self._check(lib.llm_paged_attention_tc(
-                    _ptr(q), c_longlong(q.stride(0)), _ptr(kcache), _ptr(vcache), c_longlong(kcache.shape[0]),
-                    _ptr(batch.seq_start), _ptr(batch.seq_ntok), _ptr(batch.seq_qoff), _ptr(block_table),
-                    c_int(block_table.shape[1]), _ptr(out), c_longlong(out.stride(0)), c_int(batch.n_seqs),
-                    c_int(batch.max_new_tokens), c_int(nq), c_int(nkv), c_int(hd), c_int(page), c_float(scale), c_int(window),
-                    c_int(q.shape[0]), _ptr(work), _stream()), lib)
+                    _at(q), q.stride(0), _at(kcache), _at(vcache), kcache.shape[0], _at(batch.seq_start), _at(batch.seq_ntok), _at(batch.seq_qoff),
+                    _at(block_table), block_table.shape[1], _at(out), out.stride(0), batch.n_seqs, batch.max_new_tokens, nq, nkv, hd, page,
+                    scale, window, q.shape[0], _at(work), _stream()), lib)
                 return out
             decode_only = batch.max_new_tokens == 1 and batch.n_tokens == batch.n_seqs
             use_tma = decode_only and self.tma_decode_attention and lib.llm_attention_decode_supported(
