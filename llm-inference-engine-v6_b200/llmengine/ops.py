@@ -146,6 +146,8 @@ class CudaOps:
             lib.llm_last_error.restype = ctypes.c_char_p
             for fn, kinds in _SIGNATURES[name].items():
                 getattr(lib, fn).argtypes = [_TYPES[k] for k in kinds]
+            if name == "core":
+                lib.llm_paged_attention_simt_scratch.restype = ctypes.c_longlong
             if name == "tensorcore":
                 lib.llm_attention_mma_scratch_floats.restype = ctypes.c_longlong
                 lib.llm_latent_attention_scratch_floats.restype = ctypes.c_longlong
@@ -808,11 +810,17 @@ class CudaOps:
                     self.launches += 1  # the kernel that merges the splits
                 return out
         lib = self.lib()
+        floats = int(lib.llm_paged_attention_simt_scratch(c_int(batch.n_seqs), c_int(n_tokens), c_int(batch.max_new_tokens), c_int(batch.max_seq_len),
+                                                          c_int(nq), c_int(nkv), c_int(hd)))
+        scratch = batch.ws.get("attention.segments", (floats,), torch.float32) if floats else None
         self._check(lib.llm_paged_attention_simt(_ptr(q), c_longlong(q.stride(0)), _ptr(kcache), _ptr(vcache),
-                                                 c_int(dtype_code(q.dtype)), _ptr(batch.positions), _ptr(batch.token_seq),
-                                                 _ptr(block_table), c_int(block_table.shape[1]), _ptr(out),
-                                                 c_longlong(out.stride(0)), c_int(n_tokens), c_int(nq), c_int(nkv),
-                                                 c_int(hd), c_int(page), c_float(scale), c_int(window), _stream()), lib)
+                                                 c_int(dtype_code(q.dtype)), _ptr(batch.positions), _ptr(batch.seq_start), _ptr(batch.seq_ntok),
+                                                 _ptr(batch.seq_qoff), _ptr(block_table), c_int(block_table.shape[1]), _ptr(out),
+                                                 c_longlong(out.stride(0)), c_int(batch.n_seqs), c_int(n_tokens), c_int(batch.max_new_tokens),
+                                                 c_int(batch.max_seq_len), c_int(nq), c_int(nkv), c_int(hd), c_int(page), c_float(scale),
+                                                 c_int(window), _ptr(scratch), _stream()), lib)
+        if floats:
+            self.launches += 1  # the kernel that merges the segments
         return out
 
     def attention_kernels(self, nq: int, nkv: int, hd: int, page: int):

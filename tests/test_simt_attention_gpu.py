@@ -1,0 +1,56 @@
+"""Float32 attention on CUDA cores: segments with a CTA each against one CTA that walks over all of them."""
+import math
+
+import pytest
+import torch
+from test_kernels_gpu import DEV, Batch, _attention_ref, _paged_setup
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ops():
+    from llmengine.ops import get_ops
+    return get_ops()
+
+
+@pytest.mark.parametrize("nq,nkv,hd,page,window", [(8, 2, 64, 16, 0), (6, 1, 32, 4, 0), (9, 1, 20, 16, 0), (4, 4, 128, 16, 130), (2, 1, 256, 8, 0),
+                                                   (12, 1, 18, 4, 127)])
+@pytest.mark.parametrize("length", [1, 64, 127, 128, 129, 256, 257, 400])
+def test_a_token_alone_and_in_a_prompt(ops, nq, nkv, hd, page, window, length):
+    """The last token alone (few rows: a CTA a segment), at the end of a portion, and at the end of the whole prompt beside many others
+    (more rows, and so many CTAs that each walks over all segments): bit-equal, and near float64."""
+    others = 40
+    kc, vc, table, dense = _paged_setup(torch.float32, nkv, hd, page, [length] * others, others * ((length + page - 1) // page) + 2, seed=length)
+    scale = 1.0 / math.sqrt(hd)
+    q = torch.randn(others, length, nq * hd, generator=torch.Generator().manual_seed(7)).to(DEV)
+
+    def run(entries):
+        b = Batch(entries)
+        rows = torch.cat([q[i, s:s + n] for i, (s, n) in enumerate(entries)])
+        out = torch.empty_like(rows)
+        ops.paged_attention(rows, kc, vc, b, table[:len(entries)].contiguous(), out, nq, nkv, hd, scale, window)
+        return out, b
+
+    alone, b = run([(length - 1, 1)])
+    portion, _ = run([(length - min(length, 5), min(length, 5))])
+    whole, _ = run([(0, length)] * others)
+    assert torch.equal(portion[-1], alone[0])
+    assert torch.equal(whole[length - 1], alone[0])
+    K, V = dense[0]
+    ref = _attention_ref(q[0, -1].view(nq, hd).cpu().double(), K.double(), V.double(), length - 1, nq, nkv, hd, scale, window)
+    torch.testing.assert_close(alone[0].cpu(), ref.float(), rtol=2e-5, atol=2e-5)
+
+
+def test_values_behind_a_token_do_not_reach_it(ops):
+    """A later token of the same portion whose value row is NaN leaves earlier tokens' results as they are."""
+    kc, vc, table, _ = _paged_setup(torch.float32, 2, 64, 16, [100], 9, seed=3)
+    q = torch.randn(100, 8 * 64, generator=torch.Generator().manual_seed(8)).to(DEV)
+    outs = []
+    for poison in (False, True):
+        if poison:
+            vc[table[0, 4], :, 6] = float("nan")  # position 70
+        out = torch.empty_like(q)
+        ops.paged_attention(q, kc, vc, Batch([(0, 100)]), table, out, 8, 2, 64, 0.125)
+        outs.append(out)
+    assert torch.equal(outs[0][:70], outs[1][:70]) and bool(outs[1][70:].isnan().all())
