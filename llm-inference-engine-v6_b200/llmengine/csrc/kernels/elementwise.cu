@@ -381,11 +381,43 @@ __global__ void reduce_partials_kernel(const float* __restrict__ partials, int n
   out[i] = from_f32<T>(x);
 }
 
+// The same for rows of whole groups of four on 16 bytes: a thread adds four neighbours, their parts' loads in flight together.
+template <typename T>
+__global__ void reduce_partials_vec_kernel(const float* __restrict__ partials, int n_partials, size_t stride, T* __restrict__ out, size_t groups) {
+  dep_launch();
+  dep_wait();
+  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= groups) return;
+  float4 x = reinterpret_cast<const float4*>(partials)[i];
+#pragma unroll 4
+  for (int p = 1; p < n_partials; ++p) {
+    const float4 y = reinterpret_cast<const float4*>(partials + (size_t)p * stride)[i];
+    x.x += y.x; x.y += y.y; x.z += y.z; x.w += y.w;
+  }
+  if constexpr (sizeof(T) == 4) {
+    reinterpret_cast<float4*>(out)[i] = x;
+  } else {
+    __nv_bfloat162 lo = __floats2bfloat162_rn(x.x, x.y), hi = __floats2bfloat162_rn(x.z, x.w);
+    reinterpret_cast<uint2*>(out)[i] = make_uint2(*reinterpret_cast<uint32_t*>(&lo), *reinterpret_cast<uint32_t*>(&hi));
+  }
+}
+
 extern "C" int llm_reduce_partials(const float* partials, int n_partials, long long stride, void* out, int out_dtype,
                                    long long total, cudaStream_t stream) {
   if (total == 0) return LLM_OK;
   LLM_REQUIRE(total > 0 && n_partials >= 1, "reduce_partials: bad sizes");
   const int blocks = ceil_div(total, 256);
+  // four a thread where everything lies on 16 bytes (6 parts of 77 x 3,072: 2.5 us)
+  if (total % 4 == 0 && stride % 4 == 0 && (reinterpret_cast<uintptr_t>(partials) & 15u) == 0 && (reinterpret_cast<uintptr_t>(out) & 15u) == 0 &&
+      (out_dtype == LLM_F32 || out_dtype == LLM_BF16)) {
+    const int vblocks = ceil_div(total / 4, 256);
+    if (out_dtype == LLM_F32)
+      launch_kernel(reduce_partials_vec_kernel<float>, vblocks, 256, 0, stream, partials, n_partials, (size_t)stride, (float*)out, (size_t)total / 4);
+    else
+      launch_kernel(reduce_partials_vec_kernel<bf16>, vblocks, 256, 0, stream, partials, n_partials, (size_t)stride, (bf16*)out, (size_t)total / 4);
+    LLM_CHECK_LAUNCH("reduce_partials");
+    return LLM_OK;
+  }
   if (out_dtype == LLM_F32)
     launch_kernel(reduce_partials_kernel<float>, blocks, 256, 0, stream, partials, n_partials, (size_t)stride, (float*)out, (size_t)total);
   else if (out_dtype == LLM_BF16)
@@ -430,6 +462,46 @@ __global__ void silu_mul_partials_kernel(const float* __restrict__ partials, int
   out[i] = from_f32<T>(gated_value(g, u, act, p0, p1));
 }
 
+// The same, four columns a thread (and a row of blocks a token): the loads of four parts of both halves in flight.
+template <typename T>
+__global__ void silu_mul_partials_vec_kernel(const float* __restrict__ partials, int n_partials, size_t stride, T* __restrict__ out, int ff,
+                                             int block, const RowScale rs, int act, float a0, float a1) {
+  dep_launch();
+  dep_wait();
+  const int c = 4 * (blockIdx.x * blockDim.x + threadIdx.x);
+  if (c >= ff) return;
+  const size_t r = blockIdx.y;
+  size_t gc, uc;
+  gate_up_columns(c, ff, block, &gc, &uc);
+  const float* gp = partials + r * 2 * ff + gc;
+  const float* up = partials + r * 2 * ff + uc;
+  float4 g = make_float4(0.f, 0.f, 0.f, 0.f), u = g;
+  for (int p0 = 0; p0 < n_partials; p0 += 4) {
+    float4 gv[4], uv[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const bool in = p0 + k < n_partials;
+      gv[k] = in ? *reinterpret_cast<const float4*>(gp + (size_t)(p0 + k) * stride) : make_float4(0.f, 0.f, 0.f, 0.f);
+      uv[k] = in ? *reinterpret_cast<const float4*>(up + (size_t)(p0 + k) * stride) : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      g.x += gv[k].x; g.y += gv[k].y; g.z += gv[k].z; g.w += gv[k].w;
+      u.x += uv[k].x; u.y += uv[k].y; u.z += uv[k].z; u.w += uv[k].w;
+    }
+  }
+  const float sc = row_scale(rs, r);
+  const float v0 = gated_value(g.x * sc, u.x * sc, act, a0, a1), v1 = gated_value(g.y * sc, u.y * sc, act, a0, a1);
+  const float v2 = gated_value(g.z * sc, u.z * sc, act, a0, a1), v3 = gated_value(g.w * sc, u.w * sc, act, a0, a1);
+  T* o = out + r * ff + c;
+  if constexpr (sizeof(T) == 4) {
+    *reinterpret_cast<float4*>(o) = make_float4(v0, v1, v2, v3);
+  } else {
+    __nv_bfloat162 lo = __floats2bfloat162_rn(v0, v1), hi = __floats2bfloat162_rn(v2, v3);
+    *reinterpret_cast<uint2*>(o) = make_uint2(*reinterpret_cast<uint32_t*>(&lo), *reinterpret_cast<uint32_t*>(&hi));
+  }
+}
+
 extern "C" int llm_silu_mul_partials(const float* partials, int n_partials, long long stride, void* out, int out_dtype,
                                      int n_rows, int ff, int block, const float* sumsq, int n_sumsq, float inv_dim, float eps,
                                      int act, float p0, float p1, cudaStream_t stream) {
@@ -440,6 +512,19 @@ extern "C" int llm_silu_mul_partials(const float* partials, int n_partials, long
   LLM_REQUIRE(block >= 0 && (block == 0 || ff % block == 0), "silu_mul_partials: column block %d does not divide %d", block, ff);
   const size_t total = (size_t)n_rows * ff;
   const int blocks = ceil_div((long long)total, 256);
+  // four columns a thread where a group of four lies in one block and on 16 bytes, and there are threads enough that way (64 tokens
+  // of 8,192 columns; with 8 tokens a column a thread is the faster one, 1.6 against 1.9 us)
+  if (total >= 148 * 1024 && ff % 4 == 0 && block % 4 == 0 && stride % 4 == 0 && n_rows <= 65535 && (reinterpret_cast<uintptr_t>(partials) & 15u) == 0 &&
+      (reinterpret_cast<uintptr_t>(out) & 15u) == 0 && (out_dtype == LLM_F32 || out_dtype == LLM_BF16)) {
+    const int threads = ff >= 4096 ? 128 : 64;
+    const dim3 grid(ceil_div(ff / 4, threads), n_rows);
+    if (out_dtype == LLM_F32)
+      launch_kernel(silu_mul_partials_vec_kernel<float>, grid, threads, 0, stream, partials, n_partials, (size_t)stride, (float*)out, ff, block, rs, act, p0, p1);
+    else
+      launch_kernel(silu_mul_partials_vec_kernel<bf16>, grid, threads, 0, stream, partials, n_partials, (size_t)stride, (bf16*)out, ff, block, rs, act, p0, p1);
+    LLM_CHECK_LAUNCH("silu_mul_partials");
+    return LLM_OK;
+  }
   if (out_dtype == LLM_F32)
     launch_kernel(silu_mul_partials_kernel<float>, blocks, 256, 0, stream, partials, n_partials, (size_t)stride, (float*)out, ff, total, block, rs, act, p0, p1);
   else if (out_dtype == LLM_BF16)

@@ -315,10 +315,10 @@ __global__ void __launch_bounds__(128)
         float gv[16], uv[16];
         tmem_load16(tmem_base + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0, gv);
         tmem_load16(tmem_base + ((uint32_t)(warp * 32) << 16) + (uint32_t)(c0 + BN / 2), uv);
-#pragma unroll
-        for (int i = 0; i < 16; ++i) gv[i] = gate_up<SWIGLU>(gv[i], uv[i], epi.act_p0, epi.act_p1);
         const int col0 = b_row0 / 2 + c0;  // column of the activation matrix [tokens, RB / 2]
-        if (ra < RA && col0 < RB / 2) {
+        if (ra < RA && col0 < RB / 2) {  // (rows beyond the tokens are zeros, whose division takes its slow way: 40 us for 25 with 77 tokens)
+#pragma unroll
+          for (int i = 0; i < 16; ++i) gv[i] = gate_up<SWIGLU>(gv[i], uv[i], epi.act_p0, epi.act_p1);
           TO* dst = o + (size_t)ra * ldo + col0;
           store_row16<TO>(dst, gv, min(16, RB / 2 - col0), (reinterpret_cast<uintptr_t>(dst) & 15u) == 0);
         }
@@ -567,10 +567,10 @@ __global__ void __launch_bounds__(PERSIST_THREADS)
           float gv[16], uv[16];
           tmem_load16(acc + (uint32_t)c0, gv);
           tmem_load16(acc + (uint32_t)(c0 + BN / 2), uv);
-#pragma unroll
-          for (int i = 0; i < 16; ++i) gv[i] = gate_up<SWIGLU>(gv[i], uv[i], act_p0, act_p1);
           const int col0 = b_row0 / 2 + c0;  // column of the activation matrix [tokens, RB / 2]
-          if (ra < RA && col0 < RB / 2) {
+          if (ra < RA && col0 < RB / 2) {  // (nothing to compute for rows beyond the tokens)
+#pragma unroll
+            for (int i = 0; i < 16; ++i) gv[i] = gate_up<SWIGLU>(gv[i], uv[i], act_p0, act_p1);
             TO* dst = out + (size_t)ra * ldo + col0;
             store_row16<TO>(dst, gv, min(16, RB / 2 - col0), (reinterpret_cast<uintptr_t>(dst) & 15u) == 0);
           }
@@ -996,8 +996,8 @@ extern "C" int llm_gemm_tc_supported(const void* a, const void* w, int M, int N,
 
 // out[m, n] = sum_k a[m, k] * w[n, k], a [M, K] and w [N, K] bfloat16.
 // swap = 0: tiles of 128 tokens; out dtype bf16 or f32; splits must be 1.
-// swap = 1: M <= 256 tokens; weights fill the accumulator lanes; with splits > 1, out is float32
-//           [splits, M, ldo] partials (split_stride elements apart) to be added by the consumer.
+// swap = 1: weights fill the accumulator lanes, tokens the columns (tiles of up to 256); with splits > 1, out is
+//           float32 [splits, M, ldo] partials (split_stride elements apart) to be added by the consumer.
 static int gemm_tc_impl(const void* a, const void* w, void* out, int M, int N, int K, long long lda, long long ldw,
                         long long ldo, int out_dtype, int swap, int splits, long long split_stride, int stages,
                         cudaStream_t stream, int add_into) {
@@ -1036,7 +1036,7 @@ static int gemm_tc_impl(const void* a, const void* w, void* out, int M, int N, i
     else LLM_TC_CASE(16);
 #undef LLM_TC_CASE
   } else {
-    LLM_REQUIRE(M <= 256, "gemm_tc: the swapped form takes at most 256 tokens, got %d", M);
+    LLM_REQUIRE((M + 255) / 256 <= 65535, "gemm_tc: M=%d too large", M);
     const int bn = M > 128 ? 256 : (M > 64 ? 128 : (M > 32 ? 64 : (M > 16 ? 32 : 16)));
     LLM_REQUIRE(tensor_map_for(w, N, K, ldw, BM, &ma) && tensor_map_for(a, M, K, lda, bn, &mb), "gemm_tc: cuTensorMapEncodeTiled failed");
 #define LLM_TC_CASE(BN_)                                                                                                        \

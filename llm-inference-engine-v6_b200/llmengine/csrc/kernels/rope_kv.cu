@@ -105,11 +105,34 @@ __global__ void __launch_bounds__(128)
   }
 }
 
-// bfloat16 rows without partial sums, 16 bytes at a time: an item is 8 neighbouring rotation pairs
+// Eight neighbouring sums over the parts of a product, in index order.
+__device__ __forceinline__ void sum8(const float* p, int n_parts, size_t stride, float* v) {
+  float4 lo = reinterpret_cast<const float4*>(p)[0], hi = reinterpret_cast<const float4*>(p)[1];
+#pragma unroll 3
+  for (int k = 1; k < n_parts; ++k) {
+    const float4 a = reinterpret_cast<const float4*>(p + k * stride)[0], b = reinterpret_cast<const float4*>(p + k * stride)[1];
+    lo.x += a.x; lo.y += a.y; lo.z += a.z; lo.w += a.w;
+    hi.x += b.x; hi.y += b.y; hi.z += b.z; hi.w += b.w;
+  }
+  v[0] = lo.x; v[1] = lo.y; v[2] = lo.z; v[3] = lo.w;
+  v[4] = hi.x; v[5] = hi.y; v[6] = hi.z; v[7] = hi.w;
+}
+__device__ __forceinline__ uint4 pack8(const float* v) {
+  union { uint4 u; __nv_bfloat162 h[4]; } r;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) r.h[j] = __floats2bfloat162_rn(v[2 * j], v[2 * j + 1]);
+  return r.u;
+}
+
+// bfloat16 rows, 16 bytes at a time: an item is 8 neighbouring rotation pairs
 // of a q or k head (8 elements of the first half with their 8 partners of the second half), or 8
-// neighbouring elements of v. Needs head_dim % 16 == 0 and 16-byte aligned rows.
+// neighbouring elements of v. Needs head_dim % 16 == 0 and 16-byte aligned rows. PARTS: the values are sums over a
+// product's float32 parts (256 tokens x 5,120 columns in 3 parts take 10.5 us a pair a thread; a mixed step of that
+// size is 980 us with it, 971 with this form).
+template <bool PARTS>
 __global__ void __launch_bounds__(128)
-    rope_kv_write_vec_kernel(bf16* __restrict__ qkv, long long ld_qkv, const int* __restrict__ positions,
+    rope_kv_write_vec_kernel(bf16* __restrict__ qkv, long long ld_qkv, const float* __restrict__ parts, int n_parts, size_t part_stride,
+                             const int* __restrict__ positions,
                              const int* __restrict__ token_seq, const int* __restrict__ block_table, int max_blocks,
                              const float* __restrict__ cos_t, const float* __restrict__ sin_t, bf16* __restrict__ kcache,
                              bf16* __restrict__ vcache, int nq, int nkv, int hd, int page_size) {
@@ -127,18 +150,37 @@ __global__ void __launch_bounds__(128)
     const int page = block_table[(size_t)token_seq[t] * max_blocks + pos / page_size];
     cache_base = ((size_t)page * nkv * page_size + (pos % page_size)) * hd;
   }
-  const size_t head_stride = (size_t)page_size * hd;
+  const size_t head_stride = (size_t)page_size * hd, width = (size_t)(nq + 2 * nkv) * hd;
   if (item >= n_rot) {  // 8 elements of v, copied as they are
     const int e = (item - n_rot) * 8, vh = e / hd, vi = e - vh * hd;
-    *reinterpret_cast<uint4*>(vcache + cache_base + (size_t)vh * head_stride + vi) =
-        *reinterpret_cast<const uint4*>(row + (size_t)(nq + nkv) * hd + e);
+    uint4* dst = reinterpret_cast<uint4*>(vcache + cache_base + (size_t)vh * head_stride + vi);
+    if (PARTS) {
+      float v[8];
+      sum8(parts + (size_t)t * width + (size_t)(nq + nkv) * hd + e, n_parts, part_stride, v);
+      *dst = pack8(v);
+    } else {
+      *dst = *reinterpret_cast<const uint4*>(row + (size_t)(nq + nkv) * hd + e);
+    }
     return;
   }
   const int head = item / groups, i0 = (item - head * groups) * 8;
   bf16* x = row + (size_t)head * hd;
   union { uint4 u; __nv_bfloat162 h[4]; } a, b;
-  a.u = *reinterpret_cast<const uint4*>(x + i0);
-  b.u = *reinterpret_cast<const uint4*>(x + i0 + half);
+  float fa[8], fb[8];
+  if (PARTS) {
+    const float* from = parts + (size_t)t * width + (size_t)head * hd + i0;
+    sum8(from, n_parts, part_stride, fa);
+    sum8(from + half, n_parts, part_stride, fb);
+  } else {
+    a.u = *reinterpret_cast<const uint4*>(x + i0);
+    b.u = *reinterpret_cast<const uint4*>(x + i0 + half);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const float2 av = __bfloat1622float2(a.h[j]), bv = __bfloat1622float2(b.h[j]);
+      fa[2 * j] = av.x; fa[2 * j + 1] = av.y;
+      fb[2 * j] = bv.x; fb[2 * j + 1] = bv.y;
+    }
+  }
   if (cos_t) {
     const float4* c4 = reinterpret_cast<const float4*>(cos_t + (size_t)pos * half + i0);
     const float4* s4 = reinterpret_cast<const float4*>(sin_t + (size_t)pos * half + i0);
@@ -148,14 +190,14 @@ __global__ void __launch_bounds__(128)
     *reinterpret_cast<float4*>(sn) = s4[0];
     *reinterpret_cast<float4*>(sn + 4) = s4[1];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const float2 av = __bfloat1622float2(a.h[j]), bv = __bfloat1622float2(b.h[j]);
-      const float ra0 = av.x * c[2 * j] - bv.x * sn[2 * j], rb0 = bv.x * c[2 * j] + av.x * sn[2 * j];
-      const float ra1 = av.y * c[2 * j + 1] - bv.y * sn[2 * j + 1], rb1 = bv.y * c[2 * j + 1] + av.y * sn[2 * j + 1];
-      a.h[j] = __floats2bfloat162_rn(ra0, ra1);
-      b.h[j] = __floats2bfloat162_rn(rb0, rb1);
+    for (int j = 0; j < 8; ++j) {
+      const float av = fa[j], bv = fb[j];
+      fa[j] = av * c[j] - bv * sn[j];
+      fb[j] = bv * c[j] + av * sn[j];
     }
   }
+  a.u = pack8(fa);
+  b.u = pack8(fb);
   bf16* dst = (head < nq || !kcache) ? x : kcache + cache_base + (size_t)(head - nq) * head_stride;
   *reinterpret_cast<uint4*>(dst + i0) = a.u;
   *reinterpret_cast<uint4*>(dst + i0 + half) = b.u;
@@ -179,12 +221,15 @@ extern "C" int llm_rope_kv_write(void* qkv, long long ld_qkv, int dtype, const f
   LLM_REQUIRE(!parts || (n_parts >= 1 && kcache), "rope_kv_write: partial sums need n_parts >= 1 and a cache to write to");
   const int threads = 128;
   auto al = [](const void* ptr) { return (reinterpret_cast<uintptr_t>(ptr) & 15u) == 0; };
-  if (dtype == LLM_BF16 && !parts && hd % 16 == 0 && ld_qkv % 8 == 0 && al(qkv) && al(kcache) && al(vcache) && al(cos_t) && al(sin_t)) {
+  // 16 bytes at a time; with parts from a prompt's tokens on (few tokens: a pair a thread puts more threads on them), and no row scale
+  if (dtype == LLM_BF16 && hd % 16 == 0 && ld_qkv % 8 == 0 && al(qkv) && al(kcache) && al(vcache) && al(cos_t) && al(sin_t) &&
+      (!parts || (n_tokens > 64 && !sumsq && al(parts) && part_stride % 4 == 0))) {
     const int vitems = (nq + nkv) * (hd / 16) + (vcache ? nkv * (hd / 8) : 0);
     const dim3 vgrid(n_tokens, ceil_div(vitems, threads));
     LLM_REQUIRE(vgrid.y <= 65535, "rope_kv_write: too many heads");
-    launch_kernel(rope_kv_write_vec_kernel, vgrid, threads, 0, stream, (bf16*)qkv, ld_qkv, positions, token_seq, block_table,
-                  max_blocks, cos_t, sin_t, (bf16*)kcache, (bf16*)vcache, nq, nkv, hd, page_size);
+    launch_kernel(parts ? rope_kv_write_vec_kernel<true> : rope_kv_write_vec_kernel<false>, vgrid, threads, 0, stream, (bf16*)qkv, ld_qkv, parts,
+                  n_parts, (size_t)part_stride, positions, token_seq, block_table, max_blocks, cos_t, sin_t, (bf16*)kcache, (bf16*)vcache, nq, nkv,
+                  hd, page_size);
     LLM_CHECK_LAUNCH("rope_kv_write");
     return LLM_OK;
   }

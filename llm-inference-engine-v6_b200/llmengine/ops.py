@@ -132,6 +132,7 @@ class CudaOps:
         # round alike.
         self.meet_products = False
         self._few_cache = {}
+        self._forms = {}  # _form's answers
         self._known = {}  # what the libraries answered about a geometry (their answers depend on nothing else)
         self._err_host: Optional[torch.Tensor] = None  # pinned word that queue_error_check copies the kernels' error code into
 
@@ -346,25 +347,59 @@ class CudaOps:
         return (self._known["tma"] and m > 0 and k > 0 and w.shape[0] > 0 and
                 (k | a.stride(0) | w.stride(0)) % 8 == 0 and (a.data_ptr() | w.data_ptr()) % 16 == 0)
 
-    def _splits_for(self, M: int, N: int, K: int) -> int:
-        tiles, k_tiles = (N + 127) // 128, (K + 63) // 64
-        if M > self.SWAP_MAX_TOKENS:
-            return 1
-        target = self.SPLIT_TARGET_CTAS if M <= 32 else self.SPLIT_TARGET_CTAS // 2
-        want = min(max(1, -(-target // tiles)), max(1, k_tiles // 2))
-        per_split = -(-k_tiles // want)  # (as llm_gemm_tc_splits)
-        return -(-k_tiles // per_split)
+    SWAP_MAX_TOKENS = 64  # up to here weights fill the accumulator lanes and tokens the columns, several CTAs an SM
 
-    SWAP_MAX_TOKENS = 64  # up to here weights fill the accumulator lanes and tokens the columns
+    def _form(self, M: int, N: int, K: int, may_split: bool, reduced: bool = False):
+        """-> (weights on the accumulator lanes, K splits, stages of a CTA's ring) of a product. may_split: its consumer adds parts, or
+        a kernel behind the product does (reduced), which has its own launch and traffic.
+        Beyond SWAP_MAX_TOKENS a product is bound by how fast a CTA takes its operands in, 0.5 us for a k-block of 128 x 256, so what
+        counts is the k-blocks a CTA has one after the other: tiles of 128 outputs x 128 or 256 tokens with K cut until one CTA an SM
+        has work, as long as writing and reading the parts (6 TB/s, out of L2) costs less than it saves. Measured with 77 / 256 tokens
+        (tiles of tokens -> this, in us): 2,048 outputs of 2,048 inputs 18.0 / 20.0 -> 6.9 / 11.9, of 8,192 inputs 52.6 / 54.6 ->
+        11.1 / 16.8, 3,072 of 2,048 20.2 / 22.9 -> 7.9 / 12.3. Up to 128 tokens the tile is half as wide and there are twice as many
+        CTAs even without a cut (16,384 of 2,048: 22.0 -> 16.7)."""
+        key = (M, N, K, may_split, reduced)
+        hit = self._forms.get(key)
+        if hit is None:
+            if len(self._forms) >= 4096:
+                self._forms.clear()
+            hit = self._forms[key] = self._choose_form(*key)
+        return hit
 
-    def _gemm_tc(self, a, w, out, splits: int = 1, split_stride: int = 0) -> None:
+    def _choose_form(self, M: int, N: int, K: int, may_split: bool, reduced: bool):
+        tiles, k_tiles = -(-N // 128), -(-K // 64)
+        if M <= self.SWAP_MAX_TOKENS:
+            if not may_split:
+                return 1, 1, 3
+            target = self.SPLIT_TARGET_CTAS if M <= 32 else self.SPLIT_TARGET_CTAS // 2
+            want = min(max(1, -(-target // tiles)), max(1, k_tiles // 2))
+            per_split = -(-k_tiles // want)  # (as llm_gemm_tc_splits)
+            return 1, -(-k_tiles // per_split), 3
+        wide = M > 128
+        tiles *= -(-M // 256) if wide else 1
+        best, best_us = (0 if wide else 1, 1, 8), (0.5 if wide else 0.4) * k_tiles
+        if may_split and tiles <= self.ONE_WAVE // 2:
+            for want in range(2, min(self.ONE_WAVE // tiles, k_tiles // 2) + 1):
+                per_split = -(-k_tiles // want)
+                splits = -(-k_tiles // per_split)
+                us = (0.5 if wide else 0.4) * per_split + splits * M * N * 8 / 6e6 + (3.0 if reduced else 0.0)
+                if us < best_us:
+                    best, best_us = (1, splits, 8), us
+        return best
+
+    ONE_WAVE = 148  # SMs: one CTA with the long ring each
+
+    def gemm_cuts(self, a: torch.Tensor, w: torch.Tensor) -> bool:
+        """Whether gemm_partials cuts K for these operands, so that a consumer that adds the parts saves the kernel that would."""
+        return self._tc_usable(a, w) and self._form(a.shape[0], w.shape[0], a.shape[1], True)[1] > 1
+
+    def _gemm_tc(self, a, w, out, form, split_stride: int = 0) -> None:
         M, K = a.shape
         N = w.shape[0]
-        swap = 1 if M <= self.SWAP_MAX_TOKENS else 0
+        swap, splits, stages = form
         lib = self.lib("tensorcore")
-        ldo = out.stride(-2)
-        self._check(lib.llm_gemm_tc(_at(a), _at(w), _at(out), M, N, K, a.stride(0), w.stride(0), ldo, dtype_code(out.dtype), swap, splits,
-                                    split_stride, 3 if swap else 8, _stream()), lib)
+        self._check(lib.llm_gemm_tc(_at(a), _at(w), _at(out), M, N, K, a.stride(0), w.stride(0), out.stride(-2), dtype_code(out.dtype), swap, splits,
+                                    split_stride, stages, _stream()), lib)
 
     def gemm(self, a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, ws=None) -> torch.Tensor:
         """out[m,n] = sum_k a[m,k]*w[n,k]; float32 accumulation; a and w of one dtype; out float32
@@ -377,12 +412,13 @@ class CudaOps:
         N = w.shape[0]
         assert w.shape[1] == K and out.shape == (M, N)
         if self._tc_usable(a, w):
-            splits = self._splits_for(M, N, K) if (ws is not None and out.is_contiguous()) else 1
+            form = self._form(M, N, K, ws is not None and out.is_contiguous(), True)
+            splits = form[1]
             if splits == 1:
-                self._gemm_tc(a, w, out)
+                self._gemm_tc(a, w, out, form)
             else:
                 parts = ws.get("gemm.parts", (splits, M, N), torch.float32)
-                self._gemm_tc(a, w, parts, splits, M * N)
+                self._gemm_tc(a, w, parts, form, M * N)
                 self.reduce_partials(parts, out)
             return out
         lib = self.lib()
@@ -423,9 +459,9 @@ class CudaOps:
         N = w.shape[0]
         assert w.shape[1] == K
         if self._tc_usable(a, w):
-            splits = self._splits_for(M, N, K)
-            parts = ws.get(tag, (splits, M, N), torch.float32)
-            self._gemm_tc(a, w, parts, splits, M * N)
+            form = self._form(M, N, K, True)
+            parts = ws.get(tag, (form[1], M, N), torch.float32)
+            self._gemm_tc(a, w, parts, form, M * N)
             return parts
         parts = ws.get(tag, (1, M, N), torch.float32)
         self.gemm(a, w, parts[0])
@@ -468,7 +504,7 @@ class CudaOps:
         N = w.shape[0]
         assert self.can_meet(a, w) and w.shape[1] == K and h.shape[0] >= M and h.shape[1] == N
         tiles = (N + 127) // 128
-        splits = self._splits_for(M, N, K)
+        splits = self._form(M, N, K, True)[1]
         parts = ws.get(tag, (splits, M, N), torch.float32)
         counters = ws.get_zeroed("gemm.meet_counters", (tiles,), torch.int32)
         n_sumsq = 0

@@ -95,7 +95,7 @@ class PagedAttention(Mixer):
                 row_scale, x, few = x.row_scale(ops), x.prescaled, False
             elif not (few and cache.writes and self.position.takes_partial_sums):
                 x = x.dense(ctx)
-        if n <= 64 and cache.writes and self.position.takes_partial_sums:
+        if cache.writes and self.position.takes_partial_sums and (n <= 64 or (hasattr(ops, "gemm_cuts") and ops.gemm_cuts(x[:n], self.w_qkv))):
             # few tokens: the product comes as float32 sums (in parts, unless the K pieces were added
             # inside the product), finished by the position kernel or by the attention kernel
             if few:

@@ -1,0 +1,104 @@
+"""Products of more than 64 tokens with K cut, the vector forms of the kernels that add their parts, and steps of such sizes."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+@pytest.fixture(scope="module")
+def ops():
+    from llmengine.ops import get_ops
+    return get_ops()
+
+
+def rnd(*shape, seed, dt=torch.bfloat16):
+    return torch.randn(*shape, generator=torch.Generator().manual_seed(seed)).to(dt).to(DEV)
+
+
+@pytest.mark.parametrize("m", [65, 127, 128, 129, 200, 256, 257, 300, 513])
+@pytest.mark.parametrize("n,k", [(128, 512), (130, 1032), (2048, 2048), (72, 4096), (3072, 264)])
+def test_cut_products_of_more_than_64_tokens(ops, m, n, k):
+    """Against float64: bfloat16 products are exact in float32, sums of k of them in any order are off by at most k roundings of 2^-24
+    of the absolute products (the tensor cores truncate: twice that); a bfloat16 result rounds once more."""
+    from llmengine.engine.context import Workspace
+    ws = Workspace(torch.device(DEV))
+    a, w = rnd(m, k, seed=1), rnd(n, k, seed=2)
+    exact, bound = a.double() @ w.double().T, 2 * k * 2.0 ** -24 * (a.double().abs() @ w.double().abs().T)
+    parts = ops.gemm_partials(a, w, ws, "t")
+    assert bool(((parts.double().sum(0) - exact).abs() <= bound).all())
+    for dt in (torch.float32, torch.bfloat16):
+        out = torch.full((m + 1, n), 3.0, dtype=dt, device=DEV)
+        for space in (ws, None):
+            ops.gemm(a, w, out[:m], space)
+            off = (out[:m].double() - exact).abs()
+            assert bool((off <= bound + (0 if dt == torch.float32 else 2.0 ** -8) * exact.abs()).all())
+            assert bool((out[m] == 3.0).all())
+
+
+def test_what_is_cut():
+    """The rule itself: few tokens as before, more tokens one wave of CTAs at most, and no cut where nobody adds parts."""
+    from llmengine.ops import CudaOps
+    ops = CudaOps.__new__(CudaOps)
+    ops._forms = {}
+    for m in (1, 8, 33, 64):
+        assert ops._form(m, 2048, 2048, False) == (1, 1, 3) and ops._form(m, 2048, 2048, True)[1] > 1
+    for m in (65, 128, 129, 256, 500, 1000, 2048):
+        for n in (64, 2048, 3072, 16384):
+            for k in (64, 128, 2048, 8192):
+                for may in (False, True):
+                    swap, splits, stages = ops._form(m, n, k, may)
+                    tiles = -(-n // 128) * -(-m // (128 if m <= 128 else 256))
+                    assert splits == 1 or (may and swap == 1 and tiles * splits <= 148 and -(-k // 64) >= 2 * (splits - 1))
+                    assert swap == (1 if m <= 128 or splits > 1 else 0) and stages == 8
+
+
+@pytest.mark.parametrize("parts,rows,width", [(1, 1, 4), (3, 5, 12), (9, 77, 130), (5, 65, 2048), (2, 3, 7)])
+def test_reduce_partials_forms_agree(ops, parts, rows, width):
+    p = rnd(parts, rows, width, seed=3, dt=torch.float32)
+    want = p[0].clone()
+    for i in range(1, parts):
+        want += p[i]
+    for dt in (torch.float32, torch.bfloat16):
+        out = torch.empty(rows, width, dtype=dt, device=DEV)
+        ops.reduce_partials(p, out)
+        assert torch.equal(out, want.to(dt))
+
+
+@pytest.mark.parametrize("act", ["silu", "gelu_tanh", ("clamped_swish", 1.5, 1.7)])
+@pytest.mark.parametrize("parts,rows,ff,block", [(1, 3, 128, 128), (3, 70, 384, 128), (5, 9, 176, 0), (4, 6, 100, 0), (2, 5, 6, 0)])
+def test_silu_mul_partials_forms_agree(ops, parts, rows, ff, block, act):
+    """A group of four columns at a time gives the bits of one column at a time (the same parts on an address that is no multiple of 16)."""
+    p = rnd(parts, rows, 2 * ff, seed=4, dt=torch.float32)
+    odd = torch.empty(p.numel() + 1, device=DEV)[1:].view(p.shape)
+    odd.copy_(p)
+    for dt in (torch.float32, torch.bfloat16):
+        a, b = torch.empty(rows, ff, dtype=dt, device=DEV), torch.empty(rows, ff, dtype=dt, device=DEV)
+        ops.silu_mul_partials(p, a, block=block, act=act)
+        ops.silu_mul_partials(odd, b, block=block, act=act)
+        assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("parts,n,nq,nkv,hd,page", [(1, 65, 4, 2, 64, 16), (3, 77, 6, 1, 128, 4), (6, 200, 2, 2, 16, 8)])
+@pytest.mark.parametrize("rotate", [True, False])
+def test_rotation_of_parts_forms_agree(ops, parts, n, nq, nkv, hd, page, rotate):
+    """Eight pairs at a time give the bits of a pair at a time (parts on an address that is no multiple of 16 take that way): the same
+    sums in the same order, and both forms' products and differences round once or are fused alike within a bfloat16 step."""
+    width = (nq + 2 * nkv) * hd
+    p = rnd(parts, n, width, seed=7, dt=torch.float32)
+    odd = torch.empty(p.numel() + 1, device=DEV)[1:].view(p.shape)
+    odd.copy_(p)
+    pos = torch.arange(5, 5 + n, dtype=torch.int32, device=DEV)
+    seq = torch.zeros(n, dtype=torch.int32, device=DEV)
+    blocks = -(-(n + 5) // page)
+    table = torch.randperm(blocks, generator=torch.Generator().manual_seed(1)).to(torch.int32).view(1, -1).to(DEV)
+    angle = torch.arange(n + 5)[:, None] * torch.logspace(0, -3, hd // 2)[None]
+    cos, sin = (angle.cos().to(DEV), angle.sin().to(DEV)) if rotate else (None, None)
+    got = []
+    for src in (p, odd):
+        qkv = torch.zeros(n, width, dtype=torch.bfloat16, device=DEV)
+        k, v = (torch.zeros(blocks + 1, nkv, page, hd, dtype=torch.bfloat16, device=DEV) for _ in range(2))
+        ops.rope_kv_write(qkv, pos, seq, table, cos, sin, k, v, n, nq, nkv, hd, parts=src)
+        got.append((qkv[:, :nq * hd], k, v))
+    for a, b in zip(*got):
+        torch.testing.assert_close(a, b, rtol=2.0 ** -7, atol=1e-6)
