@@ -1109,6 +1109,48 @@ class CudaOps:
             return int(self.lib("tensorcore").llm_routed_product_mma_rows(c_int(int(per_expert))))
         return int(self.lib().llm_routed_product_rows())
 
+    # The per-expert products run on tcgen05 from this many rows an expert (on average), although its tiles are 128 rows and an
+    # expert's last one is part empty. 4 of 16 experts of 2,048 x 2,048, both products with the gathering: 2,048 tokens (512 rows an
+    # expert) 188 us, as mma.sync tiles 588 us; 64 rows an expert 76 against 181 us, 32 rows 71 against 104 us. With fewer rows the
+    # products are bound by the experts' matrices, which tiles of 16 rows stream as well.
+    ROUTED_SORTED_ROWS = 32
+
+    def routed_sorted(self, dtype: torch.dtype, inner=(), per_expert: float = 0.0) -> bool:
+        """Whether a step's per-expert products run on rows gathered into the tiles' order (routed_gather, routed_product_sorted),
+        with tiles of ROUTED_SORTED_TILE rows."""
+        return (dtype == torch.bfloat16 and self.tensor_cores and self.routed_tensor_cores and per_expert >= self.ROUTED_SORTED_ROWS and
+                all(k % 8 == 0 for k in inner))
+
+    ROUTED_SORTED_TILE = 128
+
+    def routed_gather(self, a: torch.Tensor, a_div: int, tile_expert: torch.Tensor, tile_rows: torch.Tensor, out: torch.Tensor) -> torch.Tensor:
+        """out[i, :] = a[pair // a_div, :] for the pair at place i of the tiles (places of padding are left as they are)."""
+        _need(a, "routed_gather.a", torch.bfloat16); _need(out, "routed_gather.out", torch.bfloat16)
+        assert out.is_contiguous() and out.shape == (tile_rows.numel(), a.shape[1]) and tile_rows.shape[1] == self.ROUTED_SORTED_TILE
+        lib = self.lib("tensorcore")
+        self._check(lib.llm_routed_gather(_ptr(a), c_longlong(a.stride(0)), c_int(a_div), c_int(a.shape[1]), _ptr(tile_expert), _ptr(tile_rows),
+                                          c_int(tile_expert.numel()), _ptr(out), _stream()), lib)
+        return out
+
+    def routed_product_sorted(self, rows: torch.Tensor, w: torch.Tensor, tile_expert: torch.Tensor, tile_rows: torch.Tensor, out: torch.Tensor,
+                              epilogue: str, share: Optional[torch.Tensor] = None, act="silu") -> torch.Tensor:
+        """As routed_product for rows that lie in the tiles' order (bfloat16, tiles of ROUTED_SORTED_TILE rows). "share" writes float32 at the
+        pairs' own rows of out, the other epilogues bfloat16 in the tiles' order."""
+        _need(rows, "routed_product.rows", torch.bfloat16); _need(w, "routed_product.w", torch.bfloat16); _need(out, "routed_product.out")
+        E, N, K = w.shape
+        pairs = epilogue in ("silu_pairs", "gated_pairs")
+        assert w.is_contiguous() and rows.is_contiguous() and rows.shape == (tile_rows.numel(), K) and tile_rows.shape[1] == self.ROUTED_SORTED_TILE
+        assert out.shape[1] == (N // 2 if pairs else N) and out.dtype == (torch.float32 if epilogue == "share" else torch.bfloat16)
+        assert epilogue == "share" or out.shape[0] == rows.shape[0]
+        if share is not None:
+            _need(share, "routed_product.share", torch.float32)
+        lib = self.lib("tensorcore")
+        self._check(lib.llm_routed_product_tc(_ptr(rows), _ptr(w), c_int(E), c_int(N), c_int(K), _ptr(tile_expert), _ptr(tile_rows),
+                                              c_int(tile_expert.numel()), _ptr(out), c_longlong(out.stride(0)),
+                                              c_int(self.ROUTED_EPILOGUES[epilogue]), _ptr(share),
+                                              *self._act_args(act if epilogue == "gated_pairs" else "silu"), _stream()), lib)
+        return out
+
     def routed_group(self, idx: torch.Tensor, experts: int, tile: int, ws, tag: str, real_experts: Optional[int] = None):
         """Sorts the step's (token, choice) pairs by expert into tiles of `tile` rows -> (tile_expert [tiles] with -1 for
         unused tiles, tile_rows [tiles, tile] with -1 for padding); a pair is token * top + choice. Pairs of experts from

@@ -20,6 +20,26 @@ from .registry import build_part, part_class, register_part
 from .spec import GroupRoutedMLPSpec, RoutedMLPSpec, TensorNeed
 
 
+def expert_products(ops, ctx, x, idx, s, outputs, experts, w_up, w_down, epilogue, act_of, on_input, on_output):
+    """Every (token, choice) pair's row of its expert's two products, float32 [n * top, hidden] (rows of choices from `experts` on are
+    left as they are). Prompt-sized steps copy the rows into the experts' order once and run on them; smaller ones gather the rows
+    as they read them."""
+    n, dt, rows = ctx.n_tokens, x.dtype, ctx.n_tokens * s.top
+    real = {} if experts == outputs else {"real_experts": experts}
+    y = ctx.ws.get("routed.y", (rows, s.hidden), torch.float32)
+    if hasattr(ops, "routed_sorted") and ops.routed_sorted(dt, (s.hidden, s.intermediate), rows / s.experts):
+        tile_expert, tile_rows = ops.routed_group(idx, outputs, ops.ROUTED_SORTED_TILE, ctx.ws, "routed", **real)
+        xs = ops.routed_gather(x, s.top, tile_expert, tile_rows, ctx.ws.get("routed.rows", (tile_rows.numel(), s.hidden), dt))
+        act = ctx.ws.get("routed.act", (tile_rows.numel(), s.intermediate), dt)
+        ops.routed_product_sorted(xs, w_up, tile_expert, tile_rows, act, epilogue, share=on_input, **act_of)
+        return ops.routed_product_sorted(act, w_down, tile_expert, tile_rows, y, "share", share=on_output)
+    tile = ops.routed_tile_rows(n, dt, (s.hidden, s.intermediate), rows / s.experts)
+    tile_expert, tile_rows = ops.routed_group(idx, outputs, tile, ctx.ws, "routed", **real)
+    act = ctx.ws.get("routed.act", (rows, s.intermediate), dt)
+    ops.routed_product(x, s.top, w_up, tile_expert, tile_rows, act, epilogue, **({"share": on_input} if on_input is not None else {}), **act_of)
+    return ops.routed_product(act, 1, w_down, tile_expert, tile_rows, y, "share", share=on_output)
+
+
 class RoutedMLP(FeedForward):
     def __init__(self, spec: RoutedMLPSpec, env):
         super().__init__(spec, env)
@@ -62,12 +82,7 @@ class RoutedMLP(FeedForward):
         idx = ctx.ws.get("routed.idx", (n, s.top), torch.int32)
         share = ctx.ws.get("routed.share", (n, s.top), torch.float32)
         ops.route(x, self.router, self.bias, s.top, idx, share)
-        tile = ops.routed_tile_rows(n, dt, (s.hidden, s.intermediate), n * s.top / s.experts)
-        tile_expert, tile_rows = ops.routed_group(idx, s.experts, tile, ctx.ws, "routed")
-        act = ctx.ws.get("routed.act", (n * s.top, s.intermediate), dt)
-        ops.routed_product(x, s.top, self.w_up, tile_expert, tile_rows, act, "gelu")
-        y = ctx.ws.get("routed.y", (n * s.top, s.hidden), torch.float32)
-        ops.routed_product(act, 1, self.w_down, tile_expert, tile_rows, y, "share", share=share.view(-1))
+        y = expert_products(ops, ctx, x, idx, s, s.experts, s.experts, self.w_up, self.w_down, "gelu", {}, None, share.view(-1))
         out = ctx.ws.get("routed.delta", (n, s.hidden), torch.float32)
         return ops.routed_combine(y, out, s.top)
 
@@ -177,21 +192,10 @@ class GroupRoutedMLP(FeedForward):
         if s.shared_gate:
             gate = extra["gate_out"] = ctx.ws.get("routed.shared_gate", (n,), torch.float32)
         ops.route_grouped(x, self.router, self.correction, s.top, s.groups, s.keep_groups, s.norm_eps, idx, share, **extra)
-        tile = ops.routed_tile_rows(n, dt, (s.hidden, s.intermediate), n * s.top / s.experts)
-        if s.identity:
-            tile_expert, tile_rows = ops.routed_group(idx, self.outputs, tile, ctx.ws, "routed", real_experts=s.experts)
-        else:
-            tile_expert, tile_rows = ops.routed_group(idx, s.experts, tile, ctx.ws, "routed")
-        act = ctx.ws.get("routed.act", (n * s.top, s.intermediate), dt)
         on_input, on_output = (share.view(-1), None) if s.weigh == "input" else (None, share.view(-1))
-        if not self.gated:
-            ops.routed_product(x, s.top, self.w_up, tile_expert, tile_rows, act, "relu_squared", share=on_input)
-        elif s.activation == "silu":
-            ops.routed_product(x, s.top, self.w_up, tile_expert, tile_rows, act, "silu_pairs")
-        else:
-            ops.routed_product(x, s.top, self.w_up, tile_expert, tile_rows, act, "gated_pairs", act=self.act)
-        y = ctx.ws.get("routed.y", (n * s.top, s.hidden), torch.float32)
-        ops.routed_product(act, 1, self.w_down, tile_expert, tile_rows, y, "share", share=on_output)
+        epilogue = "relu_squared" if not self.gated else "silu_pairs" if s.activation == "silu" else "gated_pairs"
+        act_of = {"act": self.act} if epilogue == "gated_pairs" else {}
+        y = expert_products(ops, ctx, x, idx, s, self.outputs, s.experts, self.w_up, self.w_down, epilogue, act_of, on_input, on_output)
         if s.top == 1 and not s.identity and self.shared is None:
             return y  # one expert a token: its row, written at the token's own index, is the sum
         identity = (idx, share, s.experts, x) if s.identity else None
