@@ -45,6 +45,21 @@ struct AttLayout {
   static constexpr int Q_BYTES = ROWS * HD * 2, KV_BYTES = KEYS * HD * 2;  // KV_BYTES: one of K or V of a tile
   static constexpr int S_COL = 0, P_COL = KEYS, O_COL = KEYS + KEYS / 2;   // tensor-memory columns: S f32, P bf16 pairs, O f32
   static_assert(O_COL + HD <= TMEM_COLS_ATT, "the accumulators do not fit the allocation");
+  static constexpr int K_BYTES = KV_BYTES, V_BYTES = KV_BYTES, VBLK = DBLK, TMEM_COLS = TMEM_COLS_ATT, CTAS = 2;
+  static constexpr bool DENSE = false;
+};
+
+// The persistent kernel over keys and values that lie in dense rows instead of pages, every query head with its own: the expanded
+// form of latent attention. A head's key is KB blocks of 64 numbers of its own and one block that all heads share (the rotated
+// part, zeros behind it), its value VB blocks. 128 keys a tile and one CTA an SM: queries, two stages of keys and values are 208 KB
+// at 128 + 64 / 128 numbers.
+template <int KB, int VB_>
+struct DenseLayout {
+  static constexpr int DBLK = KB + 1, VBLK = VB_, KEYS = 128;
+  static constexpr int Q_BYTES = ROWS * DBLK * 128, K_BYTES = KEYS * DBLK * 128, V_BYTES = KEYS * VBLK * 128;
+  static constexpr int S_COL = 0, P_COL = KEYS, O_COL = KEYS + KEYS / 2, TMEM_COLS = 512, CTAS = 1;
+  static_assert(O_COL + VBLK * 64 <= TMEM_COLS, "the accumulators do not fit the allocation");
+  static constexpr bool DENSE = true;
 };
 
 struct AttnTcParams {
@@ -54,6 +69,8 @@ struct AttnTcParams {
   float scale;
   bf16* out; long long ld_out;
   int* error_out;
+  int q_width, rows_per_seq, shared_col;  // dense rows: the numbers of a query head, rows a request takes, the shared block's column
+  float* out32;                           // and the output
 };
 
 __device__ __forceinline__ void tmem_load32(uint32_t taddr, float* v) {
@@ -501,9 +518,8 @@ __host__ __device__ inline int persistent_tq_cap(int g) { return (ROWS / g) / 8 
 // (which sees the most keys) to its first, then those of request 1, and so on. seq_first[s] is the
 // number of query tiles of the requests before s (seq_first[n_seqs]: of all), so that requests with a
 // single token beside a long prompt portion add one item a kv head each and no empty ones.
-template <int HD>
+template <int KEYS>
 __device__ __forceinline__ void att_item(const AttnTcParams& p, int it, int n_seqs, const int* seq_first, AttItem* out) {
-  constexpr int KEYS = AttLayout<HD>::KEYS;
   const int g = p.nq / p.nkv, tq_cap = persistent_tq_cap(g);
   const int kvh = it % p.nkv, j = it / p.nkv;
   int lo_s = 0, hi_s = n_seqs;  // the request whose tiles hold j: seq_first[lo_s] <= j < seq_first[lo_s + 1]
@@ -529,19 +545,20 @@ enum : int { ERR_ATT_ITEM = 14 };
 
 constexpr int ATT_PERSISTENT_THREADS = 192;  // warps 0-3: softmax; warp 4: one thread issues the products; warp 5: work items and copies
 
-template <int HD>
-__global__ void __launch_bounds__(ATT_PERSISTENT_THREADS, 2)
+template <class L>
+__global__ void __launch_bounds__(ATT_PERSISTENT_THREADS, L::CTAS)
     paged_attention_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
-                                         const __grid_constant__ CUtensorMap map_v, const AttnTcParams p, int n_seqs,
+                                         const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_shared,
+                                         const AttnTcParams p, int n_seqs,
                                          int* __restrict__ work) {  // work[0]: next item, work[1]: CTAs that are done
-  using L = AttLayout<HD>;
-  constexpr int KEYS = L::KEYS, DBLK = L::DBLK, Q_BYTES = L::Q_BYTES, KV_BYTES = L::KV_BYTES;
+  constexpr int KEYS = L::KEYS, DBLK = L::DBLK, VBLK = L::VBLK, Q_BYTES = L::Q_BYTES, K_BYTES = L::K_BYTES, V_BYTES = L::V_BYTES;
+  constexpr bool DENSE = L::DENSE;
   constexpr int S_COL = L::S_COL, P_COL = L::P_COL, O_COL = L::O_COL;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
   uint8_t* q_s = smem;             // [DBLK blocks][128 rows][128 B], 128-byte swizzle
   uint8_t* kv_s = smem + Q_BYTES;  // [2 stages][K | V], each [DBLK blocks][KEYS rows][128 B]
-  uint64_t* full_k = reinterpret_cast<uint64_t*>(kv_s + 4 * KV_BYTES);  // [2] the keys of a tile have landed in the stage
+  uint64_t* full_k = reinterpret_cast<uint64_t*>(kv_s + 2 * (K_BYTES + V_BYTES));  // [2] the keys of a tile have landed in the stage
   uint64_t* full_v = full_k + 2;   // [2] the values
   uint64_t* empty_k = full_v + 2;  // [2] the scores that read the stage's keys are done
   uint64_t* empty_v = empty_k + 2; // [2] the product that read the stage's values is done
@@ -561,7 +578,7 @@ __global__ void __launch_bounds__(ATT_PERSISTENT_THREADS, 2)
   dep_launch();
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int g = p.nq / p.nkv, tq_cap = persistent_tq_cap(g);
-  const int pages_per_tile = KEYS / p.page_size;
+  const int pages_per_tile = DENSE ? 0 : KEYS / p.page_size;
 
   if (tid == 0) {
     for (int b = 0; b < 2; ++b) {
@@ -582,7 +599,7 @@ __global__ void __launch_bounds__(ATT_PERSISTENT_THREADS, 2)
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 0) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(TMEM_COLS_ATT) : "memory");
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(L::TMEM_COLS) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
   // rows of the query tile that no copy writes (128 is no multiple of every group size) read as zeros
@@ -632,7 +649,7 @@ __global__ void __launch_bounds__(ATT_PERSISTENT_THREADS, 2)
         AttItem item;
         item.n_tiles = 0;
         const int it = atomicAdd(&work[0], 1);
-        if (it < n_items) att_item<HD>(p, it, n_seqs, seq_first, &item);
+        if (it < n_items) att_item<KEYS>(p, it, n_seqs, seq_first, &item);
         ring[slot] = item;
         n = item.n_tiles;
         __threadfence_block();
@@ -651,6 +668,7 @@ __global__ void __launch_bounds__(ATT_PERSISTENT_THREADS, 2)
     // The first cache row of this lane's page of key tile c, through the block table; asked for a key
     // tile ahead of its use.
     auto page_row = [&](const Cur& c) -> int {
+      if (DENSE) return c.n == 0 ? 0 : ring[c.slot].seq * p.rows_per_seq + (ring[c.slot].kt_first + c.i) * KEYS;
       if (c.n == 0 || lane >= pages_per_tile) return 0;
       const AttItem& item = ring[c.slot];
       const int idx = ((item.kt_first + c.i) * KEYS) / p.page_size + lane;
@@ -658,12 +676,18 @@ __global__ void __launch_bounds__(ATT_PERSISTENT_THREADS, 2)
       if (page < 0) page = p.null_page;  // not held (beyond the newest key, or given back behind a window): finite values, probabilities of zero
       return (page * p.nkv + item.kvh) * p.page_size;
     };
-    auto issue_part = [&](int row, int gt, bool values) {  // keys or values of key tile gt of the stream -> stage gt % 2
-      uint8_t* dst = kv_s + (size_t)(gt & 1) * 2 * KV_BYTES + (values ? KV_BYTES : 0);
+    auto issue_part = [&](int row, int gt, bool values, int kvh) {  // keys or values of key tile gt of the stream -> stage gt % 2
+      uint8_t* dst = kv_s + (size_t)(gt & 1) * (K_BYTES + V_BYTES) + (values ? K_BYTES : 0);
       uint64_t* bar = values ? &full_v[gt & 1] : &full_k[gt & 1];
-      if (lane == 0) mbar_expect_tx(bar, (uint32_t)KV_BYTES);
+      if (lane == 0) mbar_expect_tx(bar, (uint32_t)(values ? V_BYTES : K_BYTES));
       __syncwarp();
-      if (lane < pages_per_tile) {
+      if constexpr (DENSE) {
+        if (lane < (values ? VBLK : DBLK)) {  // a lane a block of 64 numbers; the last of a key is the shared one
+          const bool shared = !values && lane == DBLK - 1;
+          const int x = shared ? p.shared_col : (kvh * (values ? VBLK : DBLK - 1) + lane) * 64;
+          tma_load_2d(dst + lane * (KEYS * 128), shared ? &map_shared : values ? &map_v : &map_k, x, row, bar);
+        }
+      } else if (lane < pages_per_tile) {
         const CUtensorMap* map = values ? &map_v : &map_k;
 #pragma unroll
         for (int b = 0; b < DBLK; ++b) tma_load_2d(dst + b * (KEYS * 128) + (size_t)lane * p.page_size * 128, map, b * 64, row, bar);
@@ -674,10 +698,11 @@ __global__ void __launch_bounds__(ATT_PERSISTENT_THREADS, 2)
       if (lane == 0) {
         const AttItem& item = ring[c.slot];
         mbar_expect_tx(q_full, (uint32_t)(g * DBLK * tq_cap * 128));
+        const int width = DENSE ? p.q_width : DBLK * 64;
         for (int hg = 0; hg < g; ++hg)
 #pragma unroll
           for (int b = 0; b < DBLK; ++b)
-            tma_load_2d(q_s + b * (ROWS * 128) + (size_t)hg * tq_cap * 128, &map_q, (item.kvh * g + hg) * HD + b * 64, item.tok_base, q_full);
+            tma_load_2d(q_s + b * (ROWS * 128) + (size_t)hg * tq_cap * 128, &map_q, (item.kvh * g + hg) * width + b * 64, item.tok_base, q_full);
       }
       __syncwarp();
     };
@@ -703,7 +728,8 @@ __global__ void __launch_bounds__(ATT_PERSISTENT_THREADS, 2)
         ok = wait0(&empty_k[gt & 1], (uint32_t)((gt >> 1) - 1) & 1u, ERR_ATT_S);
         if (!ok) break;
       }
-      issue_part(row, gt, false);
+      const int kvh = DENSE ? ring[c.slot].kvh : 0;
+      issue_part(row, gt, false, kvh);
       if (gt >= 2) {
         ok = wait0(&empty_v[gt & 1], (uint32_t)((gt >> 1) - 1) & 1u, ERR_ATT_O);
         if (!ok) {
@@ -711,7 +737,7 @@ __global__ void __launch_bounds__(ATT_PERSISTENT_THREADS, 2)
           break;
         }
       }
-      issue_part(row, gt, true);
+      issue_part(row, gt, true, kvh);
       kv_issued = gt + 1;
       c = c1;
       c1 = next(c1);
@@ -741,8 +767,8 @@ __global__ void __launch_bounds__(ATT_PERSISTENT_THREADS, 2)
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         constexpr uint32_t idesc_o = instr_desc_att(64, true);
 #pragma unroll
-        for (int b = 0; b < DBLK; ++b) {
-          const uint64_t dv = smem_desc_sw128(smem_u32(kv_s + (size_t)(t & 1) * 2 * KV_BYTES + KV_BYTES + b * (KEYS * 128)));
+        for (int b = 0; b < VBLK; ++b) {
+          const uint64_t dv = smem_desc_sw128(smem_u32(kv_s + (size_t)(t & 1) * (K_BYTES + V_BYTES) + K_BYTES + b * (KEYS * 128)));
 #pragma unroll
           for (int k = 0; k < KEYS / 16; ++k)
             mma_f16_ts(tmem_base + O_COL + (uint32_t)(b * 64), tmem_base + P_COL + (uint32_t)(k * 8), dv + (uint64_t)(k * (16 * 128 >> 4)),
@@ -766,9 +792,9 @@ __global__ void __launch_bounds__(ATT_PERSISTENT_THREADS, 2)
           asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
           constexpr uint32_t idesc_s = instr_desc_att(KEYS, false);
 #pragma unroll
-          for (int k = 0; k < HD / 16; ++k) {  // 16 dims a step: block k / 4, 32 bytes further along the swizzled row each step
+          for (int k = 0; k < DBLK * 4; ++k) {  // 16 dims a step: block k / 4, 32 bytes further along the swizzled row each step
             const uint64_t dq = smem_desc_sw128(smem_u32(q_s + (k / 4) * (ROWS * 128)));
-            const uint64_t dk = smem_desc_sw128(smem_u32(kv_s + (size_t)(gt & 1) * 2 * KV_BYTES + (k / 4) * (KEYS * 128)));
+            const uint64_t dk = smem_desc_sw128(smem_u32(kv_s + (size_t)(gt & 1) * (K_BYTES + V_BYTES) + (k / 4) * (KEYS * 128)));
             mma_f16(tmem_base + S_COL, dq + (uint64_t)(2 * (k % 4)), dk + (uint64_t)(2 * (k % 4)), idesc_s, k > 0 ? 1u : 0u);
           }
           mma_commit(s_bar);
@@ -853,7 +879,7 @@ __global__ void __launch_bounds__(ATT_PERSISTENT_THREADS, 2)
         for (int c = 0; c < KEYS / 64; ++c) tmem_store32(tmem_base + lane_base + P_COL + c * 32, packed + c * 32);
         if (i > 0 && __any_sync(0xffffffffu, move)) {
 #pragma unroll
-          for (int c = 0; c < HD / 64; ++c) {
+          for (int c = 0; c < VBLK; ++c) {
             float o[64];
             tmem_load32(tmem_base + lane_base + O_COL + c * 64, o);
             tmem_load32(tmem_base + lane_base + O_COL + c * 64 + 32, o + 32);
@@ -877,23 +903,30 @@ __global__ void __launch_bounds__(ATT_PERSISTENT_THREADS, 2)
       if (!ok) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const float inv = l_run > 0.f ? 1.f / l_run : 0.f;
-      uint4* dst = reinterpret_cast<uint4*>(p.out + (size_t)(item.tok_base + tq_row) * p.ld_out + (size_t)(item.kvh * g + hg) * HD);
+      const size_t out_at = (size_t)(item.tok_base + tq_row) * p.ld_out + (size_t)(item.kvh * g + hg) * (VBLK * 64);
+      uint4* dst = reinterpret_cast<uint4*>(p.out + out_at);
 #pragma unroll
-      for (int b = 0; b < HD / 64; ++b) {
+      for (int b = 0; b < VBLK; ++b) {
         float o[64];
         tmem_load32(tmem_base + lane_base + O_COL + b * 64, o);
         tmem_load32(tmem_base + lane_base + O_COL + b * 64 + 32, o + 32);
         tmem_load_wait();
         if (row_ok) {
+          if constexpr (DENSE) {  // float32: the gate behind it rounds once
+            float4* dst32 = reinterpret_cast<float4*>(p.out32 + out_at) + b * 16;
 #pragma unroll
-          for (int c = 0; c < 8; ++c) {
-            uint32_t w[4];
+            for (int c = 0; c < 16; ++c) dst32[c] = make_float4(o[4 * c] * inv, o[4 * c + 1] * inv, o[4 * c + 2] * inv, o[4 * c + 3] * inv);
+          } else {
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              __nv_bfloat162 t = __floats2bfloat162_rn(o[c * 8 + 2 * e] * inv, o[c * 8 + 2 * e + 1] * inv);
-              w[e] = *reinterpret_cast<uint32_t*>(&t);
+            for (int c = 0; c < 8; ++c) {
+              uint32_t w[4];
+#pragma unroll
+              for (int e = 0; e < 4; ++e) {
+                __nv_bfloat162 t = __floats2bfloat162_rn(o[c * 8 + 2 * e] * inv, o[c * 8 + 2 * e + 1] * inv);
+                w[e] = *reinterpret_cast<uint32_t*>(&t);
+              }
+              dst[b * 8 + c] = make_uint4(w[0], w[1], w[2], w[3]);
             }
-            dst[b * 8 + c] = make_uint4(w[0], w[1], w[2], w[3]);
           }
         }
       }
@@ -906,7 +939,7 @@ __global__ void __launch_bounds__(ATT_PERSISTENT_THREADS, 2)
   if (tid == 0) mbar_drain(done_bar, 0, p.error_out);
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
-  if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS_ATT) : "memory");
+  if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(L::TMEM_COLS) : "memory");
   if (tid == 0) {  // the CTA that leaves last puts the counters back to zero for the next launch
     __threadfence();
     if (atomicAdd(&work[1], 1) == (int)gridDim.x - 1) {
@@ -932,18 +965,17 @@ bool launch_att(const CUtensorMap& mk, const CUtensorMap& mv, const AttnTcParams
   return true;
 }
 
-template <int HD>
-bool launch_att_persistent(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const AttnTcParams& p, int n_seqs,
-                           long long max_items, int* work, int n_sms, cudaStream_t stream) {
-  using L = AttLayout<HD>;
-  const size_t smem = L::Q_BYTES + 4 * L::KV_BYTES + 24 * sizeof(uint64_t) + 16 + 8 * sizeof(AttItem) + (size_t)(n_seqs + 1) * sizeof(int) + 1024;
+template <class L>
+bool launch_att_persistent(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const CUtensorMap& mshared, const AttnTcParams& p,
+                           int n_seqs, long long max_items, int* work, int n_sms, cudaStream_t stream) {
+  const size_t smem = L::Q_BYTES + 2 * (L::K_BYTES + L::V_BYTES) + 24 * sizeof(uint64_t) + 16 + 8 * sizeof(AttItem) + (size_t)(n_seqs + 1) * sizeof(int) + 1024;
   static size_t attr_smem = 0;
   if (smem > attr_smem) {
-    if (cudaFuncSetAttribute(paged_attention_tc_persistent_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return false;
+    if (cudaFuncSetAttribute(paged_attention_tc_persistent_kernel<L>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) return false;
     attr_smem = smem;
   }
-  const int grid = (int)std::min<long long>(max_items, 2 * n_sms);  // (the step may hold fewer items than max_items: CTAs without one leave at once)
-  launch_kernel(paged_attention_tc_persistent_kernel<HD>, grid, ATT_PERSISTENT_THREADS, smem, stream, mq, mk, mv, p, n_seqs, work);
+  const int grid = (int)std::min<long long>(max_items, L::CTAS * n_sms);  // (the step may hold fewer items than max_items: CTAs without one leave at once)
+  launch_kernel(paged_attention_tc_persistent_kernel<L>, grid, ATT_PERSISTENT_THREADS, smem, stream, mq, mk, mv, mshared, p, n_seqs, work);
   return true;
 }
 
@@ -993,7 +1025,7 @@ extern "C" int llm_paged_attention_tc(const void* q, long long ld_q, const void*
   const long long rows = n_cache_pages * nkv * page_size;
   LLM_REQUIRE(tensor_map_for(kcache, rows, hd, hd, page_size, &mk) && tensor_map_for(vcache, rows, hd, hd, page_size, &mv),
               "attention_tc: cuTensorMapEncodeTiled failed");
-  AttnTcParams p;
+  AttnTcParams p = {};
   p.q = (const bf16*)q; p.ld_q = ld_q; p.seq_start = seq_start; p.seq_ntok = seq_ntok; p.seq_qoff = seq_qoff; p.block_table = block_table;
   p.max_blocks = max_blocks; p.nq = nq; p.nkv = nkv; p.page_size = page_size; p.window = window; p.scale = scale;
   p.out = (bf16*)out; p.ld_out = ld_out; p.error_out = error_word();
@@ -1008,8 +1040,8 @@ extern "C" int llm_paged_attention_tc(const void* q, long long ld_q, const void*
     // at most: every token a query tile of its own, or every request as many as the longest portion
     const long long max_items = std::min<long long>((long long)n_tokens, (long long)n_seqs * ((max_new_tokens + ptq - 1) / ptq)) * nkv;
     LLM_REQUIRE(max_items < (1LL << 30) && n_seqs < 40000, "attention_tc: too many query tiles");
-    const bool ok = hd == 64 ? launch_att_persistent<64>(mq, mk, mv, p, n_seqs, max_items, work, att_sm_count(), stream)
-                             : launch_att_persistent<128>(mq, mk, mv, p, n_seqs, max_items, work, att_sm_count(), stream);
+    const bool ok = hd == 64 ? launch_att_persistent<AttLayout<64>>(mq, mk, mv, mk, p, n_seqs, max_items, work, att_sm_count(), stream)
+                             : launch_att_persistent<AttLayout<128>>(mq, mk, mv, mk, p, n_seqs, max_items, work, att_sm_count(), stream);
     LLM_REQUIRE(ok, "attention_tc: cannot raise the shared memory limit");
     LLM_CHECK_LAUNCH("paged_attention_tc");
     return LLM_OK;
@@ -1020,5 +1052,164 @@ extern "C" int llm_paged_attention_tc(const void* q, long long ld_q, const void*
   else attr_ok = launch_att<128>(mk, mv, p, grid, max_blocks, stream);
   LLM_REQUIRE(attr_ok, "attention_tc: cannot raise the shared memory limit");
   LLM_CHECK_LAUNCH("paged_attention_tc");
+  return LLM_OK;
+}
+
+// ---------------------------------------------------------------------------------------------
+// Latent attention of prompt portions in its expanded form. The cache holds one latent a token, shared by the heads; the attention
+// over latents itself (latent_mma.cu) multiplies 2 (latent + rotated + latent) numbers a (query, key) pair and head, the one over
+// per-head keys and values 2 (key + rotated + value): 2,176 against 640 at a latent of 512. For that every latent of the context is
+// expanded once a step, 2 x latent x (key + value) operations a head, which a portion of some dozen tokens already earns back.
+// 2,048 tokens, 16 heads of 128 + 64 / 128 from latents of 512: rows 2.9, their product 19.8, rotation 3.6, attention 43 (500 TFLOP/s;
+// softmax-bound like the paged kernel), gate 7.6 us, together 84; over the latents 769. The roundings to bfloat16 are as many (keys
+// and values instead of mapped queries and sums): logits of whole models are as near the 32-bit engine's either way (median of a
+// row 0.0030 of its size, 128 to 2,048 tokens).
+
+namespace {
+
+// rows [n_seqs * rows_per_seq, width]: the cached rows of the requests in order of position, zeros behind a request's last token,
+// on pages that were given back, and in the columns behind the cached ones. Groups of 8 numbers, a warp a row.
+__global__ void __launch_bounds__(256)
+    latent_rows_kernel(const bf16* __restrict__ cache, const int* __restrict__ seq_len, const int* __restrict__ table, int max_blocks, int page_size,
+                       int groups_in, int groups_out, int rows_per_seq, bf16* __restrict__ out) {
+  dep_launch();
+  dep_wait();
+  const int row = blockIdx.x * 8 + (threadIdx.x >> 5), seq = blockIdx.y;
+  if (row >= rows_per_seq) return;
+  int page = -1;
+  if (row < seq_len[seq]) page = table[(size_t)seq * max_blocks + row / page_size];
+  const uint4* src = reinterpret_cast<const uint4*>(cache) + ((size_t)max(page, 0) * page_size + row % page_size) * groups_in;
+  uint4* dst = reinterpret_cast<uint4*>(out) + ((size_t)seq * rows_per_seq + row) * groups_out;
+  for (int g = threadIdx.x & 31; g < groups_out; g += 32) dst[g] = page >= 0 && g < groups_in ? src[g] : make_uint4(0, 0, 0, 0);
+}
+
+// The rotated part of every query head in place: pairs (j, j + half) of its first 2 * half numbers turned by the token's position, 8
+// pairs a thread.
+__global__ void __launch_bounds__(256)
+    rotate_heads_kernel(bf16* __restrict__ q, long long ld_q, int heads, int width, int off, int half, const float* __restrict__ cos_t,
+                        const float* __restrict__ sin_t, const int* __restrict__ positions, int n_tokens) {
+  dep_launch();
+  dep_wait();
+  const int per_head = half / 8, i = blockIdx.x * blockDim.x + threadIdx.x, t = i / (heads * per_head);
+  if (t >= n_tokens) return;
+  const int rest = i - t * heads * per_head, h = rest / per_head, j = (rest - h * per_head) * 8;
+  bf16* row = q + (size_t)t * ld_q + (size_t)h * width + off + j;
+  uint4 lo = *reinterpret_cast<const uint4*>(row), hi = *reinterpret_cast<const uint4*>(row + half);
+  const float* c = cos_t + (size_t)positions[t] * half + j;
+  const float* s = sin_t + (size_t)positions[t] * half + j;
+  __nv_bfloat162* a = reinterpret_cast<__nv_bfloat162*>(&lo);
+  __nv_bfloat162* b = reinterpret_cast<__nv_bfloat162*>(&hi);
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const float2 x = __bfloat1622float2(a[k]), y = __bfloat1622float2(b[k]);
+    a[k] = __floats2bfloat162_rn(x.x * c[2 * k] - y.x * s[2 * k], x.y * c[2 * k + 1] - y.y * s[2 * k + 1]);
+    b[k] = __floats2bfloat162_rn(y.x * c[2 * k] + x.x * s[2 * k], y.y * c[2 * k + 1] + x.y * s[2 * k + 1]);
+  }
+  *reinterpret_cast<uint4*>(row) = lo;
+  *reinterpret_cast<uint4*>(row + half) = hi;
+}
+
+// out [n_tokens, heads * dim] = x * sigmoid(gate), a float32 gate a number or one a head; 8 numbers a thread.
+__global__ void __launch_bounds__(256)
+    gate_heads_kernel(const float* __restrict__ x, bf16* __restrict__ out, const float* __restrict__ gate, long long ld_gate, int heads, int dim, int per_head, int n_tokens) {
+  dep_launch();
+  dep_wait();
+  const int per_row = heads * dim / 8, i = blockIdx.x * blockDim.x + threadIdx.x, t = i / per_row;
+  if (t >= n_tokens) return;
+  const int c = (i - t * per_row) * 8;
+  const float* g = gate + (size_t)t * ld_gate + (per_head ? c / dim : c);
+  const size_t at = (size_t)t * heads * dim + c;
+  const float4 lo = *reinterpret_cast<const float4*>(x + at), hi = *reinterpret_cast<const float4*>(x + at + 4);
+  const float2 in[4] = {{lo.x, lo.y}, {lo.z, lo.w}, {hi.x, hi.y}, {hi.z, hi.w}};
+  uint4 v;
+  __nv_bfloat162* h = reinterpret_cast<__nv_bfloat162*>(&v);
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const float2 f = in[k];
+    h[k] = __floats2bfloat162_rn(f.x * (1.0f / (1.0f + expf(-g[per_head ? 0 : 2 * k]))), f.y * (1.0f / (1.0f + expf(-g[per_head ? 0 : 2 * k + 1]))));
+  }
+  *reinterpret_cast<uint4*>(out + at) = v;
+}
+
+}  // namespace
+
+// out [n_tokens, heads * dim] bf16 = x (float32, rows of both without gaps) * sigmoid(gate), float32 rows of ld_gate: a gate a number, or
+// per_head one a head.
+extern "C" int llm_gate_heads(const float* x, void* out, const float* gate, long long ld_gate, int heads, int dim, int per_head, int n_tokens, cudaStream_t stream) {
+  if (n_tokens == 0) return LLM_OK;
+  LLM_REQUIRE(n_tokens > 0 && heads > 0 && dim > 0 && dim % 8 == 0 && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(out)) & 15u) == 0, "gate_heads: heads of whole groups of 8 numbers");
+  const long long total = (long long)n_tokens * heads * (dim / 8);
+  LLM_REQUIRE(total < (1LL << 31) - 256, "gate_heads: too many numbers");
+  launch_kernel(gate_heads_kernel, (int)((total + 255) / 256), 256, 0, stream, x, (bf16*)out, gate, ld_gate, heads, dim, per_head, n_tokens);
+  LLM_CHECK_LAUNCH("gate_heads");
+  return LLM_OK;
+}
+
+// q [n_tokens, heads * width] bf16: numbers off .. off + 2 half of every head rotated in place; half, off and width multiples of 8.
+extern "C" int llm_rotate_heads(void* q, long long ld_q, int heads, int width, int off, int half, const float* cos_t, const float* sin_t,
+                                const int* positions, int n_tokens, cudaStream_t stream) {
+  if (n_tokens == 0 || half == 0) return LLM_OK;
+  LLM_REQUIRE(n_tokens > 0 && heads > 0 && half % 8 == 0 && off % 8 == 0 && width % 8 == 0 && ld_q % 8 == 0 && off + 2 * half <= width &&
+              (reinterpret_cast<uintptr_t>(q) & 15u) == 0, "rotate_heads: parts of whole groups of 8 numbers");
+  const long long total = (long long)n_tokens * heads * (half / 8);
+  LLM_REQUIRE(total < (1LL << 31) - 256, "rotate_heads: too many numbers");
+  launch_kernel(rotate_heads_kernel, (int)((total + 255) / 256), 256, 0, stream, (bf16*)q, ld_q, heads, width, off, half, cos_t, sin_t, positions, n_tokens);
+  LLM_CHECK_LAUNCH("rotate_heads");
+  return LLM_OK;
+}
+
+extern "C" int llm_latent_rows(const void* cache, const int* seq_len, const int* block_table, int max_blocks, int page_size, int width_in, int width_out,
+                               int n_seqs, int rows_per_seq, void* out, cudaStream_t stream) {
+  if (n_seqs == 0) return LLM_OK;
+  LLM_REQUIRE(n_seqs > 0 && n_seqs <= 65535 && rows_per_seq > 0 && page_size > 0 && max_blocks > 0, "latent_rows: bad sizes");
+  LLM_REQUIRE(width_in > 0 && width_in % 8 == 0 && width_out % 8 == 0 && width_in <= width_out, "latent_rows: rows of whole groups of 8 numbers");
+  LLM_REQUIRE(((reinterpret_cast<uintptr_t>(cache) | reinterpret_cast<uintptr_t>(out)) & 15u) == 0, "latent_rows: rows must begin on 16 bytes");
+  launch_kernel(latent_rows_kernel, dim3((rows_per_seq + 7) / 8, n_seqs), 256, 0, stream, (const bf16*)cache, seq_len, block_table, max_blocks, page_size,
+                width_in / 8, width_out / 8, rows_per_seq, (bf16*)out);
+  LLM_CHECK_LAUNCH("latent_rows");
+  return LLM_OK;
+}
+
+// Whether the expanded form takes these sizes: heads whose own key part and value are 64 or both 128 numbers, a rotated part of at
+// most one block of 64.
+extern "C" int llm_latent_expanded_supported(int heads, int dim, int rot_dim, int vdim, int kv_rank) {
+  return heads > 0 && heads <= 65535 && (dim == 64 || dim == 128) && vdim == dim && rot_dim > 0 && rot_dim <= 64 && rot_dim % 8 == 0 &&
+         kv_rank > 0 && kv_rank % 8 == 0 && encode_fn() != nullptr;
+}
+
+// q [n_tokens, heads * (dim + rot_dim)] (the rotated part rotated); keys [rows, heads * dim] and values [rows, heads * vdim], row
+// strides ld_keys and ld_values; shared [rows, ld_shared]: the rotated part from column shared_col on, zeros behind it up to 64;
+// rows = n_seqs * rows_per_seq, rows_per_seq a multiple of 128. out float32 [n_tokens, heads * vdim]. (The output gate is a kernel of
+// its own: in this one's epilogue a thread reads a row of gates, line by line for itself, and 2,048 tokens took 78 us instead of 40.)
+extern "C" int llm_latent_attention_expanded(const void* q, long long ld_q, const void* keys, long long ld_keys, const void* values, long long ld_values,
+                                             const void* shared, long long ld_shared, int shared_col, int rows_per_seq, const int* seq_start,
+                                             const int* seq_ntok, const int* seq_qoff, float* out, long long ld_out, int n_seqs, int n_tokens,
+                                             int max_new_tokens, int heads, int dim, int rot_dim, int vdim, float scale, int window, int* work,
+                                             cudaStream_t stream) {
+  if (n_seqs == 0 || max_new_tokens == 0) return LLM_OK;
+  LLM_REQUIRE(llm_latent_expanded_supported(heads, dim, rot_dim, vdim, 8), "latent_expanded: sizes not supported (%d heads of %d + %d / %d)", heads, dim, rot_dim, vdim);
+  auto al = [](const void* ptr) { return (reinterpret_cast<uintptr_t>(ptr) & 15u) == 0; };
+  LLM_REQUIRE(al(q) && al(keys) && al(values) && al(shared) && al(out), "latent_expanded: operands must be 16-byte aligned");
+  LLM_REQUIRE(ld_q % 8 == 0 && ld_keys % 8 == 0 && ld_values % 8 == 0 && ld_shared % 8 == 0 && ld_out % 8 == 0 && shared_col % 8 == 0 &&
+              shared_col + 64 <= ld_shared, "latent_expanded: bad row strides");
+  LLM_REQUIRE(rows_per_seq > 0 && rows_per_seq % 128 == 0 && (long long)n_seqs * rows_per_seq < (1LL << 31) && n_seqs < 40000 && window >= 0 &&
+              n_tokens >= ROWS && work != nullptr, "latent_expanded: bad sizes");
+  LLM_REQUIRE(error_word() != nullptr, "latent_expanded: cannot allocate the error word");
+  const long long rows = (long long)n_seqs * rows_per_seq;
+  CUtensorMap mq, mk, mv, ms;
+  LLM_REQUIRE(tensor_map_for(q, n_tokens, (long long)heads * (dim + rot_dim), ld_q, ROWS, &mq) &&
+              tensor_map_for(keys, rows, (long long)heads * dim, ld_keys, 128, &mk) &&
+              tensor_map_for(values, rows, (long long)heads * vdim, ld_values, 128, &mv) &&
+              tensor_map_for(shared, rows, shared_col + 64, ld_shared, 128, &ms), "latent_expanded: cuTensorMapEncodeTiled failed");
+  AttnTcParams p = {};
+  p.seq_start = seq_start; p.seq_ntok = seq_ntok; p.seq_qoff = seq_qoff;
+  p.nq = p.nkv = heads; p.window = window; p.scale = scale; p.out32 = out; p.ld_out = ld_out; p.error_out = error_word();
+  p.q_width = dim + rot_dim; p.rows_per_seq = rows_per_seq; p.shared_col = shared_col;
+  const long long max_items = std::min<long long>((long long)n_tokens, (long long)n_seqs * ((max_new_tokens + ROWS - 1) / ROWS)) * heads;
+  LLM_REQUIRE(max_items < (1LL << 30), "latent_expanded: too many query tiles");
+  const bool ok = dim == 64 ? launch_att_persistent<DenseLayout<1, 1>>(mq, mk, mv, ms, p, n_seqs, max_items, work, att_sm_count(), stream)
+                            : launch_att_persistent<DenseLayout<2, 2>>(mq, mk, mv, ms, p, n_seqs, max_items, work, att_sm_count(), stream);
+  LLM_REQUIRE(ok, "latent_expanded: cannot raise the shared memory limit");
+  LLM_CHECK_LAUNCH("latent_attention_expanded");
   return LLM_OK;
 }

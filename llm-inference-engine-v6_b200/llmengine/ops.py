@@ -986,6 +986,81 @@ class CudaOps:
                                          _ptr(positions), c_int(dtype_code(q.dtype)), _stream()), lib)
         return ql
 
+    # The expanded form of latent attention: every latent of the contexts becomes a key and a value a head, once a step. It costs
+    # 4.2 MFLOP a cached token (16 heads of 128 + 128 from 512) on the dense products; the attention over latents costs 3.4 times the
+    # operations of the one over keys and values, on the slower tensor path. From about 50 tokens a request it is the faster way
+    # (16 heads of 128 + 64 / 128, all of it: 2,048 tokens 84 us against 769, 128 tokens behind 2,000 others 65 against 327), up to
+    # LATENT_EXPANDED_ROWS rows, which bounds what the step keeps beside the cache.
+    LATENT_EXPANDED_TOKENS = 48
+    LATENT_EXPANDED_ROWS = 32768
+
+    def latent_expanded_sizes(self, heads: int, dim: int, rot_dim: int, vdim: int, kv_rank: int, rot_dims: int) -> bool:
+        return (self.tensor_cores and self.latent_tensor_cores and rot_dims % 16 == 0 and
+                bool(self.lib("tensorcore").llm_latent_expanded_supported(c_int(heads), c_int(dim), c_int(rot_dim), c_int(vdim), c_int(kv_rank))))
+
+    def latent_expanded_rows(self, batch) -> int:
+        """Rows a request takes in the expanded form of this step's latent attention; 0: the step runs over the latents."""
+        rows = -(-batch.max_seq_len // 128) * 128
+        if (batch.n_tokens < max(128, self.LATENT_EXPANDED_TOKENS * batch.n_seqs) or batch.n_seqs * rows > self.LATENT_EXPANDED_ROWS or
+                not (self.tensor_cores and self.latent_tensor_cores)):
+            return 0
+        return rows
+
+    def latent_rows(self, cache: torch.Tensor, batch, block_table: torch.Tensor, out: torch.Tensor, rows: int) -> torch.Tensor:
+        """out [n_seqs * rows, width]: the cached rows of every request in order of position, zeros elsewhere."""
+        _need(cache, "latent_rows.cache", torch.bfloat16); _need(out, "latent_rows.out", torch.bfloat16)
+        _need(block_table, "latent_rows.block_table", torch.int32)
+        assert cache.is_contiguous() and out.is_contiguous() and block_table.is_contiguous() and out.shape[0] == batch.n_seqs * rows
+        lib = self.lib("tensorcore")
+        self._check(lib.llm_latent_rows(_ptr(cache), _ptr(batch.seq_len), _ptr(block_table), c_int(block_table.shape[1]), c_int(cache.shape[2]),
+                                        c_int(cache.shape[3]), c_int(out.shape[1]), c_int(batch.n_seqs), c_int(rows), _ptr(out), _stream()), lib)
+        return out
+
+    def rotate_heads(self, q: torch.Tensor, heads: int, width: int, off: int, cos: Optional[torch.Tensor], sin: Optional[torch.Tensor],
+                     positions: torch.Tensor) -> torch.Tensor:
+        """q [n, heads * width] bfloat16 in place: numbers off .. off + 2 * cos.shape[1] of every head turned by the token's position."""
+        if cos is None:
+            return q
+        _need(q, "rotate_heads.q", torch.bfloat16); _need(cos, "rotate_heads.cos", torch.float32); _need(sin, "rotate_heads.sin", torch.float32)
+        _need(positions, "rotate_heads.positions", torch.int32)
+        assert q.shape[1] == heads * width and cos.is_contiguous() and sin.is_contiguous() and positions.numel() >= q.shape[0]
+        lib = self.lib("tensorcore")
+        self._check(lib.llm_rotate_heads(_ptr(q), c_longlong(q.stride(0)), c_int(heads), c_int(width), c_int(off), c_int(cos.shape[1]), _ptr(cos),
+                                         _ptr(sin), _ptr(positions), c_int(q.shape[0]), _stream()), lib)
+        return q
+
+    def gate_heads(self, x: torch.Tensor, out: torch.Tensor, gate: torch.Tensor, gate_off: int, heads: int, dim: int,
+                   per_head: bool = False) -> torch.Tensor:
+        """out [n, heads * dim] (bfloat16) = x (float32) * sigmoid(gate[:, gate_off ..]) (float32 [n, width]), a gate a number or one a head."""
+        _need(x, "gate_heads.x", torch.float32); _need(out, "gate_heads.out", torch.bfloat16); _need(gate, "gate_heads.gate", torch.float32)
+        assert x.is_contiguous() and out.is_contiguous() and x.shape == out.shape and x.shape[1] == heads * dim and gate.shape[0] >= x.shape[0]
+        assert gate_off >= 0 and gate_off + (heads if per_head else heads * dim) <= gate.shape[1]
+        lib = self.lib("tensorcore")
+        self._check(lib.llm_gate_heads(_ptr(x), _ptr(out), c_void_p(gate.data_ptr() + 4 * gate_off), c_longlong(gate.stride(0)), c_int(heads), c_int(dim),
+                                       c_int(1 if per_head else 0), c_int(x.shape[0]), _stream()), lib)
+        return out
+
+    def latent_attention_expanded(self, q: torch.Tensor, keys: torch.Tensor, values: torch.Tensor, shared: torch.Tensor, shared_col: int, rows: int,
+                                  batch, out: torch.Tensor, heads: int, dim: int, rot_dim: int, vdim: int, scale: float,
+                                  window: int = 0) -> torch.Tensor:
+        """Causal attention with a key [keys of the head | shared part] and a value a head: q [n, heads * (dim + rot_dim)], keys and values
+        [n_seqs * rows, heads * dim] / [.., heads * vdim], shared: the rotated part from column shared_col on (zeros behind it up to
+        64). out float32 [n, heads * vdim]."""
+        for t, name in ((q, "q"), (keys, "keys"), (values, "values"), (shared, "shared")):
+            _need(t, "latent_expanded." + name, torch.bfloat16)
+        _need(out, "latent_expanded.out", torch.float32)
+        assert q.shape == (batch.n_tokens, heads * (dim + rot_dim)) and out.shape == (batch.n_tokens, heads * vdim)
+        assert keys.shape == (batch.n_seqs * rows, heads * dim) and values.shape == (batch.n_seqs * rows, heads * vdim)
+        assert shared.shape[0] == batch.n_seqs * rows and shared_col + 64 <= shared.shape[1]
+        work = batch.ws.get_zeroed("attention.work_counters", (2,), torch.int32)  # left at zero by the kernel
+        lib = self.lib("tensorcore")
+        self._check(lib.llm_latent_attention_expanded(
+            _ptr(q), c_longlong(q.stride(0)), _ptr(keys), c_longlong(keys.stride(0)), _ptr(values), c_longlong(values.stride(0)), _ptr(shared),
+            c_longlong(shared.stride(0)), c_int(shared_col), c_int(rows), _ptr(batch.seq_start), _ptr(batch.seq_ntok), _ptr(batch.seq_qoff),
+            _ptr(out), c_longlong(out.stride(0)), c_int(batch.n_seqs), c_int(batch.n_tokens), c_int(batch.max_new_tokens), c_int(heads), c_int(dim),
+            c_int(rot_dim), c_int(vdim), c_float(scale), c_int(window), _ptr(work), _stream()), lib)
+        return out
+
     def latent_attention(self, ql: torch.Tensor, cache: torch.Tensor, batch, block_table: torch.Tensor, out: torch.Tensor,
                          kv_rank: int, scale: float, window: int = 0, sink: Optional[torch.Tensor] = None) -> torch.Tensor:
         """Causal softmax attention of every token of the step over the cached rows lo..pos of its request: ql [n, H, Dk]
