@@ -63,6 +63,8 @@ def _stream():
 
 
 def _need(t: torch.Tensor, name: str, dtype=None, rows_contiguous: bool = True) -> None:
+    if t.is_cuda and (dtype is None or t.dtype is dtype) and (not rows_contiguous or t.is_contiguous()):
+        return  # (what nearly every operand is; the questions below cost three times as much)
     if not t.is_cuda:
         raise KernelError(f"{name}: expected a CUDA tensor (the kernels have no CPU path)")
     if dtype is not None and t.dtype != dtype:
@@ -254,7 +256,7 @@ class CudaOps:
         if delta is not None:
             _need(delta, "rmsnorm.delta", torch.float32)
             assert delta.is_contiguous() and delta.shape[-1] == dim
-            n_part, pstride = (delta.shape[0], delta.stride(0)) if delta.dim() == 3 else (1, 0)
+            n_part, pstride = (delta.shape[0], delta.shape[1] * dim) if delta.dim() == 3 else (1, 0)
         if rows is not None:
             _need(rows, "rmsnorm.rows", torch.int32)
             write_back = False
@@ -317,7 +319,8 @@ class CudaOps:
         if m > self.SWAP_MAX_TOKENS and (act[0] if isinstance(act, tuple) else act) in self.EPILOGUE_ACTIVATIONS and self._tc_usable(a, w_blocked):
             assert row_scale is None, "a row scale is applied where partial sums are consumed (few tokens)"
             lib = self.lib("tensorcore")
-            self._check(lib.llm_gemm_tc_swiglu(_at(a), _at(w_blocked), _at(out), m, ff, k, a.stride(0), w_blocked.stride(0), out.stride(0),
+            lda, ldw = k if a.is_contiguous() else a.stride(0), k if w_blocked.is_contiguous() else w_blocked.stride(0)
+            self._check(lib.llm_gemm_tc_swiglu(a.data_ptr(), w_blocked.data_ptr(), out.data_ptr(), m, ff, k, lda, ldw, ff,
                                                *self._act_args(act), _stream()), lib)
             return out
         assert ws is not None, "gemm_swiglu needs a workspace when it cannot fuse"
@@ -344,8 +347,10 @@ class CudaOps:
             self._known["tma"] = bool(self.lib("tensorcore").llm_gemm_tc_supported(c_void_p(16), c_void_p(16), c_int(1), c_int(1), c_int(8),
                                                                                    c_longlong(8), c_longlong(8)))
         m, k = a.shape
+        # (a row stride is the inner size where nothing lies between the rows: strides are slow to ask for)
+        lda, ldw = k if a.is_contiguous() else a.stride(0), w.shape[1] if w.is_contiguous() else w.stride(0)
         return (self._known["tma"] and m > 0 and k > 0 and w.shape[0] > 0 and
-                (k | a.stride(0) | w.stride(0)) % 8 == 0 and (a.data_ptr() | w.data_ptr()) % 16 == 0)
+                (k | lda | ldw) % 8 == 0 and (a.data_ptr() | w.data_ptr()) % 16 == 0)
 
     SWAP_MAX_TOKENS = 64  # up to here weights fill the accumulator lanes and tokens the columns, several CTAs an SM
 
@@ -398,7 +403,9 @@ class CudaOps:
         N = w.shape[0]
         swap, splits, stages = form
         lib = self.lib("tensorcore")
-        self._check(lib.llm_gemm_tc(_at(a), _at(w), _at(out), M, N, K, a.stride(0), w.stride(0), out.stride(-2), dtype_code(out.dtype), swap, splits,
+        lda, ldw = K if a.is_contiguous() else a.stride(0), K if w.is_contiguous() else w.stride(0)
+        ldo = N if out.is_contiguous() else out.stride(-2)
+        self._check(lib.llm_gemm_tc(a.data_ptr(), w.data_ptr(), out.data_ptr(), M, N, K, lda, ldw, ldo, dtype_code(out.dtype), swap, splits,
                                     split_stride, stages, _stream()), lib)
 
     def gemm(self, a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, ws=None) -> torch.Tensor:

@@ -95,7 +95,9 @@ class PagedAttention(Mixer):
                 row_scale, x, few = x.row_scale(ops), x.prescaled, False
             elif not (few and cache.writes and self.position.takes_partial_sums):
                 x = x.dense(ctx)
-        if cache.writes and self.position.takes_partial_sums and (n <= 64 or (hasattr(ops, "gemm_cuts") and ops.gemm_cuts(x[:n], self.w_qkv))):
+        if not isinstance(x, NormalizedRows) and x.shape[0] != n:
+            x = x[:n]
+        if cache.writes and self.position.takes_partial_sums and (n <= 64 or (hasattr(ops, "gemm_cuts") and ops.gemm_cuts(x, self.w_qkv))):
             # few tokens: the product comes as float32 sums (in parts, unless the K pieces were added
             # inside the product), finished by the position kernel or by the attention kernel
             if few:
@@ -103,9 +105,9 @@ class PagedAttention(Mixer):
                 if isinstance(x, NormalizedRows):
                     ops.gemm_few_tokens(self.w_qkv, parts[0], "plain", norm=(x.h, x.sumsq, x.weight, x.eps, x.rows), n_tokens=n, ws=ctx.ws)
                 else:
-                    ops.gemm_few_tokens(self.w_qkv, parts[0], "plain", x=x[:n], ws=ctx.ws)
+                    ops.gemm_few_tokens(self.w_qkv, parts[0], "plain", x=x, ws=ctx.ws)
             else:
-                parts = ops.gemm_partials(x[:n], self.w_qkv, ctx.ws, "attention.qkv_parts")
+                parts = ops.gemm_partials(x, self.w_qkv, ctx.ws, "attention.qkv_parts")
             tables = self.position.rotation_tables() if cache.k is not None else None
             if tables is not None and ops.decode_attention_fusable(ctx, cache.k, s.num_heads, s.num_kv_heads, s.head_dim, att):
                 # single decoded tokens: summing the parts, rotation and the cache write happen inside the attention kernel
@@ -117,7 +119,7 @@ class PagedAttention(Mixer):
             extra = {} if row_scale is None else {"row_scale": row_scale}
             self.position.rotate_and_store(qkv, ctx, cache, s.num_heads, s.num_kv_heads, s.head_dim, parts=parts, **extra)
         else:
-            ops.gemm(x[:n], self.w_qkv, qkv, ctx.ws)
+            ops.gemm(x, self.w_qkv, qkv, ctx.ws)
             self.position.rotate_and_store(qkv, ctx, cache, s.num_heads, s.num_kv_heads, s.head_dim)
         ops.paged_attention(qkv[:, :dq], cache.k, cache.v, ctx, ctx.block_tables[cache.group], att, s.num_heads,
                             s.num_kv_heads, s.head_dim, self.scale, s.window)
@@ -135,7 +137,7 @@ def add_into_stream_or_partials(ops, x: torch.Tensor, w: torch.Tensor, ctx, few:
     (so that the next norm need not run); otherwise it returns float32 partial sums."""
     res, n = ctx.residual, ctx.n_tokens
     if (not few and res is not None and res.pending is None and res.h.shape[1] == w.shape[0] and x.dtype == torch.bfloat16 and
-            hasattr(ops, "gemm_meet") and ops.can_meet(x[:n], w)):
+            getattr(ops, "meet_products", False) and ops.can_meet(x[:n], w)):
         # few tokens: the K splits meet inside the product, which adds their sum into the stream and
         # leaves, for the norm that reads the stream next, its weight times the stream and the parts of
         # the rows' sums of squares
@@ -149,7 +151,7 @@ def add_into_stream_or_partials(ops, x: torch.Tensor, w: torch.Tensor, ctx, few:
         res.sumsq, res.prescaled, res.prescaled_weight = ss, scaled, wn
         return None
     if (not few and res is not None and res.pending is None and res.h.shape[1] == w.shape[0] and x.dtype == torch.bfloat16 and
-            hasattr(ops, "gemm_add_into") and ops.can_add_into(x[:n], w)):
+            getattr(ops, "add_into_stream", False) and ops.can_add_into(x[:n], w)):
         # a prompt-sized step: the product's epilogue adds into the stream (the same float32 sums as the
         # next norm would have made from the product written out)
         res_sumsq_off(res)

@@ -90,13 +90,15 @@ class GatedMLP(FeedForward):
                 x = x.dense(ctx)
         if s.activation != "silu":
             extra["act"] = self.act
+        if x.shape[0] != n:
+            x = x[:n]
         if self.blocked:
-            ops.gemm_swiglu(x[:n], self.w_gate_up, act, ctx.ws, **extra)
+            ops.gemm_swiglu(x, self.w_gate_up, act, ctx.ws, **extra)
         elif n <= 64:  # few tokens: the products may come as partial sums, added by their consumers
-            ops.silu_mul_partials(ops.gemm_partials(x[:n], self.w_gate_up, ctx.ws, "mlp.gate_up_parts"), act, **extra)
+            ops.silu_mul_partials(ops.gemm_partials(x, self.w_gate_up, ctx.ws, "mlp.gate_up_parts"), act, **extra)
         else:
             gate_up = ctx.ws.get("mlp.gate_up", (n, 2 * s.intermediate), self.env.dtype)
-            ops.gemm(x[:n], self.w_gate_up, gate_up)
+            ops.gemm(x, self.w_gate_up, gate_up)
             ops.silu_mul(gate_up, act, **({"act": self.act} if s.activation != "silu" else {}))
         return add_into_stream_or_partials(ops, act, self.w_down, ctx, False, "mlp.delta")
 
