@@ -19,15 +19,13 @@ namespace {
 constexpr int RM_ROWS = 64, RM_COLS = 64, RM_BK = 64, RM_LD = RM_BK + 8, RM_THREADS = 128, RM_STAGES = 3;
 constexpr size_t RM_SMEM = (size_t)RM_STAGES * (RM_ROWS + RM_COLS) * RM_LD * sizeof(bf16);
 
-// WM 1: a tile of 64 rows x 64 columns, four warps of 16 x 64. WM 2 (many rows an expert): 128 x 128, eight warps of
-// 32 x 64 (four along the rows, two along the columns): six ldmatrix feed sixteen mma instead of five feeding eight,
-// and a row of the expert's matrix is fetched for twice as many rows.
-template <typename TO, int EPI, int WM>
-__global__ void __launch_bounds__(RM_THREADS * WM)
+// A tile of 64 rows x 64 columns, four warps of 16 x 64. (Many rows an expert run on tcgen05: routed_tc.cu.)
+template <typename TO, int EPI>
+__global__ void __launch_bounds__(RM_THREADS)
     routed_product_mma_kernel(const bf16* __restrict__ a, long long lda, int a_div, const bf16* __restrict__ w, long long w_stride, int N,
                               int K, const int* __restrict__ tile_expert, const int* __restrict__ tile_rows, TO* __restrict__ out,
                               long long ldo, const float* __restrict__ share, int act, float p0, float p1) {
-  constexpr int ROWS = RM_ROWS * WM, COLS = RM_COLS * WM, THREADS = RM_THREADS * WM;
+  constexpr int ROWS = RM_ROWS, COLS = RM_COLS, THREADS = RM_THREADS;
   extern __shared__ __align__(16) uint8_t smem_raw[];
   bf16 (*a_s)[ROWS][RM_LD] = reinterpret_cast<bf16 (*)[ROWS][RM_LD]>(smem_raw);
   bf16 (*w_s)[COLS][RM_LD] = reinterpret_cast<bf16 (*)[COLS][RM_LD]>(smem_raw + (size_t)RM_STAGES * ROWS * RM_LD * sizeof(bf16));
@@ -35,7 +33,6 @@ __global__ void __launch_bounds__(RM_THREADS * WM)
   dep_launch();
   dep_wait();
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int warp_m = warp % 4, warp_n = warp / 4;
   const int e = tile_expert[blockIdx.y];
   if (e < 0) return;
   const int n0 = blockIdx.x * COLS;
@@ -56,11 +53,9 @@ __global__ void __launch_bounds__(RM_THREADS * WM)
     }
   };
 
-  float acc[WM][RM_COLS / 8][4];
+  float acc[RM_COLS / 8][4];
 #pragma unroll
-  for (int i = 0; i < WM; ++i)
-#pragma unroll
-    for (int j = 0; j < RM_COLS / 8; ++j) acc[i][j][0] = acc[i][j][1] = acc[i][j][2] = acc[i][j][3] = 0.f;
+  for (int j = 0; j < RM_COLS / 8; ++j) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.f;
   const int k_tiles = (K + RM_BK - 1) / RM_BK;
 #pragma unroll
   for (int st = 0; st < RM_STAGES - 1; ++st) {  // the ring's first stages
@@ -75,52 +70,45 @@ __global__ void __launch_bounds__(RM_THREADS * WM)
     cp_async_commit();
 #pragma unroll
     for (int ks = 0; ks < RM_BK / 16; ++ks) {
-      uint32_t af[WM][4];
-#pragma unroll
-      for (int i = 0; i < WM; ++i) ldmatrix_x4(af[i], &a_s[buf][(warp_m * WM + i) * 16 + (lane % 16)][ks * 16 + (lane / 16) * 8]);
+      uint32_t af[4];
+      ldmatrix_x4(af, &a_s[buf][warp * 16 + (lane % 16)][ks * 16 + (lane / 16) * 8]);
 #pragma unroll
       for (int j2 = 0; j2 < RM_COLS / 16; ++j2) {
         uint32_t b[4];
-        ldmatrix_x4(b, &w_s[buf][warp_n * RM_COLS + j2 * 16 + (lane % 8) + (lane / 16) * 8][ks * 16 + ((lane / 8) % 2) * 8]);
-#pragma unroll
-        for (int i = 0; i < WM; ++i) {
-          mma_bf16(acc[i][2 * j2], af[i], b[0], b[1]);
-          mma_bf16(acc[i][2 * j2 + 1], af[i], b[2], b[3]);
-        }
+        ldmatrix_x4(b, &w_s[buf][j2 * 16 + (lane % 8) + (lane / 16) * 8][ks * 16 + ((lane / 8) % 2) * 8]);
+        mma_bf16(acc[2 * j2], af, b[0], b[1]);
+        mma_bf16(acc[2 * j2 + 1], af, b[2], b[3]);
       }
     }
   }
   cp_async_wait<0>();
 #pragma unroll
-  for (int i = 0; i < WM; ++i) {
+  for (int half = 0; half < 2; ++half) {
+    const int pair = rows_s[warp * 16 + lane / 4 + half * 8];
+    if (pair < 0) continue;
+    const float sc = ((EPI == 1 || EPI == 3) && share) ? share[pair] : 1.0f;
+    TO* dst = out + (size_t)pair * ldo;
 #pragma unroll
-    for (int half = 0; half < 2; ++half) {
-      const int pair = rows_s[(warp_m * WM + i) * 16 + lane / 4 + half * 8];
-      if (pair < 0) continue;
-      const float sc = ((EPI == 1 || EPI == 3) && share) ? share[pair] : 1.0f;
-      TO* dst = out + (size_t)pair * ldo;
+    for (int j = 0; j < RM_COLS / 8; ++j) {
 #pragma unroll
-      for (int j = 0; j < RM_COLS / 8; ++j) {
-#pragma unroll
-        for (int el = 0; el < 2; ++el) {
-          const int n = n0 + warp_n * RM_COLS + j * 8 + 2 * (lane % 4) + el;
-          if (n >= N) continue;
-          float v = acc[i][j][2 * half + el];
-          if (EPI == 2) {  // the thread holds a gate column and, right of it, its up column
-            if (el == 0) {
-              const float u = acc[i][j][2 * half + 1];
-              dst[n / 2] = from_f32<TO>(gated_value(v, u, act, p0, p1));
-            }
-            continue;
+      for (int el = 0; el < 2; ++el) {
+        const int n = n0 + j * 8 + 2 * (lane % 4) + el;
+        if (n >= N) continue;
+        float v = acc[j][2 * half + el];
+        if (EPI == 2) {  // the thread holds a gate column and, right of it, its up column
+          if (el == 0) {
+            const float u = acc[j][2 * half + 1];
+            dst[n / 2] = from_f32<TO>(gated_value(v, u, act, p0, p1));
           }
-          if (EPI == 0) v = 0.5f * v * (1.0f + erff(v * 0.70710678118654752440f));
-          else v *= sc;
-          if (EPI == 3) {
-            v = fmaxf(v, 0.f);
-            v *= v;
-          }
-          dst[n] = from_f32<TO>(v);
+          continue;
         }
+        if (EPI == 0) v = 0.5f * v * (1.0f + erff(v * 0.70710678118654752440f));
+        else v *= sc;
+        if (EPI == 3) {
+          v = fmaxf(v, 0.f);
+          v *= v;
+        }
+        dst[n] = from_f32<TO>(v);
       }
     }
   }
@@ -308,31 +296,29 @@ __global__ void __launch_bounds__(RM_THREADS)
 
 }  // namespace
 
-// Rows of a tile: 64; 128 when an expert gets about that many rows or more; 16 when it gets a few.
-extern "C" int llm_routed_product_mma_rows(int rows_per_expert) {
-  return rows_per_expert >= 96 ? 2 * RM_ROWS : (rows_per_expert <= 8 ? RS_ROWS : RM_ROWS);
-}
+// Rows of a tile: 64; 16 when an expert gets a few.
+extern "C" int llm_routed_product_mma_rows(int rows_per_expert) { return rows_per_expert <= 8 ? RS_ROWS : RM_ROWS; }
 
 // Whether the tensor-core kernel takes these operands: 16-byte aligned rows of K % 8 == 0.
 extern "C" int llm_routed_product_mma_supported(const void* a, long long lda, const void* w, int K) {
   return K > 0 && K % 8 == 0 && lda % 8 == 0 && (reinterpret_cast<uintptr_t>(a) & 15u) == 0 && (reinterpret_cast<uintptr_t>(w) & 15u) == 0;
 }
 
-template <typename TO, int EPI, int WM>
+template <typename TO, int EPI>
 int launch_routed(dim3 grid, cudaStream_t stream, const void* a, long long lda, int a_div, const void* w, long long ws, int N, int K,
                   const int* tile_expert, const int* tile_rows, void* out, long long ldo, const float* share, int act, float p0, float p1) {
   static bool raised = false;
   if (!raised) {
-    if (cudaFuncSetAttribute(routed_product_mma_kernel<TO, EPI, WM>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(RM_SMEM * WM)) != cudaSuccess)
+    if (cudaFuncSetAttribute(routed_product_mma_kernel<TO, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)RM_SMEM) != cudaSuccess)
       return 1;
     raised = true;
   }
-  launch_kernel(routed_product_mma_kernel<TO, EPI, WM>, grid, RM_THREADS * WM, RM_SMEM * WM, stream, (const bf16*)a, lda, a_div, (const bf16*)w,
+  launch_kernel(routed_product_mma_kernel<TO, EPI>, grid, RM_THREADS, RM_SMEM, stream, (const bf16*)a, lda, a_div, (const bf16*)w,
                 ws, N, K, tile_expert, tile_rows, (TO*)out, ldo, share, act, p0, p1);
   return 0;
 }
 
-// tile: the rows of a tile of tile_rows (64 or 128, as llm_routed_product_mma_rows said when the pairs were grouped).
+// tile: the rows of a tile of tile_rows (16 or 64, as llm_routed_product_mma_rows said when the pairs were grouped).
 extern "C" int llm_routed_product_mma(const void* a, long long lda, int a_div, const void* w, int N, int K, const int* tile_expert,
                                       const int* tile_rows, int max_tiles, int tile, void* out, long long ldo, int epilogue,
                                       const float* share, int act, float p0, float p1, cudaStream_t stream) {
@@ -341,7 +327,7 @@ extern "C" int llm_routed_product_mma(const void* a, long long lda, int a_div, c
   LLM_REQUIRE(act >= 0 && act <= 2, "routed_product_mma: unknown activation %d", act);
   LLM_REQUIRE(llm_routed_product_mma_supported(a, lda, w, K), "routed_product_mma: operands must be 16-byte aligned with K and the row stride multiples of 8");
   LLM_REQUIRE(N > 0 && a_div > 0 && max_tiles > 0 && max_tiles <= 65535, "routed_product_mma: bad sizes");
-  LLM_REQUIRE(tile == RS_ROWS || tile == RM_ROWS || tile == 2 * RM_ROWS, "routed_product_mma: tiles of %d rows (16, 64 or 128)", tile);
+  LLM_REQUIRE(tile == RS_ROWS || tile == RM_ROWS, "routed_product_mma: tiles of %d rows (16 or 64)", tile);
   LLM_REQUIRE(epilogue == 0 || epilogue == 1 || epilogue == 3 || (epilogue == 2 && N % 2 == 0), "routed_product_mma: unknown epilogue %d", epilogue);
   if (tile == RS_ROWS) {
     static bool raised_few = false;
@@ -370,22 +356,17 @@ extern "C" int llm_routed_product_mma(const void* a, long long lda, int a_div, c
     LLM_CHECK_LAUNCH("routed_product_mma");
     return LLM_OK;
   }
-  const int wm = tile / RM_ROWS;
-  dim3 grid(ceil_div(N, RM_COLS * wm), max_tiles);
+  dim3 grid(ceil_div(N, RM_COLS), max_tiles);
   const long long ws = (long long)N * K;
   int rc;
   if (epilogue == 0)
-    rc = wm == 2 ? launch_routed<bf16, 0, 2>(grid, stream, a, lda, a_div, w, ws, N, K, tile_expert, tile_rows, out, ldo, share, act, p0, p1)
-                 : launch_routed<bf16, 0, 1>(grid, stream, a, lda, a_div, w, ws, N, K, tile_expert, tile_rows, out, ldo, share, act, p0, p1);
+    rc = launch_routed<bf16, 0>(grid, stream, a, lda, a_div, w, ws, N, K, tile_expert, tile_rows, out, ldo, share, act, p0, p1);
   else if (epilogue == 2)
-    rc = wm == 2 ? launch_routed<bf16, 2, 2>(grid, stream, a, lda, a_div, w, ws, N, K, tile_expert, tile_rows, out, ldo, share, act, p0, p1)
-                 : launch_routed<bf16, 2, 1>(grid, stream, a, lda, a_div, w, ws, N, K, tile_expert, tile_rows, out, ldo, share, act, p0, p1);
+    rc = launch_routed<bf16, 2>(grid, stream, a, lda, a_div, w, ws, N, K, tile_expert, tile_rows, out, ldo, share, act, p0, p1);
   else if (epilogue == 3)
-    rc = wm == 2 ? launch_routed<bf16, 3, 2>(grid, stream, a, lda, a_div, w, ws, N, K, tile_expert, tile_rows, out, ldo, share, act, p0, p1)
-                 : launch_routed<bf16, 3, 1>(grid, stream, a, lda, a_div, w, ws, N, K, tile_expert, tile_rows, out, ldo, share, act, p0, p1);
+    rc = launch_routed<bf16, 3>(grid, stream, a, lda, a_div, w, ws, N, K, tile_expert, tile_rows, out, ldo, share, act, p0, p1);
   else
-    rc = wm == 2 ? launch_routed<float, 1, 2>(grid, stream, a, lda, a_div, w, ws, N, K, tile_expert, tile_rows, out, ldo, share, act, p0, p1)
-                 : launch_routed<float, 1, 1>(grid, stream, a, lda, a_div, w, ws, N, K, tile_expert, tile_rows, out, ldo, share, act, p0, p1);
+    rc = launch_routed<float, 1>(grid, stream, a, lda, a_div, w, ws, N, K, tile_expert, tile_rows, out, ldo, share, act, p0, p1);
   LLM_REQUIRE(rc == 0, "routed_product_mma: cannot raise the shared memory limit");
   LLM_CHECK_LAUNCH("routed_product_mma");
   return LLM_OK;

@@ -1185,7 +1185,7 @@ class CudaOps:
 
     def routed_tile_rows(self, n_tokens: int = 0, dtype: Optional[torch.dtype] = None, inner=(), per_expert: float = 0.0) -> int:
         """Rows of a tile of the per-expert products: the tensor-core kernel's in bfloat16 when every product's inner
-        size (`inner`) is a multiple of 8 (64, or 128 when an expert gets about that many rows: `per_expert`), else the
+        size (`inner`) is a multiple of 8 (64, or 16 when an expert gets a few: `per_expert`), else the
         CUDA-core kernel's."""
         if dtype == torch.bfloat16 and self.tensor_cores and self.routed_tensor_cores and inner and all(k % 8 == 0 for k in inner):
             return int(self.lib("tensorcore").llm_routed_product_mma_rows(c_int(int(per_expert))))
@@ -1263,7 +1263,7 @@ class CudaOps:
         if share is not None:
             _need(share, "routed_product.share", torch.float32)
         if a.dtype == torch.bfloat16 and self.tensor_cores and tile_rows.shape[1] != self.routed_tile_rows():
-            lib = self.lib("tensorcore")  # tiles made for the tensor-core kernel (64 or 128 rows)
+            lib = self.lib("tensorcore")  # tiles made for the tensor-core kernel (16 or 64 rows)
             assert out.dtype == (torch.float32 if epilogue == "share" else torch.bfloat16)
             self._check(lib.llm_routed_product_mma(_ptr(a), c_longlong(a.stride(0)), c_int(a_div), _ptr(w), c_int(N), c_int(K),
                                                    _ptr(tile_expert), _ptr(tile_rows), c_int(tile_expert.numel()),
