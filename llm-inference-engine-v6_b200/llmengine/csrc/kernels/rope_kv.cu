@@ -11,6 +11,13 @@
 // request is block_table[request_row][p / page_size].
 #include "common.cuh"
 
+// One rotation pair. Which product is rounded before the sum is said here, not left to the compiler, which chose differently in two forms
+// of the same kernel: a last bit of k that differs between them is cached, and shows in every later step.
+__device__ __forceinline__ void rotate_pair(float a, float b, float c, float s, float& ra, float& rb) {
+  ra = __fmaf_rn(a, c, -__fmul_rn(b, s));
+  rb = __fmaf_rn(b, c, __fmul_rn(a, s));
+}
+
 // With `parts` (float32 [n_parts, tokens, width] partial sums of the q|k|v product) the values are
 // the sums over parts in index order and only the q section of qkv is written.
 //
@@ -91,8 +98,7 @@ __global__ void __launch_bounds__(128)
   float ra = a, rb = b;
   if (cos_t) {
     const float c = cos_t[(size_t)pos * half + i], s = sin_t[(size_t)pos * half + i];
-    ra = a * c - b * s;
-    rb = b * c + a * s;
+    rotate_pair(a, b, c, s, ra, rb);
   }
   const T oa = from_f32<T>(ra), ob = from_f32<T>(rb);
   if (head < nq || !kcache) {
@@ -190,11 +196,7 @@ __global__ void __launch_bounds__(128)
     *reinterpret_cast<float4*>(sn) = s4[0];
     *reinterpret_cast<float4*>(sn + 4) = s4[1];
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const float av = fa[j], bv = fb[j];
-      fa[j] = av * c[j] - bv * sn[j];
-      fb[j] = bv * c[j] + av * sn[j];
-    }
+    for (int j = 0; j < 8; ++j) rotate_pair(fa[j], fb[j], c[j], sn[j], fa[j], fb[j]);
   }
   a.u = pack8(fa);
   b.u = pack8(fb);

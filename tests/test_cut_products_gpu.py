@@ -102,3 +102,32 @@ def test_rotation_of_parts_forms_agree(ops, parts, n, nq, nkv, hd, page, rotate)
         got.append((qkv[:, :nq * hd], k, v))
     for a, b in zip(*got):
         torch.testing.assert_close(a, b, rtol=2.0 ** -7, atol=1e-6)
+
+
+@pytest.mark.parametrize("form", ["16 bytes", "a pair a thread", "float32", "parts, 16 bytes", "parts, a pair a thread"])
+def test_every_form_of_the_rotation_rounds_alike(ops, form):
+    """x c - y s and y c + x s with the second product rounded before the sum, as float64 gives it bit for bit, in q and in the cached k: a
+    prompt's keys must not depend on which form a step of its size runs."""
+    n, nq, nkv, hd, page = 300, 6, 2, 64, 16
+    dt = torch.float32 if form == "float32" else torch.bfloat16
+    width, half = (nq + 2 * nkv) * hd, hd // 2
+    x = rnd(n, width, seed=21, dt=torch.float32)
+    parts = x[None].clone() if "parts" in form else None
+    qkv = torch.zeros(n, width, dtype=dt, device=DEV) if parts is not None else x.to(dt)
+    if "pair" in form:  # an address that is no multiple of 16
+        src = parts if parts is not None else qkv
+        odd = torch.empty(src.numel() + 1, dtype=src.dtype, device=DEV)[1:].view(src.shape)
+        odd.copy_(src)
+        parts, qkv = (odd, qkv) if parts is not None else (None, odd)
+    values = (x if parts is not None else qkv.float()).clone()
+    angle = torch.arange(n, dtype=torch.float64)[:, None] * torch.logspace(0, -3, half, dtype=torch.float64)[None]
+    cos, sin = angle.cos().float().to(DEV), angle.sin().float().to(DEV)
+    pos, seq = torch.arange(n, dtype=torch.int32, device=DEV), torch.zeros(n, dtype=torch.int32, device=DEV)
+    table = torch.arange(-(-n // page), dtype=torch.int32, device=DEV).view(1, -1)
+    k, v = (torch.zeros(table.numel() + 1, nkv, page, hd, dtype=dt, device=DEV) for _ in range(2))
+    ops.rope_kv_write(qkv, pos, seq, table, cos, sin, k, v, n, nq, nkv, hd, parts=parts)
+    y = values[:, :(nq + nkv) * hd].reshape(n, nq + nkv, hd)
+    a, b, c, s = y[..., :half].double(), y[..., half:].double(), cos[:, None].double(), sin[:, None].double()
+    want = torch.cat([(a * c - (b * s).float().double()).float(), (b * c + (a * s).float().double()).float()], -1).to(dt)
+    assert torch.equal(qkv[:, :nq * hd].reshape(n, nq, hd), want[:, :nq])
+    assert torch.equal(k[:-1].transpose(1, 2).reshape(-1, nkv, hd)[:n], want[:, nq:])
