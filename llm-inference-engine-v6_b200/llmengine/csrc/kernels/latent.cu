@@ -85,28 +85,24 @@ __global__ void latent_prep_kernel(const float* __restrict__ parts, int n_parts,
   }
 }
 
-// The same for prompt-sized steps, whose product comes as one part: a warp a token, its numbers in registers as groups of four
-// (QN groups a lane of the query latent, KN of the cached row), so that all loads of a token are in flight at once and the two sums
-// of squares are a warp's. The rotated part goes through shared memory, where a pair's partner is. 2,048 tokens, 768 + 512 + 64
-// numbers: 5.0 us; 22 as a block a token.
+// The same for bfloat16 steps of a prompt's size, whose product comes as one part: a warp a token, its numbers in registers as groups
+// of four (QN groups a lane of the query latent, KN of the cached row), so that all loads of a token are in flight at once and the two
+// sums of squares are a warp's. The rotated part goes through shared memory, where a pair's partner is. 2,048 tokens, 768 + 512 + 64
+// numbers: 5.0 us; 22 as a block a token. Its sums of squares are added in another order than the block's. In float32, where a token's
+// bits must not depend on the step it came in, every step runs the block's.
 constexpr int PREP_WARPS = 4, PREP_ROT = 256;
 
-template <typename T>
-__device__ __forceinline__ void store4(T* p, float4 v);
-template <>
-__device__ __forceinline__ void store4<float>(float* p, float4 v) { *reinterpret_cast<float4*>(p) = v; }
-template <>
-__device__ __forceinline__ void store4<bf16>(bf16* p, float4 v) {
+__device__ __forceinline__ void store4(bf16* p, float4 v) {
   __nv_bfloat162 lo = __floats2bfloat162_rn(v.x, v.y), hi = __floats2bfloat162_rn(v.z, v.w);
   *reinterpret_cast<uint2*>(p) = make_uint2(*reinterpret_cast<uint32_t*>(&lo), *reinterpret_cast<uint32_t*>(&hi));
 }
 
-template <typename T, int QN, int KN>
+template <int QN, int KN>
 __global__ void __launch_bounds__(PREP_WARPS * 32)
     latent_prep_warp_kernel(const float* __restrict__ sums, int width, int q_off, int Rq, int kv_off, int R, int dr, int rot_dims,
                             const float* __restrict__ wq, const float* __restrict__ wkv, float eps, const float* __restrict__ cos_t,
                             const float* __restrict__ sin_t, const int* __restrict__ positions, const int* __restrict__ token_seq,
-                            const int* __restrict__ block_table, int max_blocks, T* __restrict__ cq, long long ld_cq, T* __restrict__ cache,
+                            const int* __restrict__ block_table, int max_blocks, bf16* __restrict__ cq, long long ld_cq, bf16* __restrict__ cache,
                             int page_size, int n_tokens) {
   __shared__ float rot[PREP_WARPS][PREP_ROT];
   dep_launch();
@@ -134,25 +130,25 @@ __global__ void __launch_bounds__(PREP_WARPS * 32)
   ssq = warp_sum(ssq);
   ssk = warp_sum(ssk);
   const float iq = 1.0f / sqrtf(ssq / (float)Rq + eps);
-  T* q_out = cq + (size_t)tok * ld_cq;
+  bf16* q_out = cq + (size_t)tok * ld_cq;
 #pragma unroll
   for (int i = 0; i < QN; ++i) {
     const int c = 4 * (32 * i + lane);
     if (c < Rq) {
       const float4 w = *reinterpret_cast<const float4*>(wq + c);
-      store4<T>(q_out + c, make_float4(q[i].x * iq * w.x, q[i].y * iq * w.y, q[i].z * iq * w.z, q[i].w * iq * w.w));
+      store4(q_out + c, make_float4(q[i].x * iq * w.x, q[i].y * iq * w.y, q[i].z * iq * w.z, q[i].w * iq * w.w));
     }
   }
   if (cache == nullptr) return;
   const float ik = 1.0f / sqrtf(ssk / (float)R + eps);
   const int pos = positions[tok], page = block_table[(size_t)token_seq[tok] * max_blocks + pos / page_size];
-  T* dst = cache + ((size_t)page * page_size + (size_t)(pos % page_size)) * (size_t)(R + dr);
+  bf16* dst = cache + ((size_t)page * page_size + (size_t)(pos % page_size)) * (size_t)(R + dr);
 #pragma unroll
   for (int i = 0; i < KN; ++i) {
     const int c = 4 * (32 * i + lane);
     if (c < R) {
       const float4 w = *reinterpret_cast<const float4*>(wkv + c);
-      store4<T>(dst + c, make_float4(k[i].x * ik * w.x, k[i].y * ik * w.y, k[i].z * ik * w.z, k[i].w * ik * w.w));
+      store4(dst + c, make_float4(k[i].x * ik * w.x, k[i].y * ik * w.y, k[i].z * ik * w.z, k[i].w * ik * w.w));
     } else if (c < R + dr) {
       *reinterpret_cast<float4*>(&rot[warp][c - R]) = k[i];
     }
@@ -164,12 +160,11 @@ __global__ void __launch_bounds__(PREP_WARPS * 32)
     float v = kr[i];
     if (i < half) v = kr[i] * cos_t[(size_t)pos * half + i] - kr[i + half] * sin_t[(size_t)pos * half + i];
     else if (i < rot_dims) v = kr[i] * cos_t[(size_t)pos * half + i - half] + kr[i - half] * sin_t[(size_t)pos * half + i - half];
-    dst[R + i] = from_f32<T>(v);
+    dst[R + i] = from_f32<bf16>(v);
   }
 }
 
 // Whether every row begins on 16 bytes (results: 4 numbers) and fits the registers of a warp.
-template <typename T>
 bool prep_by_warps(const void* sums, int n_parts, int width, int q_off, int Rq, int kv_off, int R, int dr, const float* wq, const float* wkv, const void* cq,
                    long long ld_cq, const void* cache, int n_tokens) {
   const int all = width | q_off | Rq | kv_off | R | dr | (int)(ld_cq & 3);
@@ -439,14 +434,11 @@ extern "C" int llm_latent_prep(const float* parts, int n_parts, long long pstrid
   LLM_REQUIRE(rot_dims == 0 || (cos_t && sin_t), "latent_prep: rotation tables missing");
   const size_t smem = (size_t)(Rq + R + dr) * sizeof(float);
   LLM_REQUIRE(smem <= 48 * 1024, "latent_prep: latent sizes %d + %d + %d exceed one block's shared memory", Rq, R, dr);
-  if (dtype == LLM_F32 && prep_by_warps<float>(parts, n_parts, width, q_off, Rq, kv_off, R, dr, wq, wkv, cq, ld_cq, cache, n_tokens))
-    launch_kernel(latent_prep_warp_kernel<float, 8, 5>, ceil_div(n_tokens, PREP_WARPS), PREP_WARPS * 32, 0, stream, parts, width, q_off, Rq, kv_off, R, dr,
-                  rot_dims, wq, wkv, eps, cos_t, sin_t, positions, token_seq, block_table, max_blocks, (float*)cq, ld_cq, (float*)cache, page_size, n_tokens);
-  else if (dtype == LLM_F32)
+  if (dtype == LLM_F32)
     launch_kernel(latent_prep_kernel<float>, n_tokens, 256, smem, stream, parts, n_parts, (size_t)pstride, width, q_off, Rq, kv_off, R, dr,
                   rot_dims, wq, wkv, eps, cos_t, sin_t, positions, token_seq, block_table, max_blocks, (float*)cq, ld_cq, (float*)cache, page_size);
-  else if (dtype == LLM_BF16 && prep_by_warps<bf16>(parts, n_parts, width, q_off, Rq, kv_off, R, dr, wq, wkv, cq, ld_cq, cache, n_tokens))
-    launch_kernel(latent_prep_warp_kernel<bf16, 8, 5>, ceil_div(n_tokens, PREP_WARPS), PREP_WARPS * 32, 0, stream, parts, width, q_off, Rq, kv_off, R, dr,
+  else if (dtype == LLM_BF16 && prep_by_warps(parts, n_parts, width, q_off, Rq, kv_off, R, dr, wq, wkv, cq, ld_cq, cache, n_tokens))
+    launch_kernel(latent_prep_warp_kernel<8, 5>, ceil_div(n_tokens, PREP_WARPS), PREP_WARPS * 32, 0, stream, parts, width, q_off, Rq, kv_off, R, dr,
                   rot_dims, wq, wkv, eps, cos_t, sin_t, positions, token_seq, block_table, max_blocks, (bf16*)cq, ld_cq, (bf16*)cache, page_size, n_tokens);
   else if (dtype == LLM_BF16)
     launch_kernel(latent_prep_kernel<bf16>, n_tokens, 256, smem, stream, parts, n_parts, (size_t)pstride, width, q_off, Rq, kv_off, R, dr,

@@ -38,3 +38,27 @@ def test_warps_and_blocks_agree(ops, dt, n, Rq, R, dr, rot):
     tol = dict(rtol=2e-6, atol=1e-6) if dt == torch.float32 else dict(rtol=2.0 ** -7, atol=1e-6)
     for x, y in zip(*got):
         torch.testing.assert_close(x, y, **tol)
+
+
+@pytest.mark.parametrize("Rq,R,dr,rot", [(768, 512, 64, 64), (4, 4, 4, 2), (132, 260, 12, 0)])
+def test_float32_rows_do_not_depend_on_the_step(ops, Rq, R, dr, rot):
+    """The same float32 tokens in steps of 1, 64, 65 and 131: the same bits."""
+    page, n, g = 16, 131, torch.Generator().manual_seed(5)
+    table = torch.randperm(-(-n // page), generator=g).to(torch.int32).view(1, -1).to(DEV)
+    sums = torch.randn(n, Rq + R + dr, generator=g).to(DEV)
+    wq, wk = torch.rand(Rq, generator=g).to(DEV) + 0.5, torch.rand(R, generator=g).to(DEV) + 0.5
+    angle = torch.arange(n)[:, None] * torch.logspace(0, -2, max(rot // 2, 1))[None]
+    cos, sin = (angle.cos().to(DEV), angle.sin().to(DEV)) if rot else (None, None)
+
+    def run(step):
+        cq = torch.empty(n, Rq, device=DEV)
+        cache = torch.zeros(table.numel() + 1, 1, page, R + dr, device=DEV)
+        for at in range(0, n, step):
+            m = min(step, n - at)
+            ops.latent_prep(sums[at:at + m].clone()[None], 0, Rq, Rq, R, dr, rot, wq, wk, 1e-5, cos, sin, Batch([(at, m)]), table, cq[at:at + m], cache)
+        return cq, cache
+
+    want = run(131)
+    for step in (1, 64, 65):
+        for x, y in zip(run(step), want):
+            assert torch.equal(x, y), step
