@@ -38,11 +38,12 @@ struct AttArgs {
   float scale;
 };
 
-// acc and l of the segments so far, with the largest score m, joined with those of one more segment
+// acc and l of the segments so far, with the largest score m, joined with those of one more segment. A largest score of -inf does not
+// say that a segment holds nothing: NaNs are passed over by a maximum and stay in l and the sums, which keep them whatever their weight.
 __device__ __forceinline__ void join_weights(float m, float m_s, float& m_new, float& a, float& b) {
   m_new = fmaxf(m, m_s);
   a = m == -INFINITY ? 0.f : expf(m - m_new);
-  b = expf(m_s - m_new);
+  b = m_s == -INFINITY ? 0.f : expf(m_s - m_new);
 }
 __device__ __forceinline__ float join(float x, float a, float x_s, float b) { return fmaf(x, a, __fmul_rn(x_s, b)); }
 
@@ -249,10 +250,9 @@ __global__ void __launch_bounds__((KT / KM) * (ROWS / RM))
     }
 #pragma unroll
     for (int j = 0; j < RM; ++j) {
-      const float m_s = s_m[ty * RM + j];
-      if (m_s == -INFINITY) continue;  // the row sees no key of this segment
+      if (k0 > pos_of[j] || (p.window > 0 && k0 + SEG - 1 <= pos_of[j] - p.window)) continue;  // the row sees no key of this segment
       float m_new, a, b;
-      join_weights(m_run[j], m_s, m_new, a, b);
+      join_weights(m_run[j], s_m[ty * RM + j], m_new, a, b);
       m_run[j] = m_new;
       l_run[j] = join(l_run[j], a, s_l[ty * RM + j], b);
 #pragma unroll
@@ -294,7 +294,6 @@ __global__ void __launch_bounds__(128) paged_attention_simt_merge_kernel(const A
   for (int s = first; s <= pos / SEG; ++s) {
     const float* o = from + (size_t)s * (p.hd + 2);
     const float m_s = o[p.hd], l_s = o[p.hd + 1];
-    if (m_s == -INFINITY) continue;
     float m_new, a, b;
     join_weights(m, m_s, m_new, a, b);
     m = m_new;

@@ -54,3 +54,57 @@ def test_values_behind_a_token_do_not_reach_it(ops):
         ops.paged_attention(q, kc, vc, Batch([(0, 100)]), table, out, 8, 2, 64, 0.125)
         outs.append(out)
     assert torch.equal(outs[0][:70], outs[1][:70]) and bool(outs[1][70:].isnan().all())
+
+
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+@pytest.mark.parametrize("where", [127, 128, 129, 255, 256])
+@pytest.mark.parametrize("window", [0, 130])
+def test_a_key_that_is_no_number_reaches_every_token_that_sees_it(ops, bad, where, window):
+    """NaN (and +-inf, by a query's signs: -inf is a probability of zero, +inf has none) in the key at `where`, which alone may be what a
+    token sees of a segment of 128: a token on its own (a CTA a segment), a portion, and whole prompts beside many (one CTA walks).
+    Tokens before it, and those whose window has left it behind, keep their bits."""
+    nq, nkv, hd, page, others, length, scale = 8, 2, 64, 16, 40, 300, 0.125
+    kc, vc, table, _ = _paged_setup(torch.float32, nkv, hd, page, [length] * others, others * 19 + 2, seed=3)
+    q = torch.randn(others, length, nq * hd, generator=torch.Generator().manual_seed(9)).to(DEV)
+    q[0, :, ::hd] = q[0, :, ::hd].abs() + 0.1  # (the first number of every head: an infinite key scores +inf there)
+
+    def run(entries):
+        rows = torch.cat([q[i, s:s + n] for i, (s, n) in enumerate(entries)])
+        out = torch.empty_like(rows)
+        ops.paged_attention(rows, kc, vc, Batch(entries), table[:len(entries)].contiguous(), out, nq, nkv, hd, scale, window)
+        return out
+
+    clean = run([(0, length)] * others)[:length]
+    kc[table[0, where // page], :, where % page, 0] = bad
+    whole = run([(0, length)] * others)[:length]
+    portion = torch.cat([run([(at, min(50, length - at))]) for at in range(0, length, 50)])
+    alone = torch.cat([run([(t, 1)]) for t in range(length)])
+    sees = torch.arange(length) >= where
+    if window:
+        sees &= torch.arange(length) < where + window
+    for got in (whole, portion, alone):
+        assert bool(got[sees].isnan().all()) and torch.equal(got[~sees], clean[~sees])
+
+
+def test_keys_of_minus_infinity_weigh_nothing(ops):
+    """Scores of -inf, alone in a token's last segment and alone in its first: as if the keys were not there."""
+    nq, nkv, hd, page, length, scale = 8, 2, 64, 16, 260, 0.125
+    kc, vc, table, dense = _paged_setup(torch.float32, nkv, hd, page, [length], 19, seed=4)
+    q = torch.randn(length, nq * hd, generator=torch.Generator().manual_seed(9)).to(DEV)
+    q[:, ::hd] = q[:, ::hd].abs() + 0.1
+    for dead in (range(128, 129), range(0, 128)):
+        keys = kc.clone()
+        for t in dead:
+            keys[table[0, t // page], :, t % page, 0] = float("-inf")
+        K, V = dense[0]
+        K = K.clone()
+        K[list(dead), :, 0] = float("-inf")
+        first = dead.stop if dead.start == 0 else 0
+        whole = torch.empty_like(q)
+        ops.paged_attention(q, keys, vc, Batch([(0, length)]), table, whole, nq, nkv, hd, scale)
+        for t in (max(first, 128), 200, 259):
+            alone = torch.empty(1, nq * hd, device=DEV)
+            ops.paged_attention(q[t:t + 1], keys, vc, Batch([(t, 1)]), table, alone, nq, nkv, hd, scale)
+            assert torch.equal(alone[0], whole[t])
+            ref = _attention_ref(q[t].view(nq, hd).cpu().double(), K.double(), V.double(), t, nq, nkv, hd, scale, 0)
+            torch.testing.assert_close(alone[0].cpu(), ref.float(), rtol=2e-5, atol=2e-5)
