@@ -79,6 +79,42 @@ def test_silu_mul_partials_forms_agree(ops, parts, rows, ff, block, act):
         assert torch.equal(a, b)
 
 
+@pytest.mark.parametrize("act", ["silu", "gelu_tanh", ("clamped_swish", 1.5, 1.7)])
+@pytest.mark.parametrize("parts,rows,ff,block", [(5, 64, 2432, 128), (3, 61, 2500, 0), (4, 40, 4096, 128), (1, 300, 516, 0), (9, 37, 4100, 4), (2, 592, 256, 128)])
+def test_silu_mul_partials_four_columns_at_a_time(ops, parts, rows, ff, block, act):
+    """From 148 * 1,024 results on (rows * ff) and on 16 bytes a thread takes four columns: against float64, with and without a row scale, and
+    against the bits of a column at a time (parts on an address that is no multiple of 16). The error: `parts` additions and a handful of
+    further operations, each 2^-24 of the halves' absolute sums, of which the activation passes on at most 1.2 times (its slope)."""
+    assert rows * ff >= 148 * 1024 and ff % 4 == 0 and block % 4 == 0
+    p = rnd(parts, rows, 2 * ff, seed=14, dt=torch.float32)
+    odd = torch.empty(p.numel() + 1, device=DEV)[1:].view(p.shape)
+    odd.copy_(p)
+    sumsq = torch.rand(rows, 3, generator=torch.Generator().manual_seed(15)).to(DEV) + 0.5
+    for scaled in (False, True):
+        extra = {"row_scale": ops.row_scale(sumsq, 2, 1e-5)} if scaled else {}
+        sc = 1.0 / torch.sqrt(sumsq.double().sum(1, keepdim=True) / 2 + 1e-5) if scaled else 1.0
+        both, size = p.double().sum(0) * sc, p.double().abs().sum(0) * sc
+        if block:
+            g, u = both.view(rows, -1, 2, block)[:, :, 0].reshape(rows, ff), both.view(rows, -1, 2, block)[:, :, 1].reshape(rows, ff)
+            gs, us = size.view(rows, -1, 2, block)[:, :, 0].reshape(rows, ff), size.view(rows, -1, 2, block)[:, :, 1].reshape(rows, ff)
+        else:
+            g, u, gs, us = both[:, :ff], both[:, ff:], size[:, :ff], size[:, ff:]
+        if act == "silu":
+            want, slope = g * torch.sigmoid(g) * u, 1.1
+        elif act == "gelu_tanh":
+            want, slope = torch.nn.functional.gelu(g, approximate="tanh") * u, 1.2
+        else:
+            g = torch.clamp(g, max=act[1])
+            want, slope = g * torch.sigmoid(act[2] * g) * (torch.clamp(u, -act[1], act[1]) + 1), 1.2
+        bound = (parts + 12) * 2.0 ** -24 * slope * (gs * (us + 1) + (gs + 1) * us + gs)
+        for dt in (torch.float32, torch.bfloat16):
+            a, b = torch.empty(rows, ff, dtype=dt, device=DEV), torch.empty(rows, ff, dtype=dt, device=DEV)
+            ops.silu_mul_partials(p, a, block=block, act=act, **extra)
+            ops.silu_mul_partials(odd, b, block=block, act=act, **extra)
+            assert torch.equal(a, b)
+            assert bool(((a.double() - want).abs() <= bound + (0 if dt == torch.float32 else 2.0 ** -8) * want.abs()).all())
+
+
 @pytest.mark.parametrize("parts,n,nq,nkv,hd,page", [(1, 65, 4, 2, 64, 16), (3, 77, 6, 1, 128, 4), (6, 200, 2, 2, 16, 8)])
 @pytest.mark.parametrize("rotate", [True, False])
 def test_rotation_of_parts_forms_agree(ops, parts, n, nq, nkv, hd, page, rotate):
