@@ -99,3 +99,56 @@ def test_what_is_expanded(ops):
     for seqs, want in (([(0, 128)], 128), ([(0, 127)], 0), ([(2000, 300)], 2304), ([(0, 256), (700, 1), (800, 1), (900, 1), (3, 1), (5, 1)], 0),
                        ([(32768 - 128, 128)], 32768), ([(32768 - 127, 128)], 0)):
         assert ops.latent_expanded_rows(Batch(seqs)) == want
+
+
+def _wide_config():
+    """Vapelix with heads that the expanded form takes: 64 numbers beside a rotated part of 32 in a layer that runs twice, and 128 beside 64
+    of which 48 are rotated; every expert is chosen, so that no rounding changes a choice."""
+    from tiny_vapelix import _mixer, _moe
+    a = _mixer(3, 64, 32, 64, 64, 40, 0.12, 10000.0, {"factor": 4.0, "original": 64, "fast": 32.0, "slow": 1.0})
+    b = _mixer(2, 128, 64, 128, 128, 72, 0.07, 50000.0, dims=48)
+    return {"architecture": "Vapelix", "vocab": 301, "width": 128, "norm": {"eps": 1e-6}, "max_positions": 1024,
+            "layers": [{"type": "latent_attention", "mixer": a, "mlp": {"kind": "dense", "ff": 256}},
+                       {"type": "latent_attention", "mixer": b, "mlp": _moe(64, 3, 3)}],
+            "loop": {"start": 0, "stop": 1, "times": 2}, "token_side": {"dim": 16}}
+
+
+@pytest.mark.parametrize("sharp", [False, True])
+def test_whole_model_through_expanded_steps(tmp_path, monkeypatch, ops, sharp):
+    """A prompt, its second portion beside other requests' single tokens and beside a second prompt, then decoding over the rows that those
+    steps wrote, against the plain implementation; sharp: most heads rest on one or two keys, so that a lost or misplaced one shows."""
+    import llmengine
+    import numpy as np
+    import plain_vapelix as P
+    from test_vapelix_gpu import replay, rows_close, sharp_model_dir
+    from tiny import Trace, make_model_dir, random_ids
+    cfg = _wide_config()
+    d = str(tmp_path / "m")
+    sharp_model_dir(d, cfg, torch.bfloat16) if sharp else make_model_dir(d, cfg, torch.bfloat16)
+    pc, pw = P.read_model(d)
+    reqs = {"a": random_ids(420, 301, 1), "b": random_ids(40, 301, 2), "c": random_ids(170, 301, 3)}
+    at = {k: 0 for k in reqs}
+    t = Trace()
+
+    def step(**new):
+        t.add([(k, reqs[k][at[k]:at[k] + n], list(range(n)), at[k]) for k, n in new.items()],
+              end=[k for k, n in new.items() if at[k] + n == len(reqs[k])])
+        for k, n in new.items():
+            at[k] += n
+
+    step(a=200)         # expanded
+    step(b=30)          # over the latents
+    step(a=199, b=1)    # expanded: a portion behind 200 tokens, a single token behind 30
+    step(c=160, a=1, b=1)  # expanded: a whole prompt beside single tokens
+    while at["a"] < 420:
+        step(**{k: 1 for k in ("a", "b", "c") if at[k] < len(reqs[k])})
+    calls = []
+    expanded = ops.latent_attention_expanded
+    monkeypatch.setattr(ops, "latent_attention_expanded", lambda *a: (calls.append(a[6].n_tokens), expanded(*a))[1])
+    eng = llmengine.Engine(d, "bf16", block_size=16)
+    eng.configure_cache(num_blocks=48, block_size=16, num_slots=4)
+    rows = replay(eng, t)
+    assert calls == [200] * 3 + [200] * 3 + [162] * 3  # three runs of layers a step
+    for k, ids in reqs.items():
+        rows_close(np.stack([rows[(k, p)] for p in range(len(ids))]), P.forward(pc, pw, ids)[0].numpy(), torch.bfloat16, f"request {k}")
+    assert ops.tensor_core_error() == 0 and eng.cm.num_requests == 0
