@@ -9,7 +9,6 @@ to library or CPU code.
 from __future__ import annotations
 
 import ctypes
-import os
 from ctypes import c_float, c_int, c_longlong, c_void_p
 from typing import Optional
 
@@ -155,10 +154,6 @@ class CudaOps:
                 lib.llm_attention_mma_scratch_floats.restype = ctypes.c_longlong
                 lib.llm_latent_attention_scratch_floats.restype = ctypes.c_longlong
                 lib.llm_gemm_decode_scratch_floats.restype = ctypes.c_longlong
-                # "auto", "on" or "off" (see use_cta_pairs; for measurements, pairs are not safe to serve with)
-                pairs = os.environ.get("LLMENGINE_CTA_PAIRS", "").strip().lower()
-                if pairs in ("auto", "on", "off"):
-                    lib.llm_gemm_tc_pair(c_int({"auto": -1, "on": 1, "off": 0}[pairs]))
             self._libs[name] = lib
         return lib
 
@@ -168,7 +163,8 @@ class CudaOps:
         (the default), "auto" where the kernel library estimates them to be faster (long products
         and those of many rounds of tiles, e.g. gate|up and down of a 2,048-token prompt, not
         q|k|v or o). They are off by default because a prompt step at the Llama 3.2 3B layer sizes
-        was seen to stop inside the pair kernel, rarely and for a cause that was not found."""
+        was seen to stop inside the pair kernel, rarely and for a cause that was not found: for the product
+        on its own, never for a whole step, which nothing outside of this process can ask for."""
         mode = -1 if on == "auto" else (1 if on else 0)
         self.lib("tensorcore").llm_gemm_tc_pair(c_int(mode))
 
