@@ -54,6 +54,11 @@ class Workspace:
             self._buffers[tag].zero_()
         return out
 
+    def holds(self, tag: str, nbytes: int) -> bool:
+        """Whether get() hands out nbytes of this tag without growing its buffer."""
+        buf = self._buffers.get(tag)
+        return buf is not None and buf.numel() >= nbytes
+
     def zero(self, tag: str) -> None:
         """Clears a tag's buffer, if there is one (after a failed step left it in an unknown state)."""
         buf = self._buffers.get(tag)

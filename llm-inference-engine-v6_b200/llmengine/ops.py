@@ -993,19 +993,22 @@ class CudaOps:
     # 4.2 MFLOP a cached token (16 heads of 128 + 128 from 512) on the dense products; the attention over latents costs 3.4 times the
     # operations of the one over keys and values, on the slower tensor path. From about 50 tokens a request it is the faster way
     # (16 heads of 128 + 64 / 128, all of it: 2,048 tokens 84 us against 769, 128 tokens behind 2,000 others 65 against 327), up to
-    # LATENT_EXPANDED_ROWS rows, which bounds what the step keeps beside the cache.
+    # LATENT_EXPANDED_ROWS rows, which bounds the work on them, and LATENT_EXPANDED_BYTES of scratch, which is what a step needs beside the
+    # cache (9,344 bytes a row at those sizes: 306 MB at 32,768 rows; more heads get fewer rows). Beyond either a step runs over the latents.
     LATENT_EXPANDED_TOKENS = 48
     LATENT_EXPANDED_ROWS = 32768
+    LATENT_EXPANDED_BYTES = 320 << 20
 
     def latent_expanded_sizes(self, heads: int, dim: int, rot_dim: int, vdim: int, kv_rank: int, rot_dims: int) -> bool:
         return (self.tensor_cores and self.latent_tensor_cores and rot_dims % 16 == 0 and
                 bool(self.lib("tensorcore").llm_latent_expanded_supported(c_int(heads), c_int(dim), c_int(rot_dim), c_int(vdim), c_int(kv_rank))))
 
-    def latent_expanded_rows(self, batch) -> int:
-        """Rows a request takes in the expanded form of this step's latent attention; 0: the step runs over the latents."""
+    def latent_expanded_rows(self, batch, row_bytes: int = 0) -> int:
+        """Rows a request takes in the expanded form of this step's latent attention, of which one takes row_bytes of scratch; 0: the step
+        runs over the latents."""
         rows = -(-batch.max_seq_len // 128) * 128
         if (batch.n_tokens < max(128, self.LATENT_EXPANDED_TOKENS * batch.n_seqs) or batch.n_seqs * rows > self.LATENT_EXPANDED_ROWS or
-                not (self.tensor_cores and self.latent_tensor_cores)):
+                batch.n_seqs * rows * row_bytes > self.LATENT_EXPANDED_BYTES or not (self.tensor_cores and self.latent_tensor_cores)):
             return 0
         return rows
 

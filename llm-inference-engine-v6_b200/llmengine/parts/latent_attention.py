@@ -92,11 +92,12 @@ class LatentAttention(Mixer):
         # the heads' key maps transposed, [H, kv_rank, dim]: applied to the unrotated part of the query
         self.w_ukt = tensors[s.uk_weight].view(s.heads, s.dim, s.kv_rank).transpose(1, 2).contiguous()
         self.w_uv = tensors[s.uv_weight].view(s.heads, s.vdim, s.kv_rank).contiguous()
-        # the heads' key and value maps as one product, for steps that expand the latents
+        # the heads' key and value maps as one product, for steps that expand the latents (the value maps are its second part)
         ops, self.w_ukv = self.env.ops, None
         if (self.env.dtype == torch.bfloat16 and not s.sink and hasattr(ops, "latent_expanded_sizes") and
                 ops.latent_expanded_sizes(s.heads, s.dim, s.rot_dim, s.vdim, s.kv_rank, self.rot_dims)):
             self.w_ukv = torch.cat([tensors[s.uk_weight].view(-1, s.kv_rank), tensors[s.uv_weight].view(-1, s.kv_rank)], dim=0).contiguous()
+            self.w_uv = self.w_ukv[s.heads * s.dim:].view(s.heads, s.vdim, s.kv_rank)
         self.w_o = tensors[s.o_weight]
         self.dq_norm = tensors[s.dq_norm]
         self.dkv_norm = tensors[s.dkv_norm] if s.own_kv else None
@@ -124,8 +125,10 @@ class LatentAttention(Mixer):
                         self.cos, self.sin, ctx, ctx.block_tables[cache.group], cq, cache.k if writes else None)
         q = ctx.ws.get("latent.q", (n, H * (s.dim + s.rot_dim)), dt)
         ops.gemm(cq, self.w_uq, q, ctx.ws)
-        rows = ops.latent_expanded_rows(ctx) if self.w_ukv is not None and parts.shape[0] == 1 else 0
-        if rows:
+        rows = 0
+        if self.w_ukv is not None and parts.shape[0] == 1:
+            rows = ops.latent_expanded_rows(ctx, 2 * (s.kv_rank + 64 + H * (s.dim + s.vdim)))
+        if rows and self._room(rows, ctx):
             att = self._expanded(q, parts[0], g_off, rows, ctx, cache)
             return add_into_stream_or_partials(ops, att, self.w_o, ctx, False, "latent.delta")
         ql = ctx.ws.get("latent.ql", (n, H, Dk), dt)
@@ -146,17 +149,35 @@ class LatentAttention(Mixer):
             ops.heads_product(ol, self.w_uv, att.view(n, H, s.vdim), **gate)
         return add_into_stream_or_partials(ops, att, self.w_o, ctx, False, "latent.delta")
 
+    def _expanded_scratch(self, rows: int, ctx):
+        """tag -> (shape, type) of what the expanded form keeps beside what the form over the latents needs."""
+        s, total = self.spec, ctx.n_seqs * rows
+        return {"latent.rows": ((total, s.kv_rank + 64), self.env.dtype),  # [latent | rotated part, zeros up to 64]
+                "latent.kv": ((total, s.heads * (s.dim + s.vdim)), self.env.dtype),
+                "latent.out32": ((ctx.n_tokens, s.heads * s.vdim), torch.float32)}
+
+    def _room(self, rows: int, ctx) -> bool:
+        """Whether that scratch is there already or takes at most a quarter of the free device memory: where the page pool fills the
+        device, steps keep running over the latents, which need none of it."""
+        need = 0
+        for tag, ((n, width), dt) in self._expanded_scratch(rows, ctx).items():
+            nbytes = n * width * dt.itemsize
+            need += 0 if ctx.ws.holds(tag, nbytes) else nbytes
+        if need == 0:
+            return True
+        if "free_memory" not in ctx.shared:  # (asked of the driver once a step)
+            dev = self.env.device
+            ctx.shared["free_memory"] = torch.cuda.mem_get_info(dev)[0] + torch.cuda.memory_reserved(dev) - torch.cuda.memory_allocated(dev)
+        return 4 * need <= ctx.shared["free_memory"]
+
     def _expanded(self, q, sums, g_off: int, rows: int, ctx, cache: LayerCache) -> torch.Tensor:
         """Prompt portions: keys and values of the heads from the contexts' latents (one product), then attention over them."""
-        s, ops, dt = self.spec, self.env.ops, self.env.dtype
-        H, total = s.heads, ctx.n_seqs * rows
-        latents = ctx.ws.get("latent.rows", (total, s.kv_rank + 64), dt)  # [latent | rotated part, zeros up to 64]
+        s, ops, H = self.spec, self.env.ops, self.spec.heads
+        latents, kv, out = (ctx.ws.get(tag, *what) for tag, what in self._expanded_scratch(rows, ctx).items())
         ops.latent_rows(cache.k, ctx, ctx.block_tables[cache.group], latents, rows)
-        kv = ctx.ws.get("latent.kv", (total, H * (s.dim + s.vdim)), dt)
         ops.gemm(latents[:, :s.kv_rank], self.w_ukv, kv)
         ops.rotate_heads(q, H, s.dim + s.rot_dim, s.dim, self.cos, self.sin, ctx.positions)
-        att = ctx.ws.get("latent.out", (ctx.n_tokens, H * s.vdim), dt)
-        out = ctx.ws.get("latent.out32", (ctx.n_tokens, H * s.vdim), torch.float32)
+        att = ctx.ws.get("latent.out", (ctx.n_tokens, H * s.vdim), self.env.dtype)
         ops.latent_attention_expanded(q, kv[:, :H * s.dim], kv[:, H * s.dim:], latents, s.kv_rank, rows, ctx, out, H, s.dim, s.rot_dim, s.vdim,
                                       s.scale, s.window)
         return ops.gate_heads(out, att, sums, g_off, H, s.vdim, s.gate_per_head)

@@ -101,6 +101,39 @@ def test_what_is_expanded(ops):
         assert ops.latent_expanded_rows(Batch(seqs)) == want
 
 
+def test_scratch_of_expanded_steps_is_bounded(ops, monkeypatch):
+    """By bytes, whatever the number of heads, and by what is free: a layer whose scratch would take more runs over the latents, with the
+    same results up to rounding, and takes no memory for it."""
+    from gpu_helpers import Harness
+    from llmengine.config.vapelix import VapelixConfig
+    from llmengine.models.vapelix import describe_vapelix
+    from llmengine.parts import build_part
+    from test_vapelix_gpu import tensors_for
+    b = Batch([(16000, 300)])
+    for heads in (16, 32, 128):
+        row = 2 * (512 + 64 + heads * 256)
+        rows = ops.latent_expanded_rows(b, row)
+        assert rows == (16384 if 16384 * row <= ops.LATENT_EXPANDED_BYTES else 0) and rows * row <= 336e6
+    assert ops.latent_expanded_rows(b, 2 * (576 + 128 * 256)) == 0
+    cfg = _wide_config()
+    spec = describe_vapelix(VapelixConfig.from_dict(cfg)).layers[0].mixer
+    m = cfg["layers"][0]["mixer"]
+    outs = []
+    for free in (None, 1 << 20):
+        if free:
+            monkeypatch.setattr(torch.cuda, "mem_get_info", lambda dev=None: (free, 1 << 37))
+            monkeypatch.setattr(torch.cuda, "memory_reserved", lambda dev=None: 0)
+            monkeypatch.setattr(torch.cuda, "memory_allocated", lambda dev=None: 0)
+        h = Harness(torch.bfloat16, page=16, pages=40, nkv=1, hd=m["kv_rank"] + m["rot_dim"])
+        part = build_part("mixer", spec, h.env)
+        part.load(tensors_for(part.tensor_needs(spec), 5, torch.bfloat16)[1])
+        assert part.w_uv.untyped_storage().data_ptr() == part.w_ukv.untyped_storage().data_ptr()  # the value maps are held once
+        x = torch.randn(300, cfg["width"], generator=torch.Generator().manual_seed(6)).bfloat16().to(DEV)
+        outs.append(part.forward(x, h.ctx([(1, 300, [])]), h.cache).sum(0))
+        assert ("latent.kv" in h.ws._buffers) == (free is None)
+    assert (outs[0] - outs[1]).norm() < 2e-2 * outs[0].norm()
+
+
 def _wide_config():
     """Vapelix with heads that the expanded form takes: 64 numbers beside a rotated part of 32 in a layer that runs twice, and 128 beside 64
     of which 48 are rotated; every expert is chosen, so that no rounding changes a choice."""
