@@ -980,14 +980,6 @@ extern "C" int llm_gemm_tc_form(int M, int N, int K, int swiglu) {
   return use_persistent(M, N) ? FORM_PERSISTENT_256 : FORM_ONE_TILE;
 }
 
-// Number of K splits llm_gemm_tc will really use for (K, wanted splits).
-extern "C" int llm_gemm_tc_splits(int K, int splits) {
-  const int k_tiles = (K + BK - 1) / BK;
-  if (splits < 1) splits = 1;
-  const int per_split = (k_tiles + splits - 1) / splits;
-  return (k_tiles + per_split - 1) / per_split;
-}
-
 // Whether the tensor-core kernel takes these operands (else the caller uses the CUDA-core one).
 extern "C" int llm_gemm_tc_supported(const void* a, const void* w, int M, int N, int K, long long lda, long long ldw) {
   auto al = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; };

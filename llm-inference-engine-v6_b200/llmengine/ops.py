@@ -374,7 +374,7 @@ class CudaOps:
                 return 1, 1, 3
             target = self.SPLIT_TARGET_CTAS if M <= 32 else self.SPLIT_TARGET_CTAS // 2
             want = min(max(1, -(-target // tiles)), max(1, k_tiles // 2))
-            per_split = -(-k_tiles // want)  # (as llm_gemm_tc_splits)
+            per_split = -(-k_tiles // want)  # (as the kernel cuts: equal pieces of whole k-tiles, so there may be fewer than wanted)
             return 1, -(-k_tiles // per_split), 3
         wide = M > 128
         tiles *= -(-M // 256) if wide else 1
