@@ -14,6 +14,10 @@
 //     two-sum again; result = sum + carried errors, rounded once.
 // Long inner sizes therefore cost no accuracy: what is left is the rounding inside chains of 16. (Sums in float64 would be
 // six additions fewer a block, but the conversion of a float32 runs at a few a clock and multiprocessor.)
+//
+// w is a weight: its first chunks are fetched before the dependency wait, so no kernel launched ahead on the stream that releases
+// its dependents early (all of this library's do) may be writing it. a is read behind the wait. (Fetching w behind it too: a float32
+// decode step of 8 requests at the Llama 3.2 1B sizes 2.44 ms instead of 2.36, a tiny model's 130 us instead of 125.)
 #include "simt_common.cuh"
 
 #include <cooperative_groups.h>

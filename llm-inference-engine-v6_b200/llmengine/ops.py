@@ -107,7 +107,7 @@ class CudaOps:
         self.fused_decode_attention = True  # ... with the sum of the q|k|v parts, rotation and cache write in the same kernel
         self.latent_tensor_cores = True  # latent attention on mma.sync where the geometry allows it (off: CUDA cores)
         self.gated_attention_tensor_cores = True  # gated attention on mma.sync where the geometry allows it (off: CUDA cores)
-        self.routed_tensor_cores = True  # per-expert products of a routed feed-forward on mma.sync (off: CUDA cores)
+        self.routed_tensor_cores = True  # per-expert products of a routed feed-forward on tcgen05 or, with few rows an expert, mma.sync (off: CUDA cores)
         # Steps of few tokens: products that add their K pieces themselves, with the norm before, the residual sum
         # and SiLU * up folded in (gemm_few_tokens). Off: measured on B200 (batch 8, 2,048-token contexts, 1B layer
         # sizes) such a step takes 1.15 ms with the pieces meeting inside clusters and 1.40 ms with them meeting in
@@ -358,7 +358,8 @@ class CudaOps:
         has work, as long as writing and reading the parts (6 TB/s, out of L2) costs less than it saves. Measured with 77 / 256 tokens
         (tiles of tokens -> this, in us): 2,048 outputs of 2,048 inputs 18.0 / 20.0 -> 6.9 / 11.9, of 8,192 inputs 52.6 / 54.6 ->
         11.1 / 16.8, 3,072 of 2,048 20.2 / 22.9 -> 7.9 / 12.3. Up to 128 tokens the tile is half as wide and there are twice as many
-        CTAs even without a cut (16,384 of 2,048: 22.0 -> 16.7)."""
+        CTAs even without a cut (16,384 of 2,048: 22.0 -> 16.7). The rule has no bound on tokens of its own: it applies while the tiles
+        are at most half of the SMs, which 2,048 outputs reach at 1,024 tokens, 72 outputs at 18,944 (two parts or more have to fit one wave)."""
         key = (M, N, K, may_split, reduced)
         hit = self._forms.get(key)
         if hit is None:
@@ -388,7 +389,7 @@ class CudaOps:
                     best, best_us = (1, splits, 8), us
         return best
 
-    ONE_WAVE = 148  # SMs: one CTA with the long ring each
+    ONE_WAVE = 148  # the SMs of a B200, the one device these kernels are built for: one CTA with the long ring each
 
     def gemm_cuts(self, a: torch.Tensor, w: torch.Tensor) -> bool:
         """Whether gemm_partials cuts K for these operands, so that a consumer that adds the parts saves the kernel that would."""
@@ -407,9 +408,12 @@ class CudaOps:
     def gemm(self, a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, ws=None) -> torch.Tensor:
         """out[m,n] = sum_k a[m,k]*w[n,k]; float32 accumulation; a and w of one dtype; out float32
         or that dtype. Rows may be strided views. bfloat16 runs on the tensor cores (with a
-        workspace `ws`: cut along K and reduced when few tokens stream a weight with few output
-        tiles); float32 on CUDA cores, every output element summed over k in ascending order
-        whatever the batch."""
+        workspace `ws`: cut along K and reduced where the output's tiles leave multiprocessors idle,
+        see _form); float32 on CUDA cores, every output element summed over k in an order that K
+        alone decides, whatever the batch.
+        `w` is a weight: the kernels begin to read it before the kernels launched ahead of them on the
+        stream are done (`a` not). A `w` that one of this object's own kernels has just written needs a
+        synchronization in between; one that torch has written does not."""
         _need(a, "gemm.a"); _need(w, "gemm.w", a.dtype); _need(out, "gemm.out")
         M, K = a.shape
         N = w.shape[0]
@@ -456,7 +460,8 @@ class CudaOps:
     def gemm_partials(self, a: torch.Tensor, w: torch.Tensor, ws, tag: str) -> torch.Tensor:
         """As gemm, for consumers that add partial sums themselves: returns float32 [parts, M, N]
         (scratch `tag` of workspace `ws`); the product is the sum over parts, to be taken in index
-        order. parts is 1 unless few tokens stream a weight with few output tiles."""
+        order. parts is 1 in float32 and where K is not cut (_form): the rule asks how many CTAs the
+        output's tiles give, so a product of many tokens with few outputs is cut too. w: as in gemm."""
         _need(a, "gemm.a"); _need(w, "gemm.w", a.dtype)
         M, K = a.shape
         N = w.shape[0]
@@ -471,8 +476,8 @@ class CudaOps:
         return parts
 
     def can_add_into(self, a: torch.Tensor, w: torch.Tensor) -> bool:
-        """Whether gemm_add_into takes these operands: more tokens than the swapped form holds, on the
-        tensor-core kernel."""
+        """Whether gemm_add_into takes these operands: more than SWAP_MAX_TOKENS tokens, on the tensor-core
+        kernel."""
         return self.add_into_stream and a.shape[0] > self.SWAP_MAX_TOKENS and self._tc_usable(a, w)
 
     def gemm_add_into(self, a: torch.Tensor, w: torch.Tensor, h: torch.Tensor) -> None:
