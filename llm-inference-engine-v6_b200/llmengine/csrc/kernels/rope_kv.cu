@@ -114,11 +114,20 @@ __global__ void __launch_bounds__(128)
 // Eight neighbouring sums over the parts of a product, in index order.
 __device__ __forceinline__ void sum8(const float* p, int n_parts, size_t stride, float* v) {
   float4 lo = reinterpret_cast<const float4*>(p)[0], hi = reinterpret_cast<const float4*>(p)[1];
-#pragma unroll 3
-  for (int k = 1; k < n_parts; ++k) {
-    const float4 a = reinterpret_cast<const float4*>(p + k * stride)[0], b = reinterpret_cast<const float4*>(p + k * stride)[1];
-    lo.x += a.x; lo.y += a.y; lo.z += a.z; lo.w += a.w;
-    hi.x += b.x; hi.y += b.y; hi.z += b.z; hi.w += b.w;
+  for (int k0 = 1; k0 < n_parts; k0 += 4) {  // four parts' loads in flight
+    float4 a[4], b[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      if (k0 + k < n_parts) {
+        a[k] = reinterpret_cast<const float4*>(p + (k0 + k) * stride)[0];
+        b[k] = reinterpret_cast<const float4*>(p + (k0 + k) * stride)[1];
+      }
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+      if (k0 + k < n_parts) {
+        lo.x += a[k].x; lo.y += a[k].y; lo.z += a[k].z; lo.w += a[k].w;
+        hi.x += b[k].x; hi.y += b[k].y; hi.z += b[k].z; hi.w += b[k].w;
+      }
   }
   v[0] = lo.x; v[1] = lo.y; v[2] = lo.z; v[3] = lo.w;
   v[4] = hi.x; v[5] = hi.y; v[6] = hi.z; v[7] = hi.w;
@@ -223,10 +232,11 @@ extern "C" int llm_rope_kv_write(void* qkv, long long ld_qkv, int dtype, const f
   LLM_REQUIRE(!parts || (n_parts >= 1 && kcache), "rope_kv_write: partial sums need n_parts >= 1 and a cache to write to");
   const int threads = 128;
   auto al = [](const void* ptr) { return (reinterpret_cast<uintptr_t>(ptr) & 15u) == 0; };
-  // 16 bytes at a time; with parts from a prompt's tokens on (few tokens: a pair a thread puts more threads on them), and no row scale
+  const int vitems = (nq + nkv) * (hd / 16) + (vcache ? nkv * (hd / 8) : 0);
+  // 16 bytes at a time; with parts and no row scale from a prompt's tokens on, where that leaves threads enough (3 parts, 256 tokens of
+  // 24 heads on 8 of 128: 4.1 us, 9.4 with a pair a thread; 5 parts, 100 tokens of 5 heads on 1 of 32: 3.5 us, 2.2)
   if (dtype == LLM_BF16 && hd % 16 == 0 && ld_qkv % 8 == 0 && al(qkv) && al(kcache) && al(vcache) && al(cos_t) && al(sin_t) &&
-      (!parts || (n_tokens > 64 && !sumsq && al(parts) && part_stride % 4 == 0))) {
-    const int vitems = (nq + nkv) * (hd / 16) + (vcache ? nkv * (hd / 8) : 0);
+      (!parts || (n_tokens > 64 && (long long)n_tokens * vitems >= 148 * 64 && !sumsq && al(parts) && part_stride % 4 == 0))) {
     const dim3 vgrid(n_tokens, ceil_div(vitems, threads));
     LLM_REQUIRE(vgrid.y <= 65535, "rope_kv_write: too many heads");
     launch_kernel(parts ? rope_kv_write_vec_kernel<true> : rope_kv_write_vec_kernel<false>, vgrid, threads, 0, stream, (bf16*)qkv, ld_qkv, parts,
