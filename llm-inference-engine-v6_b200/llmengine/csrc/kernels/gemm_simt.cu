@@ -64,15 +64,17 @@ __device__ __forceinline__ void two_sum2(float2& sum, float2& lost, float2 b) {
 // outputs has 320 tiles for 296 places. Bound by instruction issue: multiply-adds are half of it, the packed two-sums, the
 // moves around them and the reads of shared memory the rest. Rows in shared memory are 64 + 4 numbers long: 8 rows read 16
 // bytes each from different banks. 300 rows, 16,384 outputs of 2,048 inputs: 787 us (25.6 TFLOP/s), 1,480 us as one tile of
-// 64 x 64 with scalar loads; 2,048 rows: 27.7 TFLOP/s.
+// 64 x 64 with scalar loads; 2,048 rows: 27.7 TFLOP/s. Rows that do not begin on four numbers, and bfloat16 ones, go through registers:
+// of odd length 700 rows, 2,048 outputs of 2,049 inputs in bfloat16 take 344 us (17 TFLOP/s; the 64 x 64 tile, which loads two thirds
+// as much for a multiply-add, 315), of a multiple of 4 by 8 bytes 300 rows, 8,192 of 2,052 inputs 466 us (21.6 TFLOP/s).
 constexpr int BM = 64, BN = 32, BK = 64, ROW = BK + 4, TILE_STAGES = 4, TJ = BN / 8;
 constexpr int Q_ROW = BN + 4;  // a row of the tile's sums
 constexpr int TILE_SMEM = TILE_STAGES * (BM + BN) * ROW * 4;
 static_assert(TILE_SMEM >= BM * Q_ROW * 8, "the sums take the place of the operands");
 
-template <typename TA, typename TW, typename TO, bool ASYNC>
+template <typename T, typename TO, bool ALIGNED>
 __global__ void __launch_bounds__(256, 2)
-    gemm_simt_tile_kernel(const TA* __restrict__ a, const TW* __restrict__ w, TO* __restrict__ out, int M, int N, int K, int m_tiles,
+    gemm_simt_tile_kernel(const T* __restrict__ a, const T* __restrict__ w, TO* __restrict__ out, int M, int N, int K, int m_tiles,
                           long long lda, long long ldw, long long ldo) {
   extern __shared__ __align__(16) float smem[];
   dep_launch();
@@ -83,30 +85,29 @@ __global__ void __launch_bounds__(256, 2)
   const int kh = half_of(K), k_begin = half ? kh : 0, k_end = half ? K : min(kh, K);
   const int n_iter = k_end > k_begin ? (k_end - k_begin + BK - 1) / BK : 0;
 
-  const int lr = tid >> 4, lk = (tid & 15) * 4;  // a thread copies 4 k of rows lr, lr + 16, ...
-  const TW* wp = w + (size_t)min(n0 + lr, N - 1) * ldw;
-  const TA* ap = a + (size_t)min(m0 + lr, M - 1) * lda;
-  // (a row beyond the matrix, or a k beyond the half, reads nothing; its address is that of the thread's first row)
-  auto load_w = [&](int it) {
-    float* dst = smem + (it % TILE_STAGES) * (BM + BN) * ROW + (BM + lr) * ROW + lk;
-    const int k = k_begin + it * BK + lk, count = count4(k, k_end);
-    const TW* src = wp + (count ? k : 0);
-#pragma unroll
-    for (int i = 0; i < BN / 16; ++i) {
-      const bool ok = n0 + lr + 16 * i < N;
-      stage4<ASYNC>(dst + i * 16 * ROW, ok ? src + i * 16 * ldw : wp, ok ? count : 0);
-    }
-  };
-  auto load_a = [&](int it) {
+  // a thread copies 4 k of rows lr, lr + RS, ...: side by side, or (rows without alignment) 32 apart, so that a warp's loads of single
+  // numbers are side by side
+  constexpr int RS = ALIGNED ? 16 : 8, ROWS_A = BM / RS, ROWS_W = BN / RS;
+  const int lr = ALIGNED ? tid >> 4 : tid >> 5, lk = ALIGNED ? (tid & 15) * 4 : tid & 31;
+  const T* wp = w + (size_t)min(n0 + lr, N - 1) * ldw;
+  const T* ap = a + (size_t)min(m0 + lr, M - 1) * lda;
+  // COUNT rows from FIRST on of the ROWS_A rows of a and then the ROWS_W of w that a thread copies (a row beyond the matrix, or a k
+  // beyond the half, reads nothing; its address is that of the thread's first row)
+  auto load = [&](int it, auto first_of, auto count_of) {
+    constexpr int FIRST = decltype(first_of)::value, COUNT = decltype(count_of)::value;
     float* dst = smem + (it % TILE_STAGES) * (BM + BN) * ROW + lr * ROW + lk;
-    const int k = k_begin + it * BK + lk, count = count4(k, k_end);
-    const TA* src = ap + (count ? k : 0);
-#pragma unroll
-    for (int i = 0; i < BM / 16; ++i) {
-      const bool ok = m0 + lr + 16 * i < M;
-      stage4<ASYNC>(dst + i * 16 * ROW, ok ? src + i * 16 * lda : ap, ok ? count : 0);
-    }
+    const int k = k_begin + it * BK + lk, count = ALIGNED ? count4(k, k_end) : max(0, min(2, (k_end - k + 31) / 32)), at = count ? k : 0;
+    auto inside = [&](int i) { return i < ROWS_A ? m0 + lr + RS * i < M : n0 + lr + RS * (i - ROWS_A) < N; };
+    stage_rows<ALIGNED, COUNT, 2, 32, T>([&](int i) { return dst + (FIRST + i) * RS * ROW; },
+                                         [&](int i) {
+                                           i += FIRST;
+                                           return i < ROWS_A ? ap + (inside(i) ? at + i * RS * lda : 0) : wp + (inside(i) ? at + (i - ROWS_A) * RS * ldw : 0);
+                                         },
+                                         [&](int i) { return inside(FIRST + i) ? count : 0; });
   };
+  using std::integral_constant;
+  auto load_w = [&](int it) { load(it, integral_constant<int, ROWS_A>{}, integral_constant<int, ROWS_W>{}); };
+  auto load_a = [&](int it) { load(it, integral_constant<int, 0>{}, integral_constant<int, ROWS_A>{}); };
   const int early = min(TILE_STAGES - 1, n_iter);
   for (int it = 0; it < early; ++it) load_w(it);  // weights are not produced by the stream
   dep_wait();
@@ -125,8 +126,7 @@ __global__ void __launch_bounds__(256, 2)
     wait_groups<TILE_STAGES - 2>();
     __syncthreads();
     if (it + TILE_STAGES - 1 < n_iter) {
-      load_w(it + TILE_STAGES - 1);
-      load_a(it + TILE_STAGES - 1);
+      load(it + TILE_STAGES - 1, integral_constant<int, 0>{}, integral_constant<int, ROWS_A + ROWS_W>{});
     }
     commit_group();
     const float* as = smem + (it % TILE_STAGES) * (BM + BN) * ROW + tm * ROW + g * 16;
@@ -208,9 +208,9 @@ constexpr int few_stages() { return MT <= 4 ? 4 : MT <= 8 ? 3 : 2; }
 template <int MT>
 constexpr int few_smem() { return (few_stages<MT>() * (NT + MT) * ROW_C + 2 * BLOCKS * (NT * MT + 4)) * 4; }
 
-template <typename TA, typename TW, typename TO, int MT, int TN, int TM, bool ASYNC>
+template <typename T, typename TO, int MT, int TN, int TM, bool ALIGNED>
 __global__ void __launch_bounds__(few_threads<MT, TN, TM>(), 1)
-    gemm_simt_few_kernel(const TA* __restrict__ a, const TW* __restrict__ w, TO* __restrict__ out, int M, int N, int K,
+    gemm_simt_few_kernel(const T* __restrict__ a, const T* __restrict__ w, TO* __restrict__ out, int M, int N, int K,
                          long long lda, long long ldw, long long ldo) {
   constexpr int FEW_THREADS = few_threads<MT, TN, TM>();
   constexpr int STAGES = few_stages<MT>(), STAGE = (NT + MT) * ROW_C, OUTS = NT * MT, SUMS = OUTS + 4;
@@ -223,32 +223,35 @@ __global__ void __launch_bounds__(few_threads<MT, TN, TM>(), 1)
   const int n_tiles = (N + NT - 1) / NT, chunks = (K + KC - 1) / KC, kh = half_of(K);
   const int mine = (int)blockIdx.x < n_tiles ? (n_tiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
   const long long n_iter = (long long)mine * chunks;
-  const int lk = tid % (KC / 4), lr = tid / (KC / 4);  // a thread's 16 bytes of a row's chunk, and its first row
+  // a thread's four numbers of a row's chunk, side by side or (several rows without alignment) KC / 4 apart, and its first row
+  constexpr bool BESIDE = ALIGNED || MT == 1;
+  constexpr int GAP = BESIDE ? 1 : KC / 4;
+  const int lk = BESIDE ? tid % (KC / 4) * 4 : tid % (KC / 4), lr = tid / (KC / 4);
   constexpr int LOAD_ROWS = FEW_THREADS / (KC / 4);
-  const int at = lr * ROW_C + lk * 4;
-  const TA* ap[(MT + LOAD_ROWS - 1) / LOAD_ROWS];
+  const int at = lr * ROW_C + lk;
+  constexpr int ROWS_X = MT / LOAD_ROWS, ROWS_W = NT / LOAD_ROWS;
+  static_assert(MT % LOAD_ROWS == 0 && NT % LOAD_ROWS == 0, "whole rows a thread");
+  const T* ap[ROWS_X];
 #pragma unroll
-  for (int i = 0; i < (MT + LOAD_ROWS - 1) / LOAD_ROWS; ++i) ap[i] = a + (size_t)min(i * LOAD_ROWS + lr, M - 1) * lda;
+  for (int i = 0; i < ROWS_X; ++i) ap[i] = a + (size_t)min(i * LOAD_ROWS + lr, M - 1) * lda;
   int load_tile = blockIdx.x, load_chunk = 0, load_stage = 0;  // of the next chunk to be requested
-  auto load_w = [&](int tile, int chunk, int stage) {
-    const TW* first = w + (size_t)min(tile * NT + lr, N - 1) * ldw;
-    const int k = chunk * KC + lk * 4, count = count4(k, K);
-    const TW* src = first + (count ? k : 0);
-#pragma unroll
-    for (int r0 = 0; r0 < NT; r0 += LOAD_ROWS) {
-      const bool ok = tile * NT + r0 + lr < N;
-      stage4<ASYNC>(smem + stage * STAGE + r0 * ROW_C + at, ok ? src + r0 * ldw : first, ok ? count : 0);
-    }
+  // COUNT of the ROWS_W rows of w and then the ROWS_X of a that a thread copies, from row FIRST of them on
+  auto load = [&](int tile, int chunk, int stage, auto first_of, auto count_of) {
+    constexpr int FIRST = decltype(first_of)::value, COUNT = decltype(count_of)::value;
+    const T* wp = w + (size_t)min(tile * NT + lr, N - 1) * ldw;
+    float* dst = smem + stage * STAGE + at;
+    const int k = chunk * KC + lk, count = max(0, min(4, (K - k + GAP - 1) / GAP)), from = count ? k : 0;
+    auto inside = [&](int i) { return i < ROWS_W ? tile * NT + i * LOAD_ROWS + lr < N : (i - ROWS_W) * LOAD_ROWS + lr < M; };
+    stage_rows<ALIGNED, COUNT, 4, GAP, T>([&](int i) { return dst + (FIRST + i) * LOAD_ROWS * ROW_C; },
+                                             [&](int i) {
+                                               i += FIRST;
+                                               return i < ROWS_W ? wp + (inside(i) ? from + i * LOAD_ROWS * ldw : 0) : ap[i < ROWS_W ? 0 : i - ROWS_W] + from;
+                                             },
+                                             [&](int i) { return inside(FIRST + i) ? count : 0; });
   };
-  auto load_x = [&](int chunk, int stage) {
-    const int k = chunk * KC + lk * 4, count = count4(k, K);
-#pragma unroll
-    for (int r0 = 0; r0 < MT; r0 += LOAD_ROWS) {
-      const int r = r0 + lr;
-      if (MT % LOAD_ROWS == 0 || r < MT)
-        stage4<ASYNC>(smem + stage * STAGE + (NT + r0) * ROW_C + at, ap[r0 / LOAD_ROWS] + (count ? k : 0), r < M ? count : 0);
-    }
-  };
+  using std::integral_constant;
+  auto load_w = [&](int tile, int chunk, int stage) { load(tile, chunk, stage, integral_constant<int, 0>{}, integral_constant<int, ROWS_W>{}); };
+  auto load_x = [&](int chunk, int stage) { load(0, chunk, stage, integral_constant<int, ROWS_W>{}, integral_constant<int, ROWS_X>{}); };
   auto step_load = [&]() {
     if (++load_chunk == chunks) {
       load_chunk = 0;
@@ -278,8 +281,7 @@ __global__ void __launch_bounds__(few_threads<MT, TN, TM>(), 1)
     float acc[TN][TM];
     if (it < n_iter) {
       if (it + STAGES - 1 < n_iter) {  // into the stage that the iteration before this one has read
-        load_w(load_tile, load_chunk, load_stage);
-        load_x(load_chunk, load_stage);
+        load(load_tile, load_chunk, load_stage, integral_constant<int, 0>{}, integral_constant<int, ROWS_W + ROWS_X>{});
         step_load();
       }
       commit_group();
@@ -375,13 +377,15 @@ __global__ void __launch_bounds__(few_threads<MT, TN, TM>(), 1)
   }
 }
 
-// Up to this many rows (in pieces of 16) the kernel for few rows is the faster one: two pieces of 16 rows take 48 us with 3,072
-// outputs of 2,048 inputs and 85 us with 2,048 of 8,192; a tile of 64 rows, whatever part of it is there, 47 and 169 us.
-constexpr int FEW_ROWS = 32;
+// Up to 16 rows the kernel for few rows is the faster one, and up to 32, in two pieces, where K is long: two pieces of 16 rows take 25 us
+// with 2,048 outputs of 2,048 inputs and 81 us with 2,048 of 8,192, a tile of 64 rows, whatever part of it is there, 39 and 150 us; with 64 of
+// 64 inputs 8.3 and 5.6 us. Without copies that run by themselves a piece is bound by its loads: only where every tile of outputs has a
+// CTA of its own (2,048 of 2,049 in bfloat16 52 and 59 us, 8,192 of 2,049 194 and 130 us).
+bool few_rows(int M, int N, int K, bool copies) { return M <= 16 || (M <= 32 && K > 256 && (copies || ceil_div(N, NT) <= simt_sm_count())); }
 
-template <typename TA, typename TW, typename TO, int MT, int TN, int TM, bool ASYNC>
-void launch_few(const TA* a, const TW* w, TO* out, int M, int N, int K, long long lda, long long ldw, long long ldo, cudaStream_t stream) {
-  auto kernel = gemm_simt_few_kernel<TA, TW, TO, MT, TN, TM, ASYNC>;
+template <typename T, typename TO, int MT, int TN, int TM, bool ALIGNED>
+void launch_few(const T* a, const T* w, TO* out, int M, int N, int K, long long lda, long long ldw, long long ldo, cudaStream_t stream) {
+  auto kernel = gemm_simt_few_kernel<T, TO, MT, TN, TM, ALIGNED>;
   constexpr int smem = few_smem<MT>();
   static_assert(smem <= 227 * 1024, "shared memory of a CTA");
   static std::atomic<unsigned long long> done{0};
@@ -389,21 +393,21 @@ void launch_few(const TA* a, const TW* w, TO* out, int M, int N, int K, long lon
   launch_kernel(kernel, min(ceil_div(N, NT), simt_sm_count()), few_threads<MT, TN, TM>(), smem, stream, a, w, out, M, N, K, lda, ldw, ldo);
 }
 
-template <typename TA, typename TW, typename TO, bool ASYNC>
-void launch(const TA* a, const TW* w, TO* out, int M, int N, int K, long long lda, long long ldw, long long ldo, cudaStream_t stream) {
-  if (M <= FEW_ROWS) {
+template <typename T, typename TO, bool ALIGNED>
+void launch(const T* a, const T* w, TO* out, int M, int N, int K, long long lda, long long ldw, long long ldo, cudaStream_t stream) {
+  if (few_rows(M, N, K, ALIGNED && sizeof(T) == 4)) {
     for (int m = 0; m < M; m += 16) {
       const int rows = min(16, M - m);
-      const TA* am = a + (size_t)m * lda;
+      const T* am = a + (size_t)m * lda;
       TO* om = out + (size_t)m * ldo;
-      if (rows == 1) launch_few<TA, TW, TO, 1, 4, 1, ASYNC>(am, w, om, rows, N, K, lda, ldw, ldo, stream);
-      else if (rows <= 4) launch_few<TA, TW, TO, 4, 2, 4, ASYNC>(am, w, om, rows, N, K, lda, ldw, ldo, stream);
-      else if (rows <= 8) launch_few<TA, TW, TO, 8, 2, 8, ASYNC>(am, w, om, rows, N, K, lda, ldw, ldo, stream);
-      else launch_few<TA, TW, TO, 16, 4, 8, ASYNC>(am, w, om, rows, N, K, lda, ldw, ldo, stream);
+      if (rows == 1) launch_few<T, TO, 1, 4, 1, ALIGNED>(am, w, om, rows, N, K, lda, ldw, ldo, stream);
+      else if (rows <= 4) launch_few<T, TO, 4, 2, 4, ALIGNED>(am, w, om, rows, N, K, lda, ldw, ldo, stream);
+      else if (rows <= 8) launch_few<T, TO, 8, 2, 8, ALIGNED>(am, w, om, rows, N, K, lda, ldw, ldo, stream);
+      else launch_few<T, TO, 16, 4, 8, ALIGNED>(am, w, om, rows, N, K, lda, ldw, ldo, stream);
     }
     return;
   }
-  auto kernel = gemm_simt_tile_kernel<TA, TW, TO, ASYNC>;
+  auto kernel = gemm_simt_tile_kernel<T, TO, ALIGNED>;
   static std::atomic<unsigned long long> done{0};
   allow_smem(kernel, TILE_SMEM, done);
   const int m_tiles = ceil_div(M, BM);
@@ -411,14 +415,13 @@ void launch(const TA* a, const TW* w, TO* out, int M, int N, int K, long long ld
                         m_tiles, lda, ldw, ldo);
 }
 
-template <typename TA, typename TW, typename TO>
+template <typename T, typename TO>
 void choose(const void* a, const void* w, void* out, int M, int N, int K, long long lda, long long ldw, long long ldo, cudaStream_t stream) {
-  // 16-byte copies need float32 rows that begin on 16 bytes
-  if constexpr (std::is_same<TA, float>::value) {
-    if (((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(w)) & 15u) == 0 && lda % 4 == 0 && ldw % 4 == 0)
-      return launch<TA, TW, TO, true>((const TA*)a, (const TW*)w, (TO*)out, M, N, K, lda, ldw, ldo, stream);
-  }
-  launch<TA, TW, TO, false>((const TA*)a, (const TW*)w, (TO*)out, M, N, K, lda, ldw, ldo, stream);
+  // groups of four k at once: rows that begin on four numbers; in bfloat16 of whole groups of four
+  const uintptr_t at = reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(w);
+  if (at % (4 * sizeof(T)) == 0 && lda % 4 == 0 && ldw % 4 == 0 && (sizeof(T) == 4 || K % 4 == 0))
+    return launch<T, TO, true>((const T*)a, (const T*)w, (TO*)out, M, N, K, lda, ldw, ldo, stream);
+  launch<T, TO, false>((const T*)a, (const T*)w, (TO*)out, M, N, K, lda, ldw, ldo, stream);
 }
 
 }  // namespace
@@ -431,11 +434,11 @@ extern "C" int llm_gemm_simt(const void* a, const void* w, void* out, int M, int
   LLM_REQUIRE(lda >= K && ldw >= K && ldo >= N, "gemm_simt: row strides smaller than the rows");
   LLM_REQUIRE(ceil_div(M, BM) <= 65535, "gemm_simt: M=%d too large", M);
   if (in_dtype == LLM_F32 && out_dtype == LLM_F32)
-    choose<float, float, float>(a, w, out, M, N, K, lda, ldw, ldo, stream);
+    choose<float, float>(a, w, out, M, N, K, lda, ldw, ldo, stream);
   else if (in_dtype == LLM_BF16 && out_dtype == LLM_BF16)
-    choose<bf16, bf16, bf16>(a, w, out, M, N, K, lda, ldw, ldo, stream);
+    choose<bf16, bf16>(a, w, out, M, N, K, lda, ldw, ldo, stream);
   else if (in_dtype == LLM_BF16 && out_dtype == LLM_F32)
-    choose<bf16, bf16, float>(a, w, out, M, N, K, lda, ldw, ldo, stream);
+    choose<bf16, float>(a, w, out, M, N, K, lda, ldw, ldo, stream);
   else
     LLM_REQUIRE(false, "gemm_simt: unsupported dtypes in=%d out=%d", in_dtype, out_dtype);
   LLM_CHECK_LAUNCH("gemm_simt");

@@ -55,3 +55,23 @@ def test_bfloat16_of_an_odd_inner_size(ops):
     one = torch.empty(3, 33, device=DEV)
     ops.gemm(a[7:10], w, one)
     assert torch.equal(one, full[7:10])
+
+
+@pytest.mark.parametrize("n,k", [(33, 100), (2400, 516), (70, 1028), (1, 4)])
+def test_bfloat16_of_whole_groups_of_four(ops, n, k):
+    """Inner sizes that the tensor cores refuse and whose rows begin on 8 bytes (and, a number further on, do not): against float64, and
+    rows of the same bits whichever kernel and whichever loads ran."""
+    a, w = _rows(130, k, 0, 7).bfloat16(), _rows(n, k, 0, 8).bfloat16()
+    odd = torch.empty(a.numel() + 1, dtype=torch.bfloat16, device=DEV)[1:].view(a.shape)
+    odd.copy_(a)
+    bound = 18 * 2.0 ** -24 * (a.double().abs() @ w.double().abs().T)
+    exact = a.double() @ w.double().T
+    for dt in (torch.float32, torch.bfloat16):
+        full = torch.empty(130, n, dtype=dt, device=DEV)
+        ops.gemm(a, w, full)
+        assert bool(((full.double() - exact).abs() <= bound + (0 if dt == torch.float32 else 2.0 ** -8) * exact.abs()).all())
+        for m in (1, 3, 8, 16, 17, 32, 33, 65):
+            for src in (a, odd):
+                out = torch.full((m + 1, n), 7.0, dtype=dt, device=DEV)
+                ops.gemm(src[2:2 + m], w, out[:m])
+                assert torch.equal(out[:m], full[2:2 + m]) and bool((out[m] == 7.0).all()), (dt, m)
