@@ -14,6 +14,8 @@
 // Bound by latency with few rows, by reads of shared memory and multiply-adds with many. A layer at the Llama 3.2 1B sizes:
 // 8 single tokens behind 256 to 768 keys 17 us and 7 for the merge (a warp a token and head, a lane a key: 630 us); a prompt
 // of 300 tokens 36 us and 7 (417 us).
+// Only keys that some row of the tile sees are fetched and scored, so a few tokens' prompt costs what it has: 5 tokens 6.1 us, a warp a
+// token and head 6.1, all 128 keys of the segment 13.9.
 //
 // Formula of the reference's attention_f32 (src/kernels.cpp:413-474): kv head = q head / (nq/nkv), score = (q . k) *
 // (1/sqrt(head_dim)) with the scale applied after the dot, softmax in float32, output = sum_t p_t * V[t].
@@ -21,6 +23,7 @@
 
 #include <cfloat>
 #include <cmath>
+#include <type_traits>
 
 namespace {
 
@@ -49,7 +52,7 @@ __device__ __forceinline__ float join(float x, float a, float x_s, float b) { re
 
 // ROWS rows a CTA; a thread has KM keys x RM rows of the scores and KM dimensions x RM rows of the output in each 64
 // dimensions; DC: how many times 64 dimensions.
-template <typename T, int ROWS, int KM, int RM, int DC, bool ASYNC>
+template <typename T, int ROWS, int KM, int RM, int DC, bool ALIGNED>
 __global__ void __launch_bounds__((KT / KM) * (ROWS / RM))
     paged_attention_simt_kernel(const AttArgs p) {
   constexpr int TX = KT / KM, THREADS = TX * (ROWS / RM), WARPS = THREADS / 32;
@@ -77,11 +80,19 @@ __global__ void __launch_bounds__((KT / KM) * (ROWS / RM))
   float* ss = qs + ROWS * row_len;             // [ROWS][S_ROW]
   const int* table = p.table + (size_t)seq * p.max_blocks;
 
-  for (int i = tid; i < ROWS * chunks; i += THREADS) {
-    const int r = i / chunks, c = i - r * chunks, g = (row0 + r) % group, t = (row0 + r) / group;
-    const T* src = (const T*)p.q + (size_t)(tok0 + (r < n_rows ? t : 0)) * p.ld_q + (size_t)(kvh * group + g) * p.hd;
-    const int n = r < n_rows ? count4(4 * c, p.hd) : 0;
-    stage4<false>(qs + r * row_len + 4 * c, n ? src + 4 * c : src, n);
+  for (int i0 = tid; i0 < n_rows * chunks; i0 += 4 * THREADS) {  // (rows beyond the tile's are read by nobody whose result is kept)
+    float4 v[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int i = i0 + u * THREADS, r = i / chunks, c = i - r * chunks;
+      const T* src = (const T*)p.q + (size_t)(tok0 + (row0 + r) / group) * p.ld_q + (size_t)(kvh * group + (row0 + r) % group) * p.hd;
+      v[u] = fetch4(src + 4 * c, i < n_rows * chunks ? count4(4 * c, p.hd) : 0);
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int i = i0 + u * THREADS, r = i / chunks, c = i - r * chunks;
+      if (i < n_rows * chunks) *reinterpret_cast<float4*>(qs + r * row_len + 4 * c) = v[u];
+    }
   }
 
   float acc[DC][KM][RM], m_run[RM], l_run[RM];
@@ -95,21 +106,31 @@ __global__ void __launch_bounds__((KT / KM) * (ROWS / RM))
       for (int i = 0; i < KM; ++i) acc[c][i][j] = 0.f;
   }
 
-  // step s of a segment: 0, 1 its key tiles, 2, 3 its value tiles
-  auto load = [&](int s) {
+  // step s of a segment: 0, 1 its key tiles, 2, 3 its value tiles; keys up to the tile's last one (what lies behind it is masked)
+  auto load = [&](int s, int n_keys) {
     const T* base = (const T*)(s < 2 ? p.k : p.v);
     float* dst = tiles + (s & 1) * KT * row_len;
-    for (int i = tid; i < KT * chunks; i += THREADS) {
-      const int key = i / chunks, c = i - key * chunks;
-      const long long off = s_key[(s & 1) * KT + key];
-      const int n = off >= 0 ? count4(4 * c, p.hd) : 0;
-      stage4<ASYNC>(dst + key * row_len + 4 * c, n ? base + off + 4 * c : base, n);
+    const int total = n_keys * chunks;
+    constexpr int U = ALIGNED && sizeof(T) == 4 ? 1 : ALIGNED && DC == 4 ? 8 : 4;  // loads through registers: several on their way
+    for (int i0 = tid; i0 < total; i0 += U * THREADS) {
+      int key[U], c[U];
+      long long off[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int i = min(i0 + u * THREADS, total - 1);  // (beyond the end: the last group again, the same bytes to the same place)
+        key[u] = i / chunks;
+        c[u] = i - key[u] * chunks;
+        off[u] = s_key[(s & 1) * KT + key[u]];
+      }
+      stage_rows<ALIGNED, U, 4, 1, T>([&](int u) { return dst + key[u] * row_len + 4 * c[u]; }, [&](int u) { return off[u] >= 0 ? base + off[u] + 4 * c[u] : base; },
+                                [&](int u) { return off[u] >= 0 ? count4(4 * c[u], p.hd) : 0; });
     }
     commit_group();
   };
 
   for (; seg < seg_end; ++seg) {
     const int k0 = seg * SEG;
+    auto keys_of = [&](int half) { return max(0, min(KT, last_pos - (k0 + half * KT) + 1)); };
     __syncthreads();  // the segment before this one has been read
     for (int i = tid; i < SEG; i += THREADS) {
       const int key = k0 + i;
@@ -121,12 +142,13 @@ __global__ void __launch_bounds__((KT / KM) * (ROWS / RM))
       s_key[i] = off;
     }
     __syncthreads();
-    load(0);
-    load(1);
+    load(0, keys_of(0));
+    load(1, keys_of(1));
 #pragma unroll
     for (int half = 0; half < 2; ++half) {
       wait_groups<1>();  // (the other key tile, then the first value tile, is on its way)
       __syncthreads();
+      const int n_keys = keys_of(half);
       float s[KM][RM];
 #pragma unroll
       for (int i = 0; i < KM; ++i)
@@ -134,38 +156,43 @@ __global__ void __launch_bounds__((KT / KM) * (ROWS / RM))
         for (int j = 0; j < RM; ++j) s[i][j] = 0.f;
       const float* kt = tiles + half * KT * row_len + tx * row_len;
       const float* qt = qs + ty * RM * row_len;
-      if (ty * RM < n_rows) {
+      auto scores = [&](auto used) {  // of the first `used` of the thread's keys
+        constexpr int USED = decltype(used)::value;
         for (int d = 0; d < hp; d += 4) {
-          float4 kv[KM];
+          float4 kv[USED];
 #pragma unroll
-          for (int i = 0; i < KM; ++i) kv[i] = *reinterpret_cast<const float4*>(kt + i * TX * row_len + d);
+          for (int i = 0; i < USED; ++i) kv[i] = *reinterpret_cast<const float4*>(kt + i * TX * row_len + d);
 #pragma unroll
           for (int j = 0; j < RM; ++j) {
             const float4 qv = *reinterpret_cast<const float4*>(qt + j * row_len + d);
 #pragma unroll
             for (int e = 0; e < 4; ++e)
 #pragma unroll
-              for (int i = 0; i < KM; ++i) s[i][j] = fmaf(part(qv, e), part(kv[i], e), s[i][j]);
+              for (int i = 0; i < USED; ++i) s[i][j] = fmaf(part(qv, e), part(kv[i], e), s[i][j]);
           }
         }
+      };
+      if (ty * RM < n_rows && n_keys > 0) {
+        if (KM > 1 && n_keys <= TX) scores(std::integral_constant<int, 1>{});
+        else if (KM > 2 && n_keys <= 2 * TX) scores(std::integral_constant<int, (KM > 2 ? 2 : KM)>{});
+        else scores(std::integral_constant<int, KM>{});
       }
 #pragma unroll
       for (int i = 0; i < KM; ++i)
 #pragma unroll
         for (int j = 0; j < RM; ++j) ss[(ty * RM + j) * S_ROW + half * KT + tx + i * TX] = s[i][j] * p.scale;
       __syncthreads();
-      load(2 + half);  // over the key tile that has just been read
+      load(2 + half, n_keys);  // over the key tile that has just been read
     }
     // softmax of the segment, a warp a row
-    for (int r = warp; r < ROWS; r += WARPS) {
+    for (int r = warp; r < n_rows; r += WARPS) {
       const int pos = start + (row0 + r) / group, from = p.window > 0 ? max(0, pos - p.window + 1) : 0;
       float4 v = *reinterpret_cast<const float4*>(ss + r * S_ROW + 4 * lane);
       const int key = k0 + 4 * lane;
-      const bool row_ok = r < n_rows;
-      v.x = row_ok && key >= from && key <= pos ? v.x : -INFINITY;
-      v.y = row_ok && key + 1 >= from && key + 1 <= pos ? v.y : -INFINITY;
-      v.z = row_ok && key + 2 >= from && key + 2 <= pos ? v.z : -INFINITY;
-      v.w = row_ok && key + 3 >= from && key + 3 <= pos ? v.w : -INFINITY;
+      v.x = key >= from && key <= pos ? v.x : -INFINITY;
+      v.y = key + 1 >= from && key + 1 <= pos ? v.y : -INFINITY;
+      v.z = key + 2 >= from && key + 2 <= pos ? v.z : -INFINITY;
+      v.w = key + 3 >= from && key + 3 <= pos ? v.w : -INFINITY;
       const float m = warp_max(fmaxf(fmaxf(v.x, v.y), fmaxf(v.z, v.w)));
       v.x = v.x == -INFINITY ? 0.f : expf(v.x - m);
       v.y = v.y == -INFINITY ? 0.f : expf(v.y - m);
@@ -198,7 +225,7 @@ __global__ void __launch_bounds__((KT / KM) * (ROWS / RM))
       if (ty * RM >= n_rows) continue;
       const float* vt = tiles + half * KT * row_len + tx * KM;
       const float* pt = ss + ty * RM * S_ROW + half * KT;
-      const int n_keys = min(KT, last_pos - (k0 + half * KT) + 1);
+      const int n_keys = keys_of(half);
       for (int key = 0; key < n_keys; key += 4) {
         float4 pv[RM];
 #pragma unroll
@@ -309,11 +336,11 @@ __global__ void __launch_bounds__(128) paged_attention_simt_merge_kernel(const A
     if (32 * i + lane < p.hd) out[32 * i + lane] = from_f32<T>(acc[i] * inv);
 }
 
-template <typename T, int ROWS, int KM, int RM, int DC, bool ASYNC>
+template <typename T, int ROWS, int KM, int RM, int DC, bool ALIGNED>
 void launch_rows(AttArgs p, int n_seqs, int max_rows, cudaStream_t stream) {
   p.row_tiles = ceil_div(max_rows, ROWS);
   const int row_len = ((p.hd + 3) & ~3) + 4, smem = (2 * KT * row_len + ROWS * (row_len + S_ROW)) * 4;
-  auto kernel = paged_attention_simt_kernel<T, ROWS, KM, RM, DC, ASYNC>;
+  auto kernel = paged_attention_simt_kernel<T, ROWS, KM, RM, DC, ALIGNED>;
   static std::atomic<unsigned long long> done{0};
   constexpr int most = (2 * KT * (64 * DC + 4) + ROWS * (64 * DC + 4 + S_ROW)) * 4;
   static_assert(most <= 224 * 1024, "shared memory of a CTA");
@@ -321,25 +348,30 @@ void launch_rows(AttArgs p, int n_seqs, int max_rows, cudaStream_t stream) {
   launch_kernel(kernel, dim3((unsigned)p.row_tiles * (unsigned)n_seqs, p.nkv * (p.scratch != nullptr ? p.n_seg : 1)), (KT / KM) * (ROWS / RM), smem, stream, p);
 }
 
-template <typename T, bool ASYNC>
+template <typename T, bool ALIGNED>
 void launch(const AttArgs& p, int n_seqs, int max_rows, bool wide, cudaStream_t stream) {
   if (wide) {
-    if (p.hd <= 64) launch_rows<T, 64, 4, 4, 1, ASYNC>(p, n_seqs, max_rows, stream);
-    else launch_rows<T, 64, 4, 4, 2, ASYNC>(p, n_seqs, max_rows, stream);
-  } else if (p.hd <= 64) launch_rows<T, 8, 1, 2, 1, ASYNC>(p, n_seqs, max_rows, stream);
-  else if (p.hd <= 128) launch_rows<T, 8, 1, 2, 2, ASYNC>(p, n_seqs, max_rows, stream);
-  else launch_rows<T, 8, 1, 2, 4, ASYNC>(p, n_seqs, max_rows, stream);
+    if (p.hd <= 64) launch_rows<T, 64, 4, 4, 1, ALIGNED>(p, n_seqs, max_rows, stream);
+    else launch_rows<T, 64, 4, 4, 2, ALIGNED>(p, n_seqs, max_rows, stream);
+  } else if (p.hd <= 64) launch_rows<T, 8, 1, 2, 1, ALIGNED>(p, n_seqs, max_rows, stream);
+  else if (p.hd <= 128) launch_rows<T, 8, 1, 2, 2, ALIGNED>(p, n_seqs, max_rows, stream);
+  else launch_rows<T, 8, 1, 2, 4, ALIGNED>(p, n_seqs, max_rows, stream);
 }
 
 // Tiles of 64 rows where a request brings more than 8 (and two key tiles, 64 queries and their scores fit beside one another):
-// a prompt of 300 tokens with 4 heads a group takes 19 tiles a key/value head instead of 150, each of which would fetch all keys.
-bool wide_rows(int max_rows, int hd) { return max_rows > 8 && hd <= 128; }
+// a prompt of 300 tokens with 4 heads a group takes 19 tiles a key/value head instead of 150, each of which would fetch all keys. Not
+// where tiles of 8 rows, and segments with CTAs of their own, would leave multiprocessors without one (a
+// prompt of 5 tokens, 24 heads on 8 of 128: 9.7 us as one tile of 64 rows a key/value head, 7.1 as two of 8; of 40 tokens, 12 heads on 1 of
+// 80 in bfloat16: 22 and 10.6 us).
+bool wide_rows(int max_rows, int hd, long long pairs, int n_seg) {
+  return max_rows > 8 && hd <= 128 && (long long)ceil_div(max_rows, 8) * pairs * n_seg > simt_sm_count();
+}
 
 // Whether every segment gets a CTA of its own: where CTAs that walk over all of them would not fill the device twice, as long
 // as the segments' results stay small.
 int segments(int n_seqs, int n_tokens, int max_new, int max_len, int nq, int nkv, int hd) {
   const int n_seg = ceil_div(max_len, SEG), max_rows = max_new * (nq / nkv);
-  const long long ctas = (long long)ceil_div(max_rows, wide_rows(max_rows, hd) ? 64 : 8) * nkv * n_seqs;
+  const long long ctas = (long long)ceil_div(max_rows, wide_rows(max_rows, hd, (long long)nkv * n_seqs, n_seg) ? 64 : 8) * nkv * n_seqs;
   const long long floats = (long long)n_tokens * nq * n_seg * (hd + 2);
   return n_seg > 1 && ctas < 2LL * simt_sm_count() && floats <= (16LL << 20) && (long long)nkv * n_seg <= 65535 ? n_seg : 1;
 }
@@ -366,14 +398,15 @@ extern "C" int llm_paged_attention_simt(const void* q, long long ld_q, const voi
   LLM_REQUIRE(n_seg == 1 || scratch != nullptr, "attention: this step needs scratch");
   const AttArgs p{q, kcache, vcache, out, seq_start, seq_ntok, seq_qoff, block_table, n_seg > 1 ? scratch : nullptr, ld_q, ld_out,
                   max_blocks, nq, nkv, hd, page_size, window, n_seg, 0, scale};
-  const bool wide = wide_rows(max_rows, hd);
+  const bool wide = wide_rows(max_rows, hd, (long long)nkv * n_seqs, ceil_div(max_len, SEG));
   if (dtype == LLM_F32) {
     // 16-byte copies of cache rows: a row is hd float32
     if (hd % 4 == 0 && ((reinterpret_cast<uintptr_t>(kcache) | reinterpret_cast<uintptr_t>(vcache)) & 15u) == 0) launch<float, true>(p, n_seqs, max_rows, wide, stream);
     else launch<float, false>(p, n_seqs, max_rows, wide, stream);
     if (n_seg > 1) launch_kernel(paged_attention_simt_merge_kernel<float>, ceil_div((long long)n_tokens * nq, 4), 128, 0, stream, p, positions, n_tokens);
   } else if (dtype == LLM_BF16) {
-    launch<bf16, false>(p, n_seqs, max_rows, wide, stream);
+    if (hd % 4 == 0 && ((reinterpret_cast<uintptr_t>(kcache) | reinterpret_cast<uintptr_t>(vcache)) & 7u) == 0) launch<bf16, true>(p, n_seqs, max_rows, wide, stream);
+    else launch<bf16, false>(p, n_seqs, max_rows, wide, stream);
     if (n_seg > 1) launch_kernel(paged_attention_simt_merge_kernel<bf16>, ceil_div((long long)n_tokens * nq, 4), 128, 0, stream, p, positions, n_tokens);
   } else
     LLM_REQUIRE(false, "attention: unknown dtype %d", dtype);

@@ -57,21 +57,6 @@ __device__ __forceinline__ void stage_rows(Dst dst, Src src, Count count) {
     }
   }
 }
-// Of 4 elements of a row, the first `count` as float32 into shared memory and zeros behind them. ASYNC: float32 rows whose
-// every fourth element is 16-byte aligned, copied without passing through registers (only what is counted is read).
-template <bool ASYNC, typename T>
-__device__ __forceinline__ void stage4(float* dst, const T* src, int count) {
-  if (ASYNC) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(4 * count) : "memory");
-  } else {
-    float4 v;
-    v.x = count > 0 ? to_f32(src[0]) : 0.f;
-    v.y = count > 1 ? to_f32(src[1]) : 0.f;
-    v.z = count > 2 ? to_f32(src[2]) : 0.f;
-    v.w = count > 3 ? to_f32(src[3]) : 0.f;
-    *reinterpret_cast<float4*>(dst) = v;
-  }
-}
 __device__ __forceinline__ int count4(int k, int K) { return max(0, min(4, K - k)); }
 __device__ __forceinline__ void commit_group() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>

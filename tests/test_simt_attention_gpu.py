@@ -108,3 +108,21 @@ def test_keys_of_minus_infinity_weigh_nothing(ops):
             assert torch.equal(alone[0], whole[t])
             ref = _attention_ref(q[t].view(nq, hd).cpu().double(), K.double(), V.double(), t, nq, nkv, hd, scale, 0)
             torch.testing.assert_close(alone[0].cpu(), ref.float(), rtol=2e-5, atol=2e-5)
+
+
+@pytest.mark.parametrize("dt", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("nq,nkv,hd,window", [(12, 1, 18, 0), (6, 2, 20, 0), (5, 5, 48, 50), (3, 1, 132, 0), (4, 4, 256, 0), (12, 1, 80, 9)])
+@pytest.mark.parametrize("seqs", [[(0, 5)], [(0, 16), (0, 17)], [(60, 3), (0, 33), (200, 1)], [(127, 2), (0, 70)]])
+def test_tiles_that_are_part_empty(ops, dt, nq, nkv, hd, window, seqs):
+    """Few keys, few rows and head sizes whose rows begin on four numbers or do not, against float64. A result is a weighted mean of values
+    of size one: some hundred float32 roundings, and in bfloat16 the operands' products exact in float32 and one rounding at the end."""
+    lens, page, scale = [s + n for s, n in seqs], 8, 1.0 / math.sqrt(hd)
+    kc, vc, table, dense = _paged_setup(dt, nkv, hd, page, lens, sum(-(-x // page) for x in lens) + 2, seed=hd)
+    b = Batch(seqs)
+    q = torch.randn(b.n_tokens, nq * hd, generator=torch.Generator().manual_seed(11)).to(dt).to(DEV)
+    out = torch.full_like(q, float("nan"))
+    ops.paged_attention(q, kc, vc, b, table, out, nq, nkv, hd, scale, window)
+    for i, (s, pos) in enumerate(b.tokens):
+        K, V = dense[s]
+        ref = _attention_ref(q[i].view(nq, hd).cpu().double(), K.double(), V.double(), pos, nq, nkv, hd, scale, window)
+        torch.testing.assert_close(out[i].float().cpu(), ref.float(), rtol=2.0 ** -8 if dt == torch.bfloat16 else 2e-5, atol=2e-5)
