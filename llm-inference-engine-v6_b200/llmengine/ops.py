@@ -380,6 +380,11 @@ class CudaOps:
         wide = M > 128
         tiles *= -(-M // 256) if wide else 1
         best, best_us = (0 if wide else 1, 1, 8), (0.5 if wide else 0.4) * k_tiles
+        # of more than 128 tokens and few k-blocks the parts cost more than the estimate knows: with a kernel that adds them, 1,024
+        # inputs and outputs 11.2 us uncut and 12.6 cut (256 tokens), 64 outputs (whose tiles take a k-block in 0.27 us) of 2,048
+        # inputs 12.1 and 13.7; with a consumer that does, 1,024 inputs and outputs 17.6 and 18.6 with the norm (1,024 tokens)
+        if wide and ((0.27 if N < 128 else 0.5) * k_tiles < 10 if reduced else k_tiles <= 16 and M > 768):
+            may_split = False
         if may_split and tiles <= self.ONE_WAVE // 2:
             for want in range(2, min(self.ONE_WAVE // tiles, k_tiles // 2) + 1):
                 per_split = -(-k_tiles // want)
@@ -399,6 +404,8 @@ class CudaOps:
         M, K = a.shape
         N = w.shape[0]
         swap, splits, stages = form
+        if splits == 1 and N < 128 and M > self.SWAP_MAX_TOKENS:
+            swap = 0  # fewer outputs than accumulator lanes: tiles of tokens with as many columns as there are outputs (64 outputs of 2,048 inputs, 77 tokens: 12.3 us, 14.0 with the weights on the lanes)
         lib = self.lib("tensorcore")
         lda, ldw = K if a.is_contiguous() else a.stride(0), K if w.is_contiguous() else w.stride(0)
         ldo = N if out.is_contiguous() else out.stride(-2)

@@ -53,6 +53,30 @@ def test_what_is_cut():
                     assert swap == (1 if m <= 128 or splits > 1 else 0) and stages == 8
 
 
+def test_what_is_not_cut():
+    """Short products of many tokens, whose parts cost more than they save; the same ones of few tokens or more inputs are cut."""
+    from llmengine.ops import CudaOps
+    ops = CudaOps.__new__(CudaOps)
+    ops._forms = {}
+    for m in (200, 256, 512):
+        assert ops._form(m, 1024, 1024, True, True)[1] == 1 and ops._form(m, 64, 2048, True, True)[1] == 1
+        assert ops._form(m, 1024, 1024, True)[1] > 1 and ops._form(m, 1024, 4096, True, True)[1] > 1 and ops._form(m, 72, 4096, True, True)[1] > 1
+    assert ops._form(77, 1024, 1024, True, True)[1] > 1 and ops._form(128, 64, 2048, True, True)[1] > 1
+    assert ops._form(1024, 1024, 1024, True)[1] == 1 and ops._form(1024, 1024, 4096, True)[1] > 1
+
+
+@pytest.mark.parametrize("m,n,k", [(65, 64, 512), (77, 8, 264), (128, 120, 1032), (100, 1, 64)])
+def test_products_of_fewer_outputs_than_lanes(ops, m, n, k):
+    """Tiles of tokens for them, without a cut: against float64, bounded as above."""
+    a, w = rnd(m, k, seed=31), rnd(n, k, seed=32)
+    exact, bound = a.double() @ w.double().T, 2 * k * 2.0 ** -24 * (a.double().abs() @ w.double().abs().T)
+    for dt in (torch.float32, torch.bfloat16):
+        out = torch.full((m + 1, n), 3.0, dtype=dt, device=DEV)
+        ops.gemm(a, w, out[:m])
+        assert bool(((out[:m].double() - exact).abs() <= bound + (0 if dt == torch.float32 else 2.0 ** -8) * exact.abs()).all())
+        assert bool((out[m] == 3.0).all())
+
+
 @pytest.mark.parametrize("parts,rows,width", [(1, 1, 4), (3, 5, 12), (9, 77, 130), (5, 65, 2048), (2, 3, 7)])
 def test_reduce_partials_forms_agree(ops, parts, rows, width):
     p = rnd(parts, rows, width, seed=3, dt=torch.float32)
