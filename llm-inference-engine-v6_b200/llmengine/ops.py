@@ -1207,6 +1207,10 @@ class CudaOps:
     # expert) 188 us, as mma.sync tiles 588 us; 64 rows an expert 76 against 181 us, 32 rows 71 against 104 us. With fewer rows the
     # products are bound by the experts' matrices, which tiles of 16 rows stream as well.
     ROUTED_SORTED_ROWS = 32
+    # ... and from this many numbers of an expert's matrix (hidden x intermediate) on: below, the gathering and the tiles' fill are what the
+    # products take (both products, 4 of 4 experts of 256 x 128: 64 tokens 20.2 us on mma.sync, 27.4 this way; 2,048 tokens 38.9 and 47.5;
+    # 8 of 64 experts of 512 x 256: 300 tokens 61.4 and 64.4, 2,048 tokens 149 and 142).
+    ROUTED_SORTED_SIZE = 1 << 18
 
     def routed_sorted(self, dtype: torch.dtype, inner=(), per_expert: float = 0.0) -> bool:
         """Whether a step's per-expert products run on rows gathered into the tiles' order (routed_gather, routed_product_sorted),

@@ -22,12 +22,13 @@ from .spec import GroupRoutedMLPSpec, RoutedMLPSpec, TensorNeed
 
 def expert_products(ops, ctx, x, idx, s, outputs, experts, w_up, w_down, epilogue, act_of, on_input, on_output):
     """Every (token, choice) pair's row of its expert's two products, float32 [n * top, hidden] (rows of choices from `experts` on are
-    left as they are). Prompt-sized steps copy the rows into the experts' order once and run on them; smaller ones gather the rows
-    as they read them."""
+    left as they are). Prompt-sized steps copy the rows into the experts' order once and run on them; smaller ones, and those of small
+    experts, gather the rows as they read them."""
     n, dt, rows = ctx.n_tokens, x.dtype, ctx.n_tokens * s.top
     real = {} if experts == outputs else {"real_experts": experts}
     y = ctx.ws.get("routed.y", (rows, s.hidden), torch.float32)
-    if hasattr(ops, "routed_sorted") and ops.routed_sorted(dt, (s.hidden, s.intermediate), rows / s.experts):
+    if (hasattr(ops, "routed_sorted") and s.hidden * s.intermediate >= ops.ROUTED_SORTED_SIZE and
+            ops.routed_sorted(dt, (s.hidden, s.intermediate), rows / s.experts)):
         tile_expert, tile_rows = ops.routed_group(idx, outputs, ops.ROUTED_SORTED_TILE, ctx.ws, "routed", **real)
         xs = ops.routed_gather(x, s.top, tile_expert, tile_rows, ctx.ws.get("routed.rows", (tile_rows.numel(), s.hidden), dt))
         act = ctx.ws.get("routed.act", (tile_rows.numel(), s.intermediate), dt)

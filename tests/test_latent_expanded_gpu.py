@@ -178,10 +178,16 @@ def test_whole_model_through_expanded_steps(tmp_path, monkeypatch, ops, sharp):
     calls = []
     expanded = ops.latent_attention_expanded
     monkeypatch.setattr(ops, "latent_attention_expanded", lambda *a: (calls.append(a[6].n_tokens), expanded(*a))[1])
+    gathers = []
+    if not sharp:  # the experts' products of prompt-sized steps on gathered rows, which is for larger experts than these
+        gather = ops.routed_gather
+        monkeypatch.setattr(ops, "ROUTED_SORTED_SIZE", 0)
+        monkeypatch.setattr(ops, "routed_gather", lambda x, *a: (gathers.append(x.shape[0]), gather(x, *a))[1])
     eng = llmengine.Engine(d, "bf16", block_size=16)
     eng.configure_cache(num_blocks=48, block_size=16, num_slots=4)
     rows = replay(eng, t)
     assert calls == [200] * 3 + [200] * 3 + [162] * 3  # three runs of layers a step
+    assert gathers == ([] if sharp else [200, 200, 162])
     for k, ids in reqs.items():
         rows_close(np.stack([rows[(k, p)] for p in range(len(ids))]), P.forward(pc, pw, ids)[0].numpy(), torch.bfloat16, f"request {k}")
     assert ops.tensor_core_error() == 0 and eng.cm.num_requests == 0
