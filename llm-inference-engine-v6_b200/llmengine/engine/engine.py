@@ -235,7 +235,8 @@ class Engine:
     def step_and_sample(self, entries) -> List[int]:
         """A step followed by the choice of one token for every wanted row (greedy or by the rows'
         temperature, seed and draw index); the tokens come back to the host. Steps in which every
-        request brings one token replay a CUDA graph when `cuda_graphs` is on."""
+        request brings one token replay a CUDA graph when `cuda_graphs` is on; it goes off, with a
+        warning, when the device has no room for a graph's own scratch (a page pool that fills it)."""
         with self._lock:
             self._ensure_cache()
             n = len(entries)
@@ -243,7 +244,11 @@ class Engine:
                 if self.graphs is None:
                     from .graphs import DecodeGraphs
                     self.graphs = DecodeGraphs(self)
-                return self.graphs.run(entries)
+                try:
+                    return self.graphs.run(entries)
+                except torch.OutOfMemoryError:  # (raised while a graph's scratch is sized: nothing of this step has run)
+                    self.cuda_graphs, self.graphs = False, None
+                    warnings.warn("no device memory for a decode graph: steps run without graphs from here on")
             ctx, logits = self.step(entries)
             tokens = self.sampler.sample(logits, ctx, ctx.n_rows)  # (waits for the stream)
             self.raise_if_kernel_error()

@@ -54,3 +54,22 @@ def test_logits_of_recorded_and_eager_steps(tmp_path, name):
         logits[graphs] = out
     for k, (a, b) in enumerate(zip(logits[False], logits[None])):
         assert np.abs(a - b).max() <= 2e-5 * max(1.0, np.abs(a).max()), f"step {k}: {np.abs(a - b).max():.3e}"
+
+
+@pytest.mark.parametrize("dtype", ["fp32", "bf16"])
+def test_no_room_for_a_graph(tmp_path, monkeypatch, dtype):
+    """An engine whose pool leaves no memory for a graph's scratch goes on without graphs: the same tokens, the same step."""
+    from llmengine.engine.graphs import DecodeGraphs
+    cfg, page = TINY["d"]
+    d = make_model_dir(str(tmp_path / "m"), cfg, torch.float32 if dtype == "fp32" else torch.bfloat16)
+    prompt = random_ids(20, cfg["vocab_size"], 5)
+    want = llmengine.Engine(d, dtype, block_size=page, num_blocks=16, max_concurrent=2, cuda_graphs=False).generate(prompt, 8)
+
+    def full(*a):
+        raise torch.OutOfMemoryError("no room")
+
+    monkeypatch.setattr(DecodeGraphs, "_capture", full)
+    eng = llmengine.Engine(d, dtype, block_size=page, num_blocks=16, max_concurrent=2)
+    with pytest.warns(UserWarning, match="without graphs"):
+        assert eng.generate(prompt, 8) == want
+    assert not eng.cuda_graphs and eng.graphs is None and eng.cm.free_pages(0) == 16
