@@ -104,6 +104,17 @@ class StepContext:
         self.delta_bias = None
         self.takes_delta_pairs = False  # set by a block while it runs a feed-forward whose two branches' sums it adds itself
 
+    def has_room(self, sizes: Dict[str, int]) -> bool:
+        """Whether scratch of these sizes (tag -> bytes) is there already or takes at most a quarter of the free device memory: where the
+        page pool fills the device, a part whose faster form needs scratch that its other form does not need runs the other."""
+        need = sum(nbytes for tag, nbytes in sizes.items() if not self.ws.holds(tag, nbytes))
+        if need == 0:
+            return True
+        if "free_memory" not in self.shared:  # (asked of the driver once a step)
+            dev = self.ws.device
+            self.shared["free_memory"] = torch.cuda.mem_get_info(dev)[0] + torch.cuda.memory_reserved(dev) - torch.cuda.memory_allocated(dev)
+        return 4 * need <= self.shared["free_memory"]
+
 
 class StepBuffers:
     """Pinned host staging and its device twin for the step's int32 arrays."""

@@ -1248,6 +1248,10 @@ class CudaOps:
                                               *self._act_args(act if epilogue == "gated_pairs" else "silu"), _stream()), lib)
         return out
 
+    def routed_tiles(self, pairs: int, experts: int, tile: int) -> int:
+        """The most tiles of `tile` rows that `pairs` pairs fill, however they fall on the experts."""
+        return int(self.lib().llm_routed_tiles(c_int(pairs), c_int(experts), c_int(tile)))
+
     def routed_group(self, idx: torch.Tensor, experts: int, tile: int, ws, tag: str, real_experts: Optional[int] = None):
         """Sorts the step's (token, choice) pairs by expert into tiles of `tile` rows -> (tile_expert [tiles] with -1 for
         unused tiles, tile_rows [tiles, tile] with -1 for padding); a pair is token * top + choice. Pairs of experts from
@@ -1255,7 +1259,7 @@ class CudaOps:
         _need(idx, "routed_group.idx", torch.int32)
         lib = self.lib()
         pairs = idx.numel()
-        tiles = int(lib.llm_routed_tiles(c_int(pairs), c_int(experts), c_int(tile)))
+        tiles = self.routed_tiles(pairs, experts, tile)
         tile_expert = ws.get(tag + ".tile_expert", (tiles,), torch.int32)
         tile_rows = ws.get(tag + ".tile_rows", (tiles, tile), torch.int32)
         self._check(lib.llm_routed_group(_ptr(idx), c_int(pairs), c_int(experts), c_int(tile), c_int(tiles), _ptr(tile_expert),

@@ -157,18 +157,8 @@ class LatentAttention(Mixer):
                 "latent.out32": ((ctx.n_tokens, s.heads * s.vdim), torch.float32)}
 
     def _room(self, rows: int, ctx) -> bool:
-        """Whether that scratch is there already or takes at most a quarter of the free device memory: where the page pool fills the
-        device, steps keep running over the latents, which need none of it."""
-        need = 0
-        for tag, ((n, width), dt) in self._expanded_scratch(rows, ctx).items():
-            nbytes = n * width * dt.itemsize
-            need += 0 if ctx.ws.holds(tag, nbytes) else nbytes
-        if need == 0:
-            return True
-        if "free_memory" not in ctx.shared:  # (asked of the driver once a step)
-            dev = self.env.device
-            ctx.shared["free_memory"] = torch.cuda.mem_get_info(dev)[0] + torch.cuda.memory_reserved(dev) - torch.cuda.memory_allocated(dev)
-        return 4 * need <= ctx.shared["free_memory"]
+        """Whether there is memory for that scratch; else steps keep running over the latents, which need none of it."""
+        return ctx.has_room({tag: n * width * dt.itemsize for tag, ((n, width), dt) in self._expanded_scratch(rows, ctx).items()})
 
     def _expanded(self, q, sums, g_off: int, rows: int, ctx, cache: LayerCache) -> torch.Tensor:
         """Prompt portions: keys and values of the heads from the contexts' latents (one product), then attention over them."""

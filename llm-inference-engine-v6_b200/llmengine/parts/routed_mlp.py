@@ -20,15 +20,22 @@ from .registry import build_part, part_class, register_part
 from .spec import GroupRoutedMLPSpec, RoutedMLPSpec, TensorNeed
 
 
+def _sorted_scratch(ops, rows: int, outputs: int, s, dt):
+    """tag -> bytes of what products on gathered rows keep in tiles (the other form: "routed.act" of `rows` rows)."""
+    places = ops.routed_tiles(rows, outputs, ops.ROUTED_SORTED_TILE) * ops.ROUTED_SORTED_TILE
+    return {"routed.rows": places * s.hidden * dt.itemsize, "routed.act": places * s.intermediate * dt.itemsize}
+
+
 def expert_products(ops, ctx, x, idx, s, outputs, experts, w_up, w_down, epilogue, act_of, on_input, on_output):
     """Every (token, choice) pair's row of its expert's two products, float32 [n * top, hidden] (rows of choices from `experts` on are
-    left as they are). Prompt-sized steps copy the rows into the experts' order once and run on them; smaller ones, and those of small
-    experts, gather the rows as they read them."""
+    left as they are). Prompt-sized steps copy the rows into the experts' order once and run on them; smaller ones, those of small
+    experts and those without memory for the copy gather the rows as they read them."""
     n, dt, rows = ctx.n_tokens, x.dtype, ctx.n_tokens * s.top
     real = {} if experts == outputs else {"real_experts": experts}
     y = ctx.ws.get("routed.y", (rows, s.hidden), torch.float32)
     if (hasattr(ops, "routed_sorted") and s.hidden * s.intermediate >= ops.ROUTED_SORTED_SIZE and
-            ops.routed_sorted(dt, (s.hidden, s.intermediate), rows / s.experts)):
+            ops.routed_sorted(dt, (s.hidden, s.intermediate), rows / s.experts) and
+            ctx.has_room(_sorted_scratch(ops, rows, outputs, s, dt))):
         tile_expert, tile_rows = ops.routed_group(idx, outputs, ops.ROUTED_SORTED_TILE, ctx.ws, "routed", **real)
         xs = ops.routed_gather(x, s.top, tile_expert, tile_rows, ctx.ws.get("routed.rows", (tile_rows.numel(), s.hidden), dt))
         act = ctx.ws.get("routed.act", (tile_rows.numel(), s.intermediate), dt)

@@ -73,3 +73,28 @@ def test_sorted_products_against_float64(ops, hidden, ff, epilogue, weigh):
 def test_steps_that_run_sorted(ops):
     assert ops.routed_sorted(torch.bfloat16, (64, 256), 32.0) and not ops.routed_sorted(torch.bfloat16, (64, 256), 31.0)
     assert not ops.routed_sorted(torch.float32, (64, 256), 500.0) and not ops.routed_sorted(torch.bfloat16, (64, 100), 500.0)
+
+
+def test_no_memory_for_the_copy(ops, monkeypatch):
+    """A step whose gathered rows would take more than a quarter of what is free gathers them as it reads them: the same results up to
+    rounding, and none of that memory taken. One that finds the scratch there already uses it, whatever is free."""
+    from gpu_helpers import Harness
+    from llmengine.parts import build_part
+    from llmengine.parts.spec import RoutedMLPSpec
+    from test_vapelix_gpu import tensors_for
+    names = [tuple(f"{k}{e}" for e in range(4)) for k in "ud"]
+    spec = RoutedMLPSpec("routed_mlp", 512, 512, 4, 2, "r", "b", *names)
+    x, outs = rnd(200, 512, seed=7), []
+    calls, gather = [], ops.routed_gather
+    monkeypatch.setattr(ops, "routed_gather", lambda a, *rest: (calls.append(a.shape[0]), gather(a, *rest))[1])
+    h = Harness(torch.bfloat16, page=16)
+    part = build_part("feed_forward", spec, h.env)
+    part.load(tensors_for(part.tensor_needs(spec), 5, torch.bfloat16)[1])
+    for step, free in enumerate((1 << 20, 1 << 33, 1 << 20)):
+        monkeypatch.setattr(torch.cuda, "mem_get_info", lambda dev=None: (free, 1 << 37))
+        monkeypatch.setattr(torch.cuda, "memory_reserved", lambda dev=None: 0)
+        monkeypatch.setattr(torch.cuda, "memory_allocated", lambda dev=None: 0)
+        outs.append(part.forward(x, h.ctx([(step + 1, 200, [])])).clone())
+        assert len(calls) == step and ("routed.rows" in h.ws._buffers) == (step > 0)
+    # both forms: float32 sums of exact products, an activation, one rounding to bfloat16 (2^-9), float32 sums again
+    assert (outs[0] - outs[1]).norm() < 2.0 ** -8 * outs[1].norm() and torch.equal(outs[1], outs[2])
