@@ -5,16 +5,18 @@
 
 namespace {
 
-constexpr int EXACT_ROW = 0x7fffffff;  // in the place of a row's exponent: the row is no fixed-point row
+// In the place of a row's exponent: the row does not fit the form, and its results are formed another way; one of them is NaN, and so they are.
+constexpr int EXACT_ROW = 0x7ffffffe, NAN_ROW = 0x7fffffff;
 
 // e with every |x| of the row below 2^e and its largest whole number clear of the top digit's last value
 __device__ __forceinline__ int row_exponent(uint32_t largest) {  // the bits of the row's largest magnitude
   if (largest == 0u) return 0;
-  if (largest >= 0x7f800000u || largest < 0x12800000u) return EXACT_ROW;  // infinities, NaN; below 2^-90
+  if (largest > 0x7f800000u) return NAN_ROW;
+  if (largest == 0x7f800000u || largest < 0x12800000u) return EXACT_ROW;  // infinities; below 2^-90
   return (int)(largest >> 23) - 126 + ((largest & 0x7fffffu) >= 0x7e0000u ? 1 : 0);
 }
 __device__ __forceinline__ float power_of_two(int e) { return __uint_as_float((uint32_t)(e + 127) << 23); }  // -126 <= e <= 127
-__device__ __forceinline__ float row_scale_of(int e) { return e == EXACT_ROW ? 0.f : power_of_two(31 - e); }
+__device__ __forceinline__ float row_scale_of(int e) { return e >= EXACT_ROW ? 0.f : power_of_two(31 - e); }
 
 __device__ __forceinline__ uint32_t whole(float x, float scale) { return (uint32_t)__float2int_rn(x * scale); }
 // Four words, the digits of a number each, into word p with digit p of each.

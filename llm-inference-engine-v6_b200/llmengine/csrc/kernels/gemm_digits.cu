@@ -17,9 +17,9 @@
 // gate and up is of that kind); chains of multiply-adds with carried errors (gemm_simt.cu) 7.8e-8 in both. Sums of whole numbers do not
 // depend on their order: a row's result is the same bits whatever else is in the batch, whatever the tile, and however K is cut.
 //
-// Rows that do not fit the form, with infinities, NaN or a largest magnitude below 2^-90, are marked (EXACT_ROW). A weight that has one
-// stays float32 on CUDA cores; the results of such a row of activations are summed by the thread that writes them with fused
-// multiply-adds in ascending k. (No weight but zero becomes the whole number zero, so that an infinity times it is one.)
+// Rows that do not fit the form, with infinities, NaN or a largest magnitude below 2^-90, are marked. A weight that has one
+// stays float32 on CUDA cores; the results of such a row of activations are NaN where it holds one, else summed by the thread that writes
+// them with fused multiply-adds in ascending k. (No weight but zero becomes the whole number zero, so that an infinity times it is one.)
 //
 // The weights are written as digits once, when a model is loaded, in 4 bytes a number as before: tiles of 128 rows x 64 k, 32 KB each, lie
 // in memory as they are to lie in shared memory (two planes of 64 bytes a row of the 128-byte swizzle), so a tile is two bulk copies
@@ -194,7 +194,9 @@ __device__ __forceinline__ float weight_at(const uint8_t* w, int k_blocks, int n
   for (int d = 0; d < 4; ++d) q |= (uint32_t)tile[tile_offset(n % BM, k % BK, d)] << (8 * d);
   return (float)(int)(q ^ 0x808080u) * power_of_two(e - 31);
 }
-__device__ __noinline__ float row_product(const DigitArgs& p, int m, int n) {
+// The result of a row that does not fit the form.
+__device__ __noinline__ float row_product(const DigitArgs& p, int m, int n, int mark) {
+  if (mark == NAN_ROW) return __uint_as_float(0x7fffffffu);
   const float* a = p.a + (size_t)m * p.lda;
   const int e = p.w_exp[n];
   float s = 0.f;
@@ -204,7 +206,7 @@ __device__ __noinline__ float row_product(const DigitArgs& p, int m, int n) {
 __device__ __forceinline__ void put_result(const DigitArgs& p, int m, int n, long long sum) {
   if (m >= p.M || n >= p.N) return;
   const int ea = p.a_exp[m];
-  p.out[(size_t)m * p.ldo + n] = ea == EXACT_ROW ? row_product(p, m, n) : digits_value(sum + p.a_sum[m], ea, p.w_exp[n]);
+  p.out[(size_t)m * p.ldo + n] = ea >= EXACT_ROW ? row_product(p, m, n, ea) : digits_value(sum + p.a_sum[m], ea, p.w_exp[n]);
 }
 
 __device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
@@ -475,7 +477,7 @@ __global__ void __launch_bounds__(FEW_WARPS * 32, 1) gemm_digits_few_kernel(cons
           long long sum = my_sum;
 #pragma unroll
           for (int i = 0; i < FEW_WARPS; ++i) sum += s_part[turn][i][tid % OUTS];
-          p.d.out[(size_t)my_m * p.d.ldo + n] = my_exp == EXACT_ROW ? row_product(p.d, my_m, n) : digits_value(sum, my_exp, p.d.w_exp[n]);
+          p.d.out[(size_t)my_m * p.d.ldo + n] = my_exp >= EXACT_ROW ? row_product(p.d, my_m, n, my_exp) : digits_value(sum, my_exp, p.d.w_exp[n]);
         }
         turn ^= 1;  // (the other half: those warps may still be reading this one, and come to the next barrier when they have)
         item = 0;
@@ -523,7 +525,7 @@ bool rows_on_16_bytes(const void* p, long long ld) { return reinterpret_cast<uin
 extern "C" int llm_weight_digits_supported(int N, int K) { return N > 0 && K > 0 && K < 32768 && encode_fn() != nullptr; }
 
 // A weight as digits: exps int32 [N], tiles uint8 [ceil(N / 128)][ceil(K / 64)][32768], 16-byte aligned. A row that does not fit the form
-// has the exponent 0x7fffffff: the caller looks for one and keeps the weight as it is.
+// has an exponent of 0x7ffffffe or more: the caller looks for one and keeps the weight as it is.
 extern "C" int llm_weight_digits(const float* w, int N, int K, long long ldw, void* tiles, int* exps, cudaStream_t stream) {
   LLM_REQUIRE(llm_weight_digits_supported(N, K) && ldw >= K && reinterpret_cast<uintptr_t>(tiles) % 16 == 0, "weight_digits: sizes not taken: N=%d K=%d", N, K);
   const int k_blocks = (K + BK - 1) / BK;
@@ -592,7 +594,10 @@ extern "C" int llm_gemm_digits_few(const void* digits, const int* a_exp, const l
   static std::atomic<unsigned long long> done{0};
   int dev = 0;
   if (cudaGetDevice(&dev) == cudaSuccess && !(dev < 64 && (done.load(std::memory_order_relaxed) >> dev & 1ull))) {
-    LLM_REQUIRE(cudaFuncSetAttribute(gemm_digits_few_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, FEW_SMEM) == cudaSuccess,
+    // Loads on their way to registers are held in L1, so no more of it than this may become shared memory: behind a kernel that wants all
+    // of it (float32 decoding attention) the multiprocessors would be left as they are, and 16,384 outputs of 2,048 inputs take 31 us, not 21.
+    LLM_REQUIRE(cudaFuncSetAttribute(gemm_digits_few_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, FEW_SMEM) == cudaSuccess &&
+                    cudaFuncSetAttribute(gemm_digits_few_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, 45) == cudaSuccess,
                 "gemm_digits_few: cannot reserve shared memory");
     if (dev < 64) done.fetch_or(1ull << dev);
   }

@@ -482,7 +482,7 @@ class CudaOps:
         tiles = torch.empty(size, dtype=torch.uint8, device=w.device)
         exps = torch.empty(n, dtype=torch.int32, device=w.device)
         self._check(lib.llm_weight_digits(_ptr(w), c_int(n), c_int(k), c_longlong(w.stride(0)), _ptr(tiles), _ptr(exps), _stream()), lib)
-        if bool((exps == 0x7fffffff).any()):  # (waits: products read a weight ahead of what the stream is still running)
+        if bool((exps >= 0x7ffffffe).any()):  # (waits: products read a weight ahead of what the stream is still running)
             return None
         return DigitWeight(tiles, exps, n, k)
 
