@@ -974,8 +974,9 @@ class CudaOps:
                     self.launches += 1  # the kernel that merges the splits
                 return out
         lib = self.lib()
+        rows16 = q.dtype == torch.float32 and (q.data_ptr() | kcache.data_ptr() | vcache.data_ptr()) % 16 == 0 and q.stride(0) % 4 == 0
         floats = int(lib.llm_paged_attention_simt_scratch(c_int(batch.n_seqs), c_int(n_tokens), c_int(batch.max_new_tokens), c_int(batch.max_seq_len),
-                                                          c_int(nq), c_int(nkv), c_int(hd)))
+                                                          c_int(nq), c_int(nkv), c_int(hd), c_int(rows16)))
         scratch = batch.ws.get("attention.segments", (floats,), torch.float32) if floats else None
         self._check(lib.llm_paged_attention_simt(_ptr(q), c_longlong(q.stride(0)), _ptr(kcache), _ptr(vcache),
                                                  c_int(dtype_code(q.dtype)), _ptr(batch.positions), _ptr(batch.seq_start), _ptr(batch.seq_ntok),

@@ -126,3 +126,24 @@ def test_tiles_that_are_part_empty(ops, dt, nq, nkv, hd, window, seqs):
         K, V = dense[s]
         ref = _attention_ref(q[i].view(nq, hd).cpu().double(), K.double(), V.double(), pos, nq, nkv, hd, scale, window)
         torch.testing.assert_close(out[i].float().cpu(), ref.float(), rtol=2.0 ** -8 if dt == torch.bfloat16 else 2e-5, atol=2e-5)
+
+
+@pytest.mark.parametrize("nq,nkv,hd,page,window", [(4, 4, 64, 16, 0), (16, 2, 128, 16, 0), (3, 1, 20, 4, 0), (10, 2, 64, 8, 700)])
+@pytest.mark.parametrize("lengths", [(1, 1023, 1024, 1025), (2048, 2049, 5, 1500), (4096, 300, 129, 3100), (4097, 64, 2000, 1)])
+def test_single_tokens_behind_many_segments(ops, nq, nkv, hd, page, window, lengths):
+    """Single tokens of several requests, up to 4 segments of 128 keys a CTA and beyond (where segments and a merge take over), against
+    the last token of portions of five: bit-equal, whatever the other requests' lengths."""
+    kc, vc, table, dense = _paged_setup(torch.float32, nkv, hd, page, list(lengths), sum(-(-n // page) for n in lengths) + 2, seed=hd)
+    q = torch.randn(len(lengths), 5, nq * hd, generator=torch.Generator().manual_seed(12)).to(DEV)
+    rows = q[:, -1].contiguous()
+    out = torch.full_like(rows, float("nan"))
+    ops.paged_attention(rows, kc, vc, Batch([(n - 1, 1) for n in lengths]), table, out, nq, nkv, hd, 0.2, window)
+    for i, n in enumerate(lengths):
+        m = min(n, 5)
+        portion, rows_i = torch.empty(m, nq * hd, device=DEV), q[i, 5 - m:].contiguous()
+        ops.paged_attention(rows_i, kc, vc, Batch([(n - m, m)]), table[i:i + 1].contiguous(), portion, nq, nkv, hd, 0.2, window)
+        if m > 1:
+            assert torch.equal(portion[-1], out[i]), n
+        K, V = dense[i]
+        ref = _attention_ref(rows[i].view(nq, hd).cpu().double(), K.double(), V.double(), n - 1, nq, nkv, hd, 0.2, window)
+        torch.testing.assert_close(out[i].cpu(), ref.float(), rtol=2e-5, atol=2e-5)
