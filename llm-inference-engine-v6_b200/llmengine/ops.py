@@ -84,6 +84,11 @@ def _stream():
     return c_void_p(torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()))
 
 
+def _raw_stream() -> int:
+    """The same for a launcher with argument types."""
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+
+
 def _need(t: torch.Tensor, name: str, dtype=None, rows_contiguous: bool = True) -> None:
     if t.is_cuda and (dtype is None or t.dtype is dtype) and (not rows_contiguous or t.is_contiguous()):
         return  # (what nearly every operand is; the questions below cost three times as much)
@@ -269,17 +274,22 @@ class CudaOps:
         without bias) out = w * (x - mean(x)) / sqrt(mean((x - mean(x))^2) + eps).
         With `delta` and write_back, h[r] is replaced by x (the fused residual sum).
         With `rows` (int32), output row i reads source row rows[i] and h is left as it is. digits: where the rows go as digits too."""
-        _need(h, "rmsnorm.h", torch.float32); _need(weight, "rmsnorm.weight", torch.float32); _need(out, "rmsnorm.out")
+        f32 = torch.float32
+        if not (h.dtype is f32 and weight.dtype is f32 and h.is_cuda and weight.is_cuda and out.is_cuda and weight.is_contiguous()):
+            _need(h, "rmsnorm.h", f32); _need(weight, "rmsnorm.weight", f32); _need(out, "rmsnorm.out")
         lib = self.lib()
-        dim = h.shape[-1]
-        n_out = (rows.numel() if n_rows is None else n_rows) if rows is not None else (h.shape[0] if n_rows is None else n_rows)
-        assert h.is_contiguous() and out.is_contiguous() and weight.numel() == dim and out.shape[-1] == dim
-        assert out.shape[0] >= n_out
+        h_shape, out_shape = h.shape, out.shape  # (each question of a tensor costs some 0.2 us: asked once)
+        dim = h_shape[-1]
+        n_out = (rows.numel() if n_rows is None else n_rows) if rows is not None else (h_shape[0] if n_rows is None else n_rows)
+        assert h.is_contiguous() and out.is_contiguous() and weight.numel() == dim and out_shape[-1] == dim
+        assert out_shape[0] >= n_out
         n_part, pstride = 0, 0
         if delta is not None:
-            _need(delta, "rmsnorm.delta", torch.float32)
-            assert delta.is_contiguous() and delta.shape[-1] == dim
-            n_part, pstride = (delta.shape[0], delta.shape[1] * dim) if delta.dim() == 3 else (1, 0)
+            if not (delta.dtype is f32 and delta.is_cuda):
+                _need(delta, "rmsnorm.delta", f32)
+            shape = delta.shape
+            assert delta.is_contiguous() and shape[-1] == dim
+            n_part, pstride = (shape[0], shape[1] * dim) if len(shape) == 3 else (1, 0)
         if rows is not None:
             _need(rows, "rmsnorm.rows", torch.int32)
             write_back = False
@@ -288,8 +298,9 @@ class CudaOps:
             self._check(lib.llm_rmsnorm_digits(_at(h), _at(delta), n_part, pstride, _at(weight), _at(rows), _at(out), n_out, dim, eps, back,
                                                1 if center else 0, *digits.args(), _stream()), lib)
             return out
-        self._check(lib.llm_rmsnorm(_at(h), _at(delta), n_part, pstride, _at(weight), _at(rows), _at(out), dtype_code(out.dtype), n_out, dim,
-                                    eps, back, 1 if center else 0, _stream()), lib)
+        self._check(lib.llm_rmsnorm(h.data_ptr(), None if delta is None else delta.data_ptr(), n_part, pstride, weight.data_ptr(),
+                                    None if rows is None else rows.data_ptr(), out.data_ptr(), dtype_code(out.dtype), n_out, dim, eps, back,
+                                    1 if center else 0, _raw_stream()), lib)
         return out
 
     def residual_add(self, h: torch.Tensor, delta: torch.Tensor, n_rows: Optional[int] = None) -> torch.Tensor:
@@ -355,14 +366,16 @@ class CudaOps:
         exists; otherwise the product runs first (as partial sums when few tokens are in the step)."""
         _need(a, "gemm_swiglu.a"); _need(w_blocked, "gemm_swiglu.w", a.dtype); _need(out, "gemm_swiglu.out", a.dtype)
         m, k = a.shape
-        ff = out.shape[1]
-        assert w_blocked.shape == (2 * ff, k) and out.shape[0] == m and out.is_contiguous() and ff % 128 == 0
-        if m > self.SWAP_MAX_TOKENS and (act[0] if isinstance(act, tuple) else act) in self.EPILOGUE_ACTIVATIONS and self._tc_usable(a, w_blocked):
+        rows, ff = out.shape
+        assert w_blocked.shape == (2 * ff, k) and rows == m and out.is_contiguous() and ff % 128 == 0
+        operands = None
+        if m > self.SWAP_MAX_TOKENS and (act[0] if isinstance(act, tuple) else act) in self.EPILOGUE_ACTIVATIONS:
+            operands = self._tc_operands(a, w_blocked)
+        if operands is not None:
             assert row_scale is None, "a row scale is applied where partial sums are consumed (few tokens)"
             lib = self.lib("tensorcore")
-            lda, ldw = k if a.is_contiguous() else a.stride(0), k if w_blocked.is_contiguous() else w_blocked.stride(0)
-            self._check(lib.llm_gemm_tc_swiglu(a.data_ptr(), w_blocked.data_ptr(), out.data_ptr(), m, ff, k, lda, ldw, ff,
-                                               *self._act_args(act), _stream()), lib)
+            _, _, _, lda, ldw, at, wt = operands
+            self._check(lib.llm_gemm_tc_swiglu(at, wt, out.data_ptr(), m, ff, k, lda, ldw, ff, *self._act_args(act), _raw_stream()), lib)
             return out
         assert ws is not None, "gemm_swiglu needs a workspace when it cannot fuse"
         if m <= self.SWAP_MAX_TOKENS:
@@ -380,18 +393,25 @@ class CudaOps:
     # eight times as much and half as many CTAs do better (batch 64: 37.4 k against 36.5 k tokens/s).
     SPLIT_TARGET_CTAS = 296
 
-    def _tc_usable(self, a: torch.Tensor, w: torch.Tensor) -> bool:
-        """bfloat16 operands that the tensor-core kernel takes (16-byte aligned rows of K % 8 == 0)."""
-        if a.dtype != torch.bfloat16 or not self.tensor_cores:
-            return False
+    def _tc_operands(self, a: torch.Tensor, w: torch.Tensor):
+        """(M, N, K, row strides, addresses) of bfloat16 operands that the tensor-core kernel takes (16-byte aligned rows of K % 8 == 0);
+        None of others."""
+        if a.dtype is not torch.bfloat16 or not self.tensor_cores:
+            return None
         if "tma" not in self._known:  # (whether the driver encodes tensor maps: asked of the library once, about operands it takes)
             self._known["tma"] = bool(self.lib("tensorcore").llm_gemm_tc_supported(c_void_p(16), c_void_p(16), c_int(1), c_int(1), c_int(8),
                                                                                    c_longlong(8), c_longlong(8)))
         m, k = a.shape
+        n, kw = w.shape
         # (a row stride is the inner size where nothing lies between the rows: strides are slow to ask for)
-        lda, ldw = k if a.is_contiguous() else a.stride(0), w.shape[1] if w.is_contiguous() else w.stride(0)
-        return (self._known["tma"] and m > 0 and k > 0 and w.shape[0] > 0 and
-                (k | lda | ldw) % 8 == 0 and (a.data_ptr() | w.data_ptr()) % 16 == 0)
+        lda, ldw = k if a.is_contiguous() else a.stride(0), kw if w.is_contiguous() else w.stride(0)
+        at, wt = a.data_ptr(), w.data_ptr()
+        if self._known["tma"] and m > 0 and k > 0 and n > 0 and (k | lda | ldw) % 8 == 0 and (at | wt) % 16 == 0:
+            return m, n, k, lda, ldw, at, wt
+        return None
+
+    def _tc_usable(self, a: torch.Tensor, w: torch.Tensor) -> bool:
+        return self._tc_operands(a, w) is not None
 
     SWAP_MAX_TOKENS = 64  # up to here weights fill the accumulator lanes and tokens the columns, several CTAs an SM
 
@@ -441,21 +461,16 @@ class CudaOps:
 
     ONE_WAVE = 148  # the SMs of a B200, the one device these kernels are built for: one CTA with the long ring each
 
-    def gemm_cuts(self, a: torch.Tensor, w: torch.Tensor) -> bool:
-        """Whether gemm_partials cuts K for these operands, so that a consumer that adds the parts saves the kernel that would."""
-        return self._tc_usable(a, w) and self._form(a.shape[0], w.shape[0], a.shape[1], True)[1] > 1
-
-    def _gemm_tc(self, a, w, out, form, split_stride: int = 0) -> None:
-        M, K = a.shape
-        N = w.shape[0]
+    def _gemm_tc(self, operands, out, form, split_stride: int = 0) -> None:
+        """operands: as _tc_operands gives them."""
+        M, N, K, lda, ldw, at, wt = operands
         swap, splits, stages = form
         if splits == 1 and N < 128 and M > self.SWAP_MAX_TOKENS:
             swap = 0  # fewer outputs than accumulator lanes: tiles of tokens with as many columns as there are outputs (64 outputs of 2,048 inputs, 77 tokens: 12.3 us, 14.0 with the weights on the lanes)
         lib = self.lib("tensorcore")
-        lda, ldw = K if a.is_contiguous() else a.stride(0), K if w.is_contiguous() else w.stride(0)
         ldo = N if out.is_contiguous() else out.stride(-2)
-        self._check(lib.llm_gemm_tc(a.data_ptr(), w.data_ptr(), out.data_ptr(), M, N, K, lda, ldw, ldo, dtype_code(out.dtype), swap, splits,
-                                    split_stride, stages, _stream()), lib)
+        self._check(lib.llm_gemm_tc(at, wt, out.data_ptr(), M, N, K, lda, ldw, ldo, dtype_code(out.dtype), swap, splits, split_stride, stages,
+                                    _raw_stream()), lib)
 
     # Float32 matrices of at least so many numbers, with rows of at least so many, are held as digits. With shorter rows a few rows of
     # activations are faster on CUDA cores (digits, those of the activations made, against CUDA cores, us: 2,048 outputs of 512 inputs 1
@@ -537,14 +552,15 @@ class CudaOps:
             self._gemm_digits(a, w, out)
             return out
         _need(a, "gemm.a"); _need(w, "gemm.w", a.dtype); _need(out, "gemm.out")
-        if self._tc_usable(a, w):
+        operands = self._tc_operands(a, w)
+        if operands is not None:
             form = self._form(M, N, K, ws is not None and out.is_contiguous(), True)
             splits = form[1]
             if splits == 1:
-                self._gemm_tc(a, w, out, form)
+                self._gemm_tc(operands, out, form)
             else:
                 parts = ws.get("gemm.parts", (splits, M, N), torch.float32)
-                self._gemm_tc(a, w, parts, form, M * N)
+                self._gemm_tc(operands, parts, form, M * N)
                 self.reduce_partials(parts, out)
             return out
         lib = self.lib()
@@ -576,21 +592,39 @@ class CudaOps:
                                               *gargs, c_int(1 if gate_per_head else 0), _stream()), lib)
         return True
 
+    def _tc_partials(self, a, w, ws, tag: str, only_cut: bool):
+        operands = self._tc_operands(a, w)
+        if operands is None:
+            return None
+        M, N, K = operands[:3]
+        assert w.shape[1] == K
+        form = self._form(M, N, K, True)
+        if only_cut and form[1] == 1:
+            return None
+        parts = ws.get(tag, (form[1], M, N), torch.float32)
+        self._gemm_tc(operands, parts, form, M * N)
+        return parts
+
+    def gemm_cut_partials(self, a, w, ws, tag: str) -> Optional[torch.Tensor]:
+        """gemm_partials where it cuts K for these operands, so that a consumer that adds the parts saves the kernel that would; else None,
+        with nothing done."""
+        if isinstance(w, DigitWeight):
+            return None
+        _need(a, "gemm.a"); _need(w, "gemm.w", a.dtype)
+        return self._tc_partials(a, w, ws, tag, True)
+
     def gemm_partials(self, a, w, ws, tag: str) -> torch.Tensor:
         """As gemm, for consumers that add partial sums themselves: returns float32 [parts, M, N]
         (scratch `tag` of workspace `ws`); the product is the sum over parts, to be taken in index
         order. parts is 1 in float32 and where K is not cut (_form): the rule asks how many CTAs the
         output's tiles give, so a product of many tokens with few outputs is cut too. a, w: as in gemm."""
-        M, K = a.shape
-        N = w.shape[0]
-        assert w.shape[1] == K
         if not isinstance(w, DigitWeight):
             _need(a, "gemm.a"); _need(w, "gemm.w", a.dtype)
-        if self._tc_usable(a, w):
-            form = self._form(M, N, K, True)
-            parts = ws.get(tag, (form[1], M, N), torch.float32)
-            self._gemm_tc(a, w, parts, form, M * N)
+        parts = self._tc_partials(a, w, ws, tag, False)
+        if parts is not None:
             return parts
+        M, N = a.shape[0], w.shape[0]
+        assert w.shape[1] == a.shape[1]
         parts = ws.get(tag, (1, M, N), torch.float32)
         self.gemm(a, w, parts[0], ws)
         return parts
@@ -824,27 +858,38 @@ class CudaOps:
         sums over parts (times row_scale, if given); then only the q section of qkv is written (k and v
         go to the cache)."""
         assert row_scale is None or parts is not None
-        _need(qkv, "rope.qkv"); _need(positions, "rope.positions", torch.int32)
-        _need(token_seq, "rope.token_seq", torch.int32); _need(block_table, "rope.block_table", torch.int32)
-        page_size = 1
+        f32, i32 = torch.float32, torch.int32
+        dtype = qkv.dtype
+        if not (qkv.is_cuda and qkv.is_contiguous() and positions.dtype is i32 and positions.is_cuda and positions.is_contiguous() and
+                token_seq.dtype is i32 and token_seq.is_cuda and token_seq.is_contiguous() and block_table.dtype is i32 and block_table.is_cuda):
+            _need(qkv, "rope.qkv"); _need(positions, "rope.positions", i32)
+            _need(token_seq, "rope.token_seq", i32); _need(block_table, "rope.block_table", i32)
+        page_size, k_at, v_at, cos_at, sin_at, parts_at = 1, None, None, None, None, None
         if kcache is not None:
-            _need(kcache, "rope.kcache", qkv.dtype); _need(vcache, "rope.vcache", qkv.dtype)
-            assert kcache.is_contiguous() and vcache.is_contiguous() and kcache.shape == vcache.shape
-            assert kcache.shape[1] == nkv and kcache.shape[3] == hd
-            page_size = kcache.shape[2]
+            if not (kcache.dtype is dtype and vcache.dtype is dtype and kcache.is_cuda and vcache.is_cuda):
+                _need(kcache, "rope.kcache", dtype); _need(vcache, "rope.vcache", dtype)
+            shape = kcache.shape
+            assert kcache.is_contiguous() and vcache.is_contiguous() and shape == vcache.shape
+            assert shape[1] == nkv and shape[3] == hd
+            page_size, k_at, v_at = shape[2], kcache.data_ptr(), vcache.data_ptr()
         if cos is not None:
-            _need(cos, "rope.cos", torch.float32); _need(sin, "rope.sin", torch.float32)
+            if not (cos.dtype is f32 and sin.dtype is f32 and cos.is_cuda and sin.is_cuda):
+                _need(cos, "rope.cos", f32); _need(sin, "rope.sin", f32)
             assert cos.is_contiguous() and sin.is_contiguous() and cos.shape[1] == hd // 2
-        assert qkv.shape[1] == (nq + 2 * nkv) * hd and block_table.is_contiguous()
+            cos_at, sin_at = cos.data_ptr(), sin.data_ptr()
+        width, blocks = qkv.shape[1], block_table.shape[1]
+        assert width == (nq + 2 * nkv) * hd and block_table.is_contiguous()
         lib = self.lib()
         n_parts, pstride = 0, 0
         if parts is not None:
-            _need(parts, "rope.parts", torch.float32)
-            assert parts.is_contiguous() and parts.dim() == 3 and parts.shape[2] == qkv.shape[1] and parts.shape[1] >= n_tokens
-            n_parts, pstride = parts.shape[0], parts.stride(0)
-        self._check(lib.llm_rope_kv_write(_at(qkv), qkv.stride(0), dtype_code(qkv.dtype), _at(parts), n_parts, pstride, _at(positions),
-                                          _at(token_seq), _at(block_table), block_table.shape[1], _at(cos), _at(sin), _at(kcache), _at(vcache),
-                                          n_tokens, nq, nkv, hd, page_size, *_row_scale_args(row_scale), _stream()), lib)
+            if not (parts.dtype is f32 and parts.is_cuda):
+                _need(parts, "rope.parts", f32)
+            shape = parts.shape
+            assert parts.is_contiguous() and len(shape) == 3 and shape[2] == width and shape[1] >= n_tokens
+            n_parts, pstride, parts_at = shape[0], shape[1] * width, parts.data_ptr()
+        self._check(lib.llm_rope_kv_write(qkv.data_ptr(), width if qkv.is_contiguous() else qkv.stride(0), dtype_code(dtype), parts_at, n_parts, pstride,
+                                          positions.data_ptr(), token_seq.data_ptr(), block_table.data_ptr(), blocks, cos_at, sin_at, k_at, v_at,
+                                          n_tokens, nq, nkv, hd, page_size, *_row_scale_args(row_scale), _raw_stream()), lib)
 
     # decoding: the key range is cut at absolute multiples of `split_keys` (a multiple of 64); see _split_policy
     ATTENTION_TARGET_CTAS = 592
@@ -931,22 +976,29 @@ class CudaOps:
         context (positions, token_seq, seq_start, seq_ntok, seq_qoff, the counts, scratch).
         bfloat16 with head sizes 16/32/64/128 runs on tensor cores (with the key range cut into
         splits when every request brings one token); anything else on CUDA cores in float32."""
-        _need(q, "attention.q"); _need(kcache, "attention.kcache", q.dtype); _need(vcache, "attention.vcache", q.dtype)
-        _need(out, "attention.out", q.dtype); _need(block_table, "attention.block_table", torch.int32)
+        dtype = q.dtype
+        if not (q.is_cuda and kcache.dtype is dtype and vcache.dtype is dtype and out.dtype is dtype and kcache.is_cuda and vcache.is_cuda and
+                out.is_cuda and out.is_contiguous() and block_table.dtype is torch.int32 and block_table.is_cuda):
+            _need(kcache, "attention.kcache", dtype); _need(vcache, "attention.vcache", dtype)
+            _need(out, "attention.out", dtype); _need(block_table, "attention.block_table", torch.int32)
+        _need(q, "attention.q")
+        pages, heads, page, size = kcache.shape
         assert kcache.is_contiguous() and vcache.is_contiguous() and block_table.is_contiguous()
-        assert kcache.shape[1] == nkv and kcache.shape[3] == hd
-        n_tokens, page = batch.n_tokens, kcache.shape[2]
-        if q.dtype == torch.bfloat16 and self.tensor_cores:
+        assert heads == nkv and size == hd
+        n_tokens = batch.n_tokens
+        if dtype is torch.bfloat16 and self.tensor_cores:
             lib = self.lib("tensorcore")
-            if (self.tcgen05_attention and batch.max_new_tokens >= self.TC_ATTENTION_MIN_TOKENS and
-                    block_table.shape[1] <= self.TC_ATTENTION_MAX_BLOCKS and
-                    self._answer(lib, "llm_attention_tc_supported", nq, nkv, hd, page, q.stride(0), out.stride(0))):
+            ld_q, (out_rows, ld_out), blocks = q.stride(0), out.shape, block_table.shape[1]
+            if not out.is_contiguous():
+                ld_out = out.stride(0)
+            if (self.tcgen05_attention and batch.max_new_tokens >= self.TC_ATTENTION_MIN_TOKENS and blocks <= self.TC_ATTENTION_MAX_BLOCKS and
+                    self._answer(lib, "llm_attention_tc_supported", nq, nkv, hd, page, ld_q, ld_out)):
                 # prompt portions: tcgen05 kernel (128 rows per CTA, scores and output in tensor memory)
                 work = batch.ws.get_zeroed("attention.work_counters", (2,), torch.int32)  # left at zero by the kernel
                 self._check(lib.llm_paged_attention_tc(
-                    _at(q), q.stride(0), _at(kcache), _at(vcache), kcache.shape[0], _at(batch.seq_start), _at(batch.seq_ntok), _at(batch.seq_qoff),
-                    _at(block_table), block_table.shape[1], _at(out), out.stride(0), batch.n_seqs, batch.max_new_tokens, nq, nkv, hd, page,
-                    scale, window, q.shape[0], _at(work), _stream()), lib)
+                    q.data_ptr(), ld_q, kcache.data_ptr(), vcache.data_ptr(), pages, batch.seq_start.data_ptr(), batch.seq_ntok.data_ptr(),
+                    batch.seq_qoff.data_ptr(), block_table.data_ptr(), blocks, out.data_ptr(), ld_out, batch.n_seqs, batch.max_new_tokens, nq, nkv, hd,
+                    page, scale, window, q.shape[0], work.data_ptr(), _raw_stream()), lib)
                 return out
             decode_only = batch.max_new_tokens == 1 and batch.n_tokens == batch.n_seqs
             use_tma = decode_only and self.tma_decode_attention and lib.llm_attention_decode_supported(

@@ -67,7 +67,7 @@ class PagedAttention(Mixer):
         """The step has few enough tokens for the products that add their K pieces inside a cluster and
         take the work around them in (ops.gemm_few_tokens)."""
         s, ops, n = self.spec, self.env.ops, ctx.n_tokens
-        return (self.env.dtype == torch.bfloat16 and hasattr(ops, "gemm_few_tokens") and
+        return (self.env.dtype == torch.bfloat16 and getattr(ops, "few_token_products", False) and
                 ops.few_token_splits(self.w_qkv.shape[0], s.hidden, n, "plain") > 0 and
                 ops.few_token_splits(s.hidden, s.num_heads * s.head_dim, n, "residual") > 0)
 
@@ -98,7 +98,10 @@ class PagedAttention(Mixer):
                 x = x.dense(ctx)
         if not isinstance(x, NormalizedRows) and x.shape[0] != n:
             x = x[:n]
-        if cache.writes and self.position.takes_partial_sums and (n <= 64 or (hasattr(ops, "gemm_cuts") and ops.gemm_cuts(x, self.w_qkv))):
+        parts = None
+        if n > 64 and cache.writes and self.position.takes_partial_sums and hasattr(ops, "gemm_cut_partials"):
+            parts = ops.gemm_cut_partials(x, self.w_qkv, ctx.ws, "attention.qkv_parts")  # None: not cut
+        if cache.writes and self.position.takes_partial_sums and (n <= 64 or parts is not None):
             # few tokens: the product comes as float32 sums (in parts, unless the K pieces were added
             # inside the product), finished by the position kernel or by the attention kernel
             if few:
@@ -107,7 +110,7 @@ class PagedAttention(Mixer):
                     ops.gemm_few_tokens(self.w_qkv, parts[0], "plain", norm=(x.h, x.sumsq, x.weight, x.eps, x.rows), n_tokens=n, ws=ctx.ws)
                 else:
                     ops.gemm_few_tokens(self.w_qkv, parts[0], "plain", x=x, ws=ctx.ws)
-            else:
+            elif parts is None:
                 parts = ops.gemm_partials(x, self.w_qkv, ctx.ws, "attention.qkv_parts")
             tables = self.position.rotation_tables() if cache.k is not None else None
             if tables is not None and ops.decode_attention_fusable(ctx, cache.k, s.num_heads, s.num_kv_heads, s.head_dim, att):

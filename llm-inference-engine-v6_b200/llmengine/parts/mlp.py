@@ -59,7 +59,7 @@ class GatedMLP(FeedForward):
 
     def _few_tokens(self, ctx) -> bool:
         s, ops, n = self.spec, self.env.ops, ctx.n_tokens
-        return (self.blocked and s.activation == "silu" and hasattr(ops, "gemm_few_tokens") and
+        return (self.blocked and s.activation == "silu" and getattr(ops, "few_token_products", False) and
                 ops.few_token_splits(2 * s.intermediate, s.hidden, n, "swiglu") > 0 and
                 ops.few_token_splits(s.hidden, s.intermediate, n, "residual") > 0)
 
