@@ -12,6 +12,7 @@
 #include "common.cuh"
 #include "mma_common.cuh"
 
+#include <algorithm>
 #include <cmath>
 
 namespace {
@@ -116,12 +117,15 @@ __global__ void __launch_bounds__(RM_THREADS)
 
 
 // Few rows an expert (steps of single tokens): a tile of 16 rows x 64 columns, the four warps side by side along the
-// columns, and a ring of six stages: the expert's matrix is all that moves, and what bounds the kernel is how many of
-// its bytes are on their way to an SM at a time (a stage holds 9 KB of it and 2 KB of rows).
-constexpr int RS_ROWS = 16, RS_STAGES = 6;
-constexpr size_t RS_SMEM = (size_t)RS_STAGES * (RS_ROWS + RM_COLS) * RM_LD * sizeof(bf16);
+// columns, and a ring of six stages, or four: the expert's matrix is all that moves, and what bounds the kernel is how many of
+// its bytes are on their way to an SM at a time (a stage holds 9 KB of it and 2 KB of rows). With six stages three CTAs share a
+// multiprocessor, with four four: where the tiles that are likely there are more than 3 x 148 and no more than 4 x 148, the shorter rings
+// spare a second round for a few (8 tokens by 4 of 16 experts of 2,048 x 2,048, 460 CTAs: a step of three such layers 684 us with six, 662 with four;
+// 4 tokens, 350 CTAs: 610 with six stages, 633 with four).
+constexpr int RS_ROWS = 16;
+constexpr size_t rs_smem(int stages) { return (size_t)stages * (RS_ROWS + RM_COLS) * RM_LD * sizeof(bf16); }
 
-template <typename TO, int EPI>
+template <typename TO, int EPI, int RS_STAGES>
 __global__ void __launch_bounds__(RM_THREADS)
     routed_product_mma_few_kernel(const bf16* __restrict__ a, long long lda, int a_div, const bf16* __restrict__ w, long long w_stride, int N,
                                   int K, const int* __restrict__ tile_expert, const int* __restrict__ tile_rows, TO* __restrict__ out,
@@ -318,10 +322,29 @@ int launch_routed(dim3 grid, cudaStream_t stream, const void* a, long long lda, 
   return 0;
 }
 
+template <typename TO, int EPI, int STAGES>
+int launch_few_stages(int max_tiles, cudaStream_t stream, const void* a, long long lda, int a_div, const void* w, int N, int K, const int* tile_expert,
+                      const int* tile_rows, void* out, long long ldo, const float* share, int act, float p0, float p1) {
+  auto kernel = routed_product_mma_few_kernel<TO, EPI, STAGES>;
+  static bool raised = false;
+  if (!raised) {
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rs_smem(STAGES)) != cudaSuccess) return 1;
+    raised = true;
+  }
+  launch_kernel(kernel, dim3(ceil_div(N, RM_COLS), max_tiles), RM_THREADS, rs_smem(STAGES), stream, (const bf16*)a, lda, a_div, (const bf16*)w,
+                (long long)N * K, N, K, tile_expert, tile_rows, (TO*)out, ldo, share, act, p0, p1);
+  return 0;
+}
+template <typename TO, int EPI, typename... Args>
+int launch_few(bool four, Args... args) {
+  return four ? launch_few_stages<TO, EPI, 4>(args...) : launch_few_stages<TO, EPI, 6>(args...);
+}
+
+// likely_tiles: how many of the tiles are likely there (for the choice of a form; any number gives the same results).
 // tile: the rows of a tile of tile_rows (16 or 64, as llm_routed_product_mma_rows said when the pairs were grouped).
 extern "C" int llm_routed_product_mma(const void* a, long long lda, int a_div, const void* w, int N, int K, const int* tile_expert,
                                       const int* tile_rows, int max_tiles, int tile, void* out, long long ldo, int epilogue,
-                                      const float* share, int act, float p0, float p1, cudaStream_t stream) {
+                                      const float* share, int act, float p0, float p1, int likely_tiles, cudaStream_t stream) {
   // act, p0, p1: the activation of epilogue 2 (0: silu; 2: both sides limited by p0, slope p1)
   if (max_tiles == 0) return LLM_OK;
   LLM_REQUIRE(act >= 0 && act <= 2, "routed_product_mma: unknown activation %d", act);
@@ -330,29 +353,13 @@ extern "C" int llm_routed_product_mma(const void* a, long long lda, int a_div, c
   LLM_REQUIRE(tile == RS_ROWS || tile == RM_ROWS, "routed_product_mma: tiles of %d rows (16 or 64)", tile);
   LLM_REQUIRE(epilogue == 0 || epilogue == 1 || epilogue == 3 || (epilogue == 2 && N % 2 == 0), "routed_product_mma: unknown epilogue %d", epilogue);
   if (tile == RS_ROWS) {
-    static bool raised_few = false;
-    if (!raised_few) {
-      LLM_REQUIRE(cudaFuncSetAttribute(routed_product_mma_few_kernel<bf16, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)RS_SMEM) == cudaSuccess &&
-                  cudaFuncSetAttribute(routed_product_mma_few_kernel<bf16, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)RS_SMEM) == cudaSuccess &&
-                  cudaFuncSetAttribute(routed_product_mma_few_kernel<bf16, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)RS_SMEM) == cudaSuccess &&
-                  cudaFuncSetAttribute(routed_product_mma_few_kernel<float, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)RS_SMEM) == cudaSuccess,
-                  "routed_product_mma: cannot raise the shared memory limit");
-      raised_few = true;
-    }
-    dim3 grid_few(ceil_div(N, RM_COLS), max_tiles);
-    const long long wsf = (long long)N * K;
-    if (epilogue == 0)
-      launch_kernel(routed_product_mma_few_kernel<bf16, 0>, grid_few, RM_THREADS, RS_SMEM, stream, (const bf16*)a, lda, a_div, (const bf16*)w, wsf,
-                    N, K, tile_expert, tile_rows, (bf16*)out, ldo, share, act, p0, p1);
-    else if (epilogue == 2)
-      launch_kernel(routed_product_mma_few_kernel<bf16, 2>, grid_few, RM_THREADS, RS_SMEM, stream, (const bf16*)a, lda, a_div, (const bf16*)w, wsf,
-                    N, K, tile_expert, tile_rows, (bf16*)out, ldo, share, act, p0, p1);
-    else if (epilogue == 3)
-      launch_kernel(routed_product_mma_few_kernel<bf16, 3>, grid_few, RM_THREADS, RS_SMEM, stream, (const bf16*)a, lda, a_div, (const bf16*)w, wsf,
-                    N, K, tile_expert, tile_rows, (bf16*)out, ldo, share, act, p0, p1);
-    else
-      launch_kernel(routed_product_mma_few_kernel<float, 1>, grid_few, RM_THREADS, RS_SMEM, stream, (const bf16*)a, lda, a_div, (const bf16*)w, wsf,
-                    N, K, tile_expert, tile_rows, (float*)out, ldo, share, act, p0, p1);
+    const long long ctas = (long long)ceil_div(N, RM_COLS) * std::min(likely_tiles, max_tiles);
+    const bool four = ctas > 3 * 148 && ctas <= 4 * 148;
+    const int rc = epilogue == 0   ? launch_few<bf16, 0>(four, max_tiles, stream, a, lda, a_div, w, N, K, tile_expert, tile_rows, out, ldo, share, act, p0, p1)
+                   : epilogue == 2 ? launch_few<bf16, 2>(four, max_tiles, stream, a, lda, a_div, w, N, K, tile_expert, tile_rows, out, ldo, share, act, p0, p1)
+                   : epilogue == 3 ? launch_few<bf16, 3>(four, max_tiles, stream, a, lda, a_div, w, N, K, tile_expert, tile_rows, out, ldo, share, act, p0, p1)
+                                   : launch_few<float, 1>(four, max_tiles, stream, a, lda, a_div, w, N, K, tile_expert, tile_rows, out, ldo, share, act, p0, p1);
+    LLM_REQUIRE(rc == 0, "routed_product_mma: cannot raise the shared memory limit");
     LLM_CHECK_LAUNCH("routed_product_mma");
     return LLM_OK;
   }

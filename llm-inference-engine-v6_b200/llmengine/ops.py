@@ -1454,7 +1454,7 @@ class CudaOps:
                                                    _ptr(tile_expert), _ptr(tile_rows), c_int(tile_expert.numel()),
                                                    c_int(tile_rows.shape[1]), _ptr(out),
                                                    c_longlong(out.stride(0)), c_int(self.ROUTED_EPILOGUES[epilogue]), _ptr(share),
-                                                   *act_args, _stream()), lib)
+                                                   *act_args, c_int(round(E * (1.0 - (1.0 - 1.0 / E) ** out.shape[0]))), _stream()), lib)
             return out
         assert tile_rows.shape[1] == self.routed_tile_rows()
         lib = self.lib()

@@ -81,3 +81,31 @@ def test_routed_products_tensor_cores_against_cuda_cores_and_formula(E, N, K, pa
         ops.routed_product(x.repeat_interleave(pairs_per_token, 0).contiguous(), 1, w, te, tr, y, "share", share=share)
         want = picked * share.double().cpu()[:, None]
         assert (y.double().cpu() - want).abs().max() < 1e-3 * max(1.0, want.abs().max().item())
+
+
+@pytest.mark.parametrize("N,K,n", [(2040, 8, 8), (2040, 200, 8), (2048, 264, 16), (2040, 2048, 11)])
+def test_routed_products_of_few_rows_have_the_same_bits_with_rings_of_four_and_six_stages(N, K, n):
+    """From 445 to 592 likely CTAs (32 column tiles by 14 to 16 of 16 experts) the ring has four stages; the same rows by the first and the
+    last few columns alone, a CTA an expert, go through the ring of six: both add the same products in one order."""
+    ops = get_ops()
+    from llmengine.engine.context import Workspace
+    ws = Workspace(DEV)
+    E, top = 16, 4
+    g = torch.Generator().manual_seed(N + K + n)
+    x = torch.randn(n, K, generator=g).to(torch.bfloat16).to(DEV)
+    w = (torch.randn(E, N, K, generator=g) * 0.2).to(torch.bfloat16).to(DEV)
+    idx = torch.stack([torch.randperm(E, generator=g)[:top] for _ in range(n)]).to(torch.int32).to(DEV)
+    te, tr = ops.routed_group(idx, E, 16, ws, "few")
+    for epilogue, dtype in (("gelu", torch.bfloat16), ("share", torch.float32), ("relu_squared", torch.bfloat16), ("silu_pairs", torch.bfloat16)):
+        def run(cols):
+            part = w[:, cols].contiguous()
+            rows, a_div = (x.repeat_interleave(top, 0).contiguous(), 1) if epilogue == "share" else (x, top)
+            out = torch.zeros(n * top, part.shape[1] // (2 if epilogue == "silu_pairs" else 1), dtype=dtype, device=DEV)
+            return ops.routed_product(rows, a_div, part, te, tr, out, epilogue)
+        whole, first, last = run(slice(0, N)), run(slice(0, 64)), run(slice(N - 24, N))
+        assert torch.equal(whole[:, :first.shape[1]], first) and torch.equal(whole[:, -last.shape[1]:], last), epilogue
+        if epilogue == "share":  # float32 sums of bfloat16 products: K roundings of 2^-24 of the terms' sizes, kept loosely
+            pairs = [(p, idx.reshape(-1)[p].item()) for p in range(n * top)]
+            want = torch.stack([w[e].double().cpu() @ x[p // top].double().cpu() for p, e in pairs])
+            size = torch.stack([w[e].double().cpu().abs() @ x[p // top].double().cpu().abs() for p, e in pairs])
+            assert ((whole.double().cpu() - want).abs() <= K * 2.0 ** -24 * size + 1e-30).all()
