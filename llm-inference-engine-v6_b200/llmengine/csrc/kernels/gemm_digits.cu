@@ -26,9 +26,10 @@
 // of what memory gives fastest, one piece. (Made into digits on their way into shared memory by sixteen warps they came at 5.2 TB/s in the
 // longest product and 1.3 to 3.8 in a layer's.) The activations are written as digits by a kernel of their own and come by TMA, plane
 // behind plane (64-byte swizzle) with the highest first: the planes i + j >= 3 that a weight digit i meets are the first i + 1, its products
-// with them lie in neighbouring accumulators, and one instruction forms them all: 4 for 32 k with up to 64 tokens, not 10 (an
-// instruction takes 80 clocks at least, else 2 a column: kind::i8 runs at 2,048 multiply-adds a clock and multiprocessor, which bounds
-// the product from about 32 tokens on).
+// with them lie in neighbouring accumulators, and one instruction forms them all: 4 for 32 k, not 10. Tiles have at most 64 tokens, so
+// that two CTAs share a multiprocessor and one's products run while the other waits for its copies or writes its results: 2,048 rows by
+// 16,384 outputs of 2,048 inputs 632 us, 3,800 multiply-adds a clock and multiprocessor (tiles of 128 tokens, one CTA: 781); 300 rows
+// 140 us (as three or four tiles of more than 64: 162, 182). The rate of the unit bounds the product from about 64 tokens on.
 // The reference computes the same products with a scalar loop (matmul_f32, src/kernels.cpp:33-57).
 #include "digits.cuh"
 #include "tc_common.cuh"
@@ -43,7 +44,7 @@ constexpr int READERS = 8, WARP_COPY = READERS, WARP_MMA = READERS + 1;  // warp
 constexpr int DIGIT_THREADS = (READERS + 2) * 32;
 constexpr int W_BYTES = 4 * BM * BK;  // of a tile of weights (BK = 64 k)
 constexpr int LEVELS = 4;
-constexpr int MAX_TOKENS = 128;    // of a tile: four accumulators of 128 columns are tensor memory's 512
+constexpr int MAX_TOKENS = 64;     // of a tile: four accumulators of 64 columns, and two CTAs, are tensor memory's 512
 
 // A block's largest of one number a thread (256 threads).
 __device__ __forceinline__ uint32_t block_largest(uint32_t v, uint32_t* red) {
@@ -283,7 +284,6 @@ __global__ void __launch_bounds__(DIGIT_THREADS, 2) gemm_digits_kernel(const __g
   } else if (warp == WARP_MMA && lane == 0) {
     // ---------------------------------------------------------------- products
     // (what does not change is worked out before the loop: made anew, descriptors took the thread 200 clocks an instruction)
-    const int together = min(4, 256 / p.bn);  // planes of activations that one instruction takes
     const uint64_t desc_w = smem_desc_sw128(smem_u32(smem)), desc_a = smem_desc_sw64(smem_u32(smem) + W_BYTES);
     uint32_t idesc[4];
 #pragma unroll
@@ -299,12 +299,7 @@ __global__ void __launch_bounds__(DIGIT_THREADS, 2) gemm_digits_kernel(const __g
         for (int i = 3; i >= 0; --i) {  // (digit 3 first: it meets all four planes, and so begins every accumulator)
           const uint64_t dw = desc_w + (at + (uint32_t)((i >> 1) * (BM * 128 / 16) + (i & 1) * 4 + half * 2)), da = desc_a + (at + (uint32_t)(half * 2));
           const uint32_t more = it > 0 || half > 0 || i < 3 ? 1u : 0u;
-          if (together == 4) {
-            mma_i8(tmem_base + (uint32_t)((3 - i) * p.bn), dw, da, idesc[i], more);
-          } else {
-            for (int b = 0; b <= i; b += together)
-              mma_i8(tmem_base + (uint32_t)((3 - i + b) * p.bn), dw, da + (uint32_t)(b * p.bn * BK / 16), digit_instr_desc(min(together, i + 1 - b) * p.bn), more);
-          }
+          mma_i8(tmem_base + (uint32_t)((3 - i) * p.bn), dw, da, idesc[i], more);
         }
       }
       mma_commit(&empty[ring.s]);
@@ -489,22 +484,25 @@ __global__ void __launch_bounds__(FEW_WARPS * 32, 1) gemm_digits_few_kernel(cons
 
 constexpr int SMS = 148;  // of a B200
 
-// Tokens of a tile and pieces that K is cut into (a cluster), by the clocks that the last CTA is done after: a k-block takes the longer of
-// its weights' way from memory, 1,400 at the rate that all have together, and its products, twenty of 2 clocks a token; a CTA's beginning
-// and end some 4,000. Of up to 64 tokens two CTAs share a multiprocessor.
+// Tokens of a tile and pieces that K is cut into (a cluster), by the clocks that the last CTA is done after: rounds of two CTAs a
+// multiprocessor, or of one where they do not suffice. A k-block takes the longer of its weights' way from memory, 1,400 at the rate that
+// all have together, and its products, twenty of a clock a token; the two-stage ring of a CTA alone leaves some 600 in which nothing
+// runs. A CTA's beginning and end are some 4,000, the exchange of a cluster's sums 1,500. Of more than 64 tokens tiles of 48 are tried as
+// well, which fill the last round better (us with 64, with 48: 160 x 16,384 x 2,048 94, 84; 1,024 x 3,072 x 2,048 94, 79; 300 x 2,048 x 8,192
+// 85, 76; but 2,048 x 16,384 x 2,048 632, 731).
 void choose_tiles(int M, int n_tiles, int k_blocks, int only_cuts, int* bn, int* t_tiles, int* cuts) {
   long long best = 1LL << 62;
-  const int least = (M + MAX_TOKENS - 1) / MAX_TOKENS;
-  for (int t = least; t <= least + 2; ++t) {
-    const int tokens = ((M + t - 1) / t + 15) / 16 * 16, together = tokens <= 64 ? 2 : 1;
+  const int splits[2] = {(M + MAX_TOKENS - 1) / MAX_TOKENS, M > MAX_TOKENS ? (M + 47) / 48 : 1};
+  for (int t : splits) {
+    const int tokens = ((M + t - 1) / t + 15) / 16 * 16;
     const long long tiles = (long long)n_tiles * t;
     for (int c = 1; c <= 8; c *= 2) {
-      if (only_cuts ? c != only_cuts : c > 1 && (tiles * c > SMS * together || 2 * c > k_blocks)) continue;
-      const long long per = (k_blocks + c - 1) / c, ctas = tiles * c, block = std::max(1400, 40 * tokens);
-      const long long clocks = ctas <= SMS ? per * block + 4000 : (ctas + together * SMS - 1) / (together * SMS) * (per * block * together + 4000);
+      if (only_cuts ? c != only_cuts : c > 1 && (tiles * c > 2 * SMS || 2 * c > k_blocks)) continue;
+      const long long per = (k_blocks + c - 1) / c, ctas = tiles * c, ends = c > 1 ? 5500 : 4000;
+      const long long clocks = ctas <= SMS ? per * (std::max(1400, 20 * tokens) + (tokens > 16 ? 600 : 0)) + ends
+                                           : (ctas + 2 * SMS - 1) / (2 * SMS) * 2 * (per * std::max(t == 1 ? 1400 : 0, 20 * tokens) + ends);
       if (clocks < best) best = clocks, *bn = tokens, *t_tiles = t, *cuts = c;
     }
-    if (M <= 16 * t) break;
   }
 }
 
@@ -560,8 +558,8 @@ extern "C" int llm_gemm_digits(const void* digits, const int* a_exp, const long 
   choose_tiles(M, n_tiles, p.k_blocks, cuts, &p.bn, &p.t_tiles, &cuts);
   LLM_REQUIRE((long long)n_tiles * p.t_tiles * 8 < (1LL << 31), "gemm_digits: M=%d N=%d too large", M, N);
   p.per_cut = (p.k_blocks + cuts - 1) / cuts;
-  p.stages = p.bn <= 16 ? 3 : p.bn <= 64 ? 2 : 3;  // two CTAs a multiprocessor, or one
-  p.tmem_cols = p.bn <= 16 ? 64 : p.bn <= 32 ? 128 : p.bn <= 64 ? 256 : 512;
+  p.stages = p.bn <= 16 ? 3 : 2;  // two CTAs a multiprocessor
+  p.tmem_cols = p.bn <= 16 ? 64 : p.bn <= 32 ? 128 : 256;
   p.error_out = error_word();
   CUtensorMap ma;
   LLM_REQUIRE(digits_map(digits, M, p.k_blocks, p.bn, &ma), "gemm_digits: cuTensorMapEncodeTiled failed");
