@@ -533,6 +533,7 @@ void launch_one(const AttArgs& p, int n_seqs, int max_len, cudaStream_t stream) 
   static std::atomic<unsigned long long> done{0};
   constexpr int most = (SEG * 132 + SEG / 2 * 128 + ONE_ROWS * (132 + S_ROW) + ONE_SLOTS * ONE_ROWS * 132) * 4;
   static_assert(most <= 224 * 1024, "shared memory of a CTA");
+  static_assert(4 * (ONE_THREADS / 128) >= ONE_ROWS, "sets of four rows take every group");
   allow_smem(kernel, most, done);
   launch_kernel_cluster(kernel, dim3((unsigned)ctas, (unsigned)p.nkv, (unsigned)n_seqs), ONE_THREADS, smem, dim3((unsigned)ctas), stream, p);
 }
@@ -545,6 +546,7 @@ void launch_rows(AttArgs p, int n_seqs, int max_rows, cudaStream_t stream) {
   static std::atomic<unsigned long long> done{0};
   constexpr int most = (2 * KT * (64 * DC + 4) + ROWS * (64 * DC + 4 + S_ROW)) * 4;
   static_assert(most <= 224 * 1024, "shared memory of a CTA");
+  static_assert(4 * (ONE_THREADS / 128) >= ONE_ROWS, "sets of four rows take every group");
   allow_smem(kernel, most, done);
   launch_kernel(kernel, dim3((unsigned)p.row_tiles * (unsigned)n_seqs, p.nkv * (p.scratch != nullptr ? p.n_seg : 1)), (KT / KM) * (ROWS / RM), smem, stream, p);
 }
@@ -600,7 +602,8 @@ extern "C" int llm_paged_attention_simt(const void* q, long long ld_q, const voi
   if (dtype == LLM_F32 && at % 16 == 0 && ld_q % 4 == 0 && one_token(n_seqs, max_new, max_len, nq, nkv, hd)) {
     const AttArgs p{q, kcache, vcache, out, seq_start, seq_ntok, seq_qoff, block_table, nullptr, ld_q, ld_out,
                     max_blocks, nq, nkv, hd, page_size, window, 1, 0, scale};
-    const int group = nq / nkv, rm = group <= 2 ? 0 : group <= 4 ? 1 : 2, no = group == 1 ? 0 : 2 * ONE_THREADS >= group * hd ? 1 : 2;
+    // a row's sums take hd whole threads: ONE_THREADS / hd sets of them, one, two or four rows each (four always suffice: hd <= 128)
+    const int group = nq / nkv, sets = ONE_THREADS / hd, rm = group <= 2 ? 0 : group <= 4 ? 1 : 2, no = group == 1 ? 0 : 2 * sets >= group ? 1 : 2;
     constexpr void (*const forms[3][3])(const AttArgs&, int, int, cudaStream_t) = {{launch_one<1, 1>, launch_one<1, 2>, launch_one<1, 4>},
                                                                                    {launch_one<2, 1>, launch_one<2, 2>, launch_one<2, 4>},
                                                                                    {launch_one<4, 1>, launch_one<4, 2>, launch_one<4, 4>}};

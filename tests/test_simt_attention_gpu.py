@@ -147,3 +147,24 @@ def test_single_tokens_behind_many_segments(ops, nq, nkv, hd, page, window, leng
         K, V = dense[i]
         ref = _attention_ref(rows[i].view(nq, hd).cpu().double(), K.double(), V.double(), n - 1, nq, nkv, hd, 0.2, window)
         torch.testing.assert_close(out[i].cpu(), ref.float(), rtol=2e-5, atol=2e-5)
+
+
+@pytest.mark.parametrize("group", range(1, 9))
+def test_single_tokens_with_every_head_size(ops, group):
+    """Every head size that single tokens' kernel takes, whole sets of threads or not (5 heads of 96 numbers are 480 sums of 512, yet two
+    sets of 96 threads with two rows each have four): bit-equal to the last token of a portion of two, and near float64."""
+    lengths = (1, 64, 300)
+    for hd in range(4, 129, 4):
+        kc, vc, table, dense = _paged_setup(torch.float32, 1, hd, 16, list(lengths), sum(-(-n // 16) for n in lengths) + 2, seed=hd)
+        q = torch.randn(len(lengths), 2, group * hd, generator=torch.Generator().manual_seed(13)).to(DEV)
+        rows = q[:, -1].contiguous()
+        out = torch.full_like(rows, float("nan"))
+        ops.paged_attention(rows, kc, vc, Batch([(n - 1, 1) for n in lengths]), table, out, group, 1, hd, 0.2)
+        for i, n in enumerate(lengths):
+            if n > 1:
+                portion = torch.empty(2, group * hd, device=DEV)
+                ops.paged_attention(q[i].contiguous(), kc, vc, Batch([(n - 2, 2)]), table[i:i + 1].contiguous(), portion, group, 1, hd, 0.2)
+                assert torch.equal(portion[-1], out[i]), (hd, n)
+            K, V = dense[i]
+            ref = _attention_ref(rows[i].view(group, hd).cpu().double(), K.double(), V.double(), n - 1, group, 1, hd, 0.2, 0)
+            torch.testing.assert_close(out[i].cpu(), ref.float(), rtol=2e-5, atol=2e-5)
