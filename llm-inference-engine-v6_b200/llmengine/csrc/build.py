@@ -36,10 +36,10 @@ NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-lineinfo", 
 CXX_FLAGS = ["-O2", "-std=c++17", "-fPIC", "-fvisibility=hidden", "-Wall", "-Wextra", "-Wno-unused-parameter"]
 
 # name -> CUDA sources. "core" is what every model and precision needs; "tensorcore" holds the
-# tcgen05/TMA kernels: the bfloat16 path and the larger float32 products.
+# tcgen05/TMA kernels that only the bfloat16 path uses.
 KERNEL_LIBRARIES: Dict[str, List[str]] = {
     "core": ["status.cu", "elementwise.cu", "gemm_simt.cu", "rope_kv.cu", "attention_simt.cu", "latent.cu", "routed.cu", "gated_attention.cu", "selective_scan.cu", "linear_state.cu", "sampling.cu"],
-    "tensorcore": ["status.cu", "gemm_tc.cu", "gemm_decode.cu", "gemm_digits.cu", "attention_mma.cu", "attention_tc.cu", "attention_decode.cu", "latent_mma.cu", "routed_mma.cu", "routed_tc.cu"],
+    "tensorcore": ["status.cu", "gemm_tc.cu", "gemm_decode.cu", "attention_mma.cu", "attention_tc.cu", "attention_decode.cu", "latent_mma.cu", "routed_mma.cu", "routed_tc.cu"],
 }
 HOST_SOURCES = ["cache_manager.cpp", "scheduler.cpp", "bindings.cpp"]
 REF_DIR = os.path.join(HERE, "ref")

@@ -6,9 +6,7 @@
 // inv_rms = 1/sqrt(sum(x^2)/dim + eps)), silu_f32 (src/kernels.cpp:26-31: v/(1+exp(-v))) with the
 // product by `up` as a separate multiply (src/engine.cpp:388-389), embed_lookup_f32
 // (src/kernels.cpp:59-66).
-#include "digits.cuh"
-
-#include <type_traits>
+#include "common.cuh"
 
 // ------------------------------------------------------------------------------------ embedding
 // sumsq (may be null): sumsq[row] = sum of the squares of the row, for a norm that is folded into
@@ -127,13 +125,12 @@ __device__ __forceinline__ void store4<bf16>(bf16* dst, float a, float b, float 
   *reinterpret_cast<uint2*>(dst) = v;
 }
 
-// dim % 4 == 0 and dim <= 4 * R * blockDim: the row stays in registers between the two passes. With DIGITS the row is written as digits too
-// (digits.cuh; a kernel of its own behind this one: 2 us).
-template <typename TOut, int R, bool DIGITS = false>
+// dim % 4 == 0 and dim <= 4 * R * blockDim: the row stays in registers between the two passes.
+template <typename TOut, int R>
 __global__ void __launch_bounds__(1024) rmsnorm_vec_kernel(float* __restrict__ h, const float* __restrict__ delta, int n_partials,
                                                            size_t partial_stride, const float* __restrict__ w,
                                                            const int* __restrict__ rows, TOut* __restrict__ out, int dim,
-                                                           float eps, int write_back, int center, const DigitRows to) {
+                                                           float eps, int write_back, int center) {
   __shared__ float red[33];
   dep_launch();
   float4 wv[R];
@@ -212,14 +209,8 @@ __global__ void __launch_bounds__(1024) rmsnorm_vec_kernel(float* __restrict__ h
 #pragma unroll
   for (int k = 0; k < R; ++k) {
     const int i = (threadIdx.x + k * blockDim.x) * 4;
-    if (DIGITS) x[k] = make_float4((wv[k].x * x[k].x) * inv, (wv[k].y * x[k].y) * inv, (wv[k].z * x[k].z) * inv, (wv[k].w * x[k].w) * inv);
-    if (i < dim) {
-      if (DIGITS) store4<TOut>(o + i, x[k].x, x[k].y, x[k].z, x[k].w);
-      else store4<TOut>(o + i, (wv[k].x * x[k].x) * inv, (wv[k].y * x[k].y) * inv, (wv[k].z * x[k].z) * inv, (wv[k].w * x[k].w) * inv);
-    }
-  }
-  if constexpr (DIGITS) {
-    put_digit_row(x, dim, blockIdx.x, to);
+    if (i < dim)
+      store4<TOut>(o + i, (wv[k].x * x[k].x) * inv, (wv[k].y * x[k].y) * inv, (wv[k].z * x[k].z) * inv, (wv[k].w * x[k].w) * inv);
   }
 }
 
@@ -269,7 +260,7 @@ __global__ void rmsnorm_kernel(float* __restrict__ h, const float* __restrict__ 
 
 template <typename TOut>
 static void launch_rmsnorm(float* h, const float* delta, int n_partials, size_t partial_stride, const float* w, const int* rows,
-                           TOut* out, int n_out_rows, int dim, float eps, int write_back, int center, const DigitRows& to, cudaStream_t stream) {
+                           TOut* out, int n_out_rows, int dim, float eps, int write_back, int center, cudaStream_t stream) {
   auto al = [](const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; };
   const bool vec = dim % 4 == 0 && dim <= 16384 && al(h) && al(w) && al(out) && (!delta || (al(delta) && partial_stride % 4 == 0));
   if (vec) {
@@ -279,19 +270,12 @@ static void launch_rmsnorm(float* h, const float* delta, int n_partials, size_t 
     // launch is resident at once and all of its bytes are on their way together.
     if (n_out_rows >= 512 && quads >= 256 && quads <= 4096) threads = ((quads / 4 + 31) / 32) * 32;
     const int per_thread = (quads + threads - 1) / threads;
-    auto launch_vec = [&](auto r) {
-      constexpr int R = decltype(r)::value;
-      auto kernel = rmsnorm_vec_kernel<TOut, R>;
-      if constexpr (std::is_same<TOut, float>::value)
-        if (to.digits) kernel = rmsnorm_vec_kernel<TOut, R, true>;
-      launch_kernel(kernel, n_out_rows, threads, 0, stream, h, delta, n_partials, partial_stride, w, rows, out, dim, eps, write_back, center, to);
-    };
     if (per_thread == 1)
-      launch_vec(std::integral_constant<int, 1>());
+      launch_kernel(rmsnorm_vec_kernel<TOut, 1>, n_out_rows, threads, 0, stream, h, delta, n_partials, partial_stride, w, rows, out, dim, eps, write_back, center);
     else if (per_thread == 2)
-      launch_vec(std::integral_constant<int, 2>());
+      launch_kernel(rmsnorm_vec_kernel<TOut, 2>, n_out_rows, threads, 0, stream, h, delta, n_partials, partial_stride, w, rows, out, dim, eps, write_back, center);
     else
-      launch_vec(std::integral_constant<int, 4>());
+      launch_kernel(rmsnorm_vec_kernel<TOut, 4>, n_out_rows, threads, 0, stream, h, delta, n_partials, partial_stride, w, rows, out, dim, eps, write_back, center);
     return;
   }
   int threads = 128;
@@ -299,37 +283,21 @@ static void launch_rmsnorm(float* h, const float* delta, int n_partials, size_t 
   launch_kernel(rmsnorm_kernel<TOut>, n_out_rows, threads, 0, stream, h, delta, n_partials, partial_stride, w, rows, out, dim, eps, write_back, center);
 }
 
-static int rmsnorm(float* h, const float* delta, int n_partials, long long partial_stride,
+extern "C" int llm_rmsnorm(float* h, const float* delta, int n_partials, long long partial_stride,
                            const float* w, const int* rows, void* out, int out_dtype, int n_out_rows,
-                           int dim, float eps, int write_back, int center, const DigitRows& to, cudaStream_t stream) {
+                           int dim, float eps, int write_back, int center, cudaStream_t stream) {
   if (n_out_rows == 0) return LLM_OK;
-  const uintptr_t at = reinterpret_cast<uintptr_t>(h) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(delta);
-  LLM_REQUIRE(!to.digits || (out_dtype == LLM_F32 && dim % 4 == 0 && dim <= 16384 && at % 16 == 0 && partial_stride % 4 == 0),
-              "rmsnorm: rows of %d numbers, or rows that do not begin on 16 bytes, are not written as digits", dim);
   LLM_REQUIRE(n_out_rows > 0 && dim > 0, "rmsnorm: bad sizes rows=%d dim=%d", n_out_rows, dim);
   LLM_REQUIRE(!(rows && write_back), "rmsnorm: write_back with a row list is not allowed");
   LLM_REQUIRE(!delta || n_partials >= 1, "rmsnorm: delta needs n_partials >= 1");
   if (out_dtype == LLM_F32)
-    launch_rmsnorm<float>(h, delta, n_partials, (size_t)partial_stride, w, rows, (float*)out, n_out_rows, dim, eps, write_back, center, to, stream);
+    launch_rmsnorm<float>(h, delta, n_partials, (size_t)partial_stride, w, rows, (float*)out, n_out_rows, dim, eps, write_back, center, stream);
   else if (out_dtype == LLM_BF16)
-    launch_rmsnorm<bf16>(h, delta, n_partials, (size_t)partial_stride, w, rows, (bf16*)out, n_out_rows, dim, eps, write_back, center, to, stream);
+    launch_rmsnorm<bf16>(h, delta, n_partials, (size_t)partial_stride, w, rows, (bf16*)out, n_out_rows, dim, eps, write_back, center, stream);
   else
     LLM_REQUIRE(false, "rmsnorm: unknown out dtype %d", out_dtype);
   LLM_CHECK_LAUNCH("rmsnorm");
   return LLM_OK;
-}
-
-extern "C" int llm_rmsnorm(float* h, const float* delta, int n_partials, long long partial_stride, const float* w, const int* rows, void* out,
-                           int out_dtype, int n_out_rows, int dim, float eps, int write_back, int center, cudaStream_t stream) {
-  return rmsnorm(h, delta, n_partials, partial_stride, w, rows, out, out_dtype, n_out_rows, dim, eps, write_back, center, DigitRows{}, stream);
-}
-
-// The same of float32 rows, written as digits too.
-extern "C" int llm_rmsnorm_digits(float* h, const float* delta, int n_partials, long long partial_stride, const float* w, const int* rows, float* out,
-                                  int n_out_rows, int dim, float eps, int write_back, int center, void* digits, int* exps, long long* sums,
-                                  cudaStream_t stream) {
-  return rmsnorm(h, delta, n_partials, partial_stride, w, rows, out, LLM_F32, n_out_rows, dim, eps, write_back, center,
-                 DigitRows{(uint8_t*)digits, exps, sums}, stream);
 }
 
 // ------------------------------------------------------------------------------------ residual add
@@ -379,46 +347,6 @@ __global__ void silu_mul_kernel(const T* __restrict__ in, T* __restrict__ out, i
   const float g = to_f32(in[r * 2 * ff + gc]);
   const float u = to_f32(in[r * 2 * ff + uc]);
   out[i] = from_f32<T>(gated_value(g, u, act, p0, p1));
-}
-
-// The same of float32 rows [gate | up], written as digits too for the product behind (digits.cuh): a block a row, ff <= 4 * R * blockDim. In
-// place of the kernel above and one that makes the digits: 8,192 columns, 1 to 8 rows: 2.9 us, not 1.9 and 2.8.
-template <int R>
-__global__ void __launch_bounds__(1024) silu_mul_digits_kernel(const float* __restrict__ in, float* __restrict__ out, int ff, int act, float p0,
-                                                               float p1, const DigitRows to) {
-  dep_launch();
-  dep_wait();
-  const float* gate = in + (size_t)blockIdx.x * 2 * ff;
-  float4 g[R], x[R];
-#pragma unroll
-  for (int k = 0; k < R; ++k) {
-    const int i = (threadIdx.x + k * blockDim.x) * 4;
-    g[k] = i < ff ? *reinterpret_cast<const float4*>(gate + i) : make_float4(0.f, 0.f, 0.f, 0.f);
-    x[k] = i < ff ? *reinterpret_cast<const float4*>(gate + ff + i) : make_float4(0.f, 0.f, 0.f, 0.f);
-  }
-#pragma unroll
-  for (int k = 0; k < R; ++k) {
-    const int i = (threadIdx.x + k * blockDim.x) * 4;
-    x[k] = make_float4(gated_value(g[k].x, x[k].x, act, p0, p1), gated_value(g[k].y, x[k].y, act, p0, p1), gated_value(g[k].z, x[k].z, act, p0, p1),
-                       gated_value(g[k].w, x[k].w, act, p0, p1));
-    if (i < ff) *reinterpret_cast<float4*>(out + (size_t)blockIdx.x * ff + i) = x[k];
-  }
-  put_digit_row(x, ff, blockIdx.x, to);
-}
-
-// in [n_rows, 2 * ff], out [n_rows, ff] float32, all of them and their rows on 16 bytes, ff at most 16,384
-extern "C" int llm_silu_mul_digits(const float* in, float* out, int n_rows, int ff, int act, float p0, float p1, void* digits, int* exps,
-                                   long long* sums, cudaStream_t stream) {
-  if (n_rows == 0) return LLM_OK;
-  LLM_REQUIRE(n_rows > 0 && ff > 0 && ff % 4 == 0 && ff <= 16384 && (reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out)) % 16 == 0,
-              "silu_mul_digits: rows=%d ff=%d not taken", n_rows, ff);
-  LLM_REQUIRE(act >= 0 && act <= 2, "silu_mul_digits: unknown activation %d", act);
-  const DigitRows to{(uint8_t*)digits, exps, sums};
-  const int quads = ff / 4, threads = quads <= 1024 ? (quads + 31) / 32 * 32 : 1024, per_thread = (quads + threads - 1) / threads;
-  auto kernel = per_thread == 1 ? silu_mul_digits_kernel<1> : per_thread == 2 ? silu_mul_digits_kernel<2> : silu_mul_digits_kernel<4>;
-  launch_kernel(kernel, n_rows, threads, 0, stream, in, out, ff, act, p0, p1, to);
-  LLM_CHECK_LAUNCH("silu_mul_digits");
-  return LLM_OK;
 }
 
 extern "C" int llm_silu_mul(const void* in, void* out, int dtype, int n_rows, int ff, int block, int act, float p0, float p1, cudaStream_t stream) {

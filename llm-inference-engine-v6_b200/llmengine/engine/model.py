@@ -68,9 +68,6 @@ class Model:
             part.load(tensors)
         self.weight_bytes = sum(t.numel() * t.element_size() for t in tensors.values())
         self.tensor_names = sorted(tensors)
-        del tensors
-        if self.env.device.type == "cuda":
-            torch.cuda.empty_cache()  # what parts now hold in another form goes back to the device: the page pool comes next
 
     # ------------------------------------------------------------------ cache
     def kv_bytes_per_token(self) -> int:
@@ -154,8 +151,7 @@ class Model:
             if self.final_norm.can_defer and self.head.wants_lazy_norm(ctx):
                 x = self.final_norm.forward(res, ctx, rows=ctx.logit_rows, n_rows=ctx.n_rows, lazy=True)
             else:
-                extra = {"digits": True} if self.final_norm.can_write_digits and self.head.takes_digit_rows else {}
-                x = self.final_norm.forward(res, ctx, rows=ctx.logit_rows, n_rows=ctx.n_rows, **extra)
+                x = self.final_norm.forward(res, ctx, rows=ctx.logit_rows, n_rows=ctx.n_rows)
         else:
             x = ctx.ws.get("norm.rows_out", (1, self.spec.hidden_size), self.env.dtype)[:0]
         return self.head.forward(x, ctx)

@@ -48,29 +48,6 @@ class RowScale:
         return (_ptr(self.sumsq), c_int(self.sumsq.shape[1]), c_float(1.0 / self.dim), c_float(self.eps))
 
 
-class DigitWeight:
-    """A float32 weight [rows, inner] as whole numbers (CudaOps.digit_weight): tiles of digits and an exponent a row."""
-    dtype = torch.float32
-
-    def __init__(self, tiles: torch.Tensor, exps: torch.Tensor, rows: int, inner: int):
-        self.tiles, self.exps, self.shape = tiles, exps, (rows, inner)
-
-
-class DigitRows:
-    """Float32 activation rows [rows, inner] (`values`) and the same as digits, for a product with a DigitWeight: what the kernel that made
-    the rows left beside them. Good until the next rows of the workspace are written as digits: there is one place for them."""
-    dtype = torch.float32
-
-    def __init__(self, values: torch.Tensor, ws):
-        self.values, self.shape = values, values.shape
-        n, k = values.shape
-        self.digits = ws.get("digits.rows", (n, -(-k // 64) * 256), torch.uint8)
-        self.exps, self.sums = ws.get("digits.exponents", (n,), torch.int32), ws.get("digits.sums", (n,), torch.int64)
-
-    def args(self):
-        return self.digits.data_ptr(), self.exps.data_ptr(), self.sums.data_ptr()
-
-
 _NO_ROW_SCALE = (c_void_p(0), c_int(0), c_float(0.0), c_float(0.0))
 
 
@@ -106,7 +83,6 @@ _TYPES = {"p": c_void_p, "i": c_int, "q": c_longlong, "f": c_float}
 _SIGNATURES = {
     "core": {
         "llm_rmsnorm": "ppiqpppiiifiip",
-        "llm_rmsnorm_digits": "ppiqpppiifiipppp",
         "llm_rope_kv_write": "pqipiqpppipppp" + "iiiii" + "piffp",
         "llm_gemm_simt": "pppiiiqqqiip",
         "llm_silu_mul": "ppiiiiiffp",
@@ -115,9 +91,6 @@ _SIGNATURES = {
         "llm_gemm_tc": "pppiiiqqqiiiqip",
         "llm_gemm_tc_swiglu": "pppiiiqqqiffp",
         "llm_paged_attention_tc": "pqppqppppipqiiiiiifiipp",
-        "llm_row_digits": "piiqpppp",
-        "llm_gemm_digits": "pppppppiiiqqip",
-        "llm_gemm_digits_few": "pppppppiiiqqp",
     },
 }
 
@@ -269,11 +242,11 @@ class CudaOps:
 
     def rmsnorm(self, h: torch.Tensor, weight: torch.Tensor, eps: float, out: torch.Tensor,
                 delta: Optional[torch.Tensor] = None, rows: Optional[torch.Tensor] = None,
-                n_rows: Optional[int] = None, write_back: bool = True, center: bool = False, digits: Optional[DigitRows] = None) -> torch.Tensor:
+                n_rows: Optional[int] = None, write_back: bool = True, center: bool = False) -> torch.Tensor:
         """x = h[r] (+ delta[r], or + sum_p delta[p][r] for a 3-d delta); out = (w*x)/rms(x), or with `center` (a layer norm
         without bias) out = w * (x - mean(x)) / sqrt(mean((x - mean(x))^2) + eps).
         With `delta` and write_back, h[r] is replaced by x (the fused residual sum).
-        With `rows` (int32), output row i reads source row rows[i] and h is left as it is. digits: where the rows go as digits too."""
+        With `rows` (int32), output row i reads source row rows[i] and h is left as it is."""
         f32 = torch.float32
         if not (h.dtype is f32 and weight.dtype is f32 and h.is_cuda and weight.is_cuda and out.is_cuda and weight.is_contiguous()):
             _need(h, "rmsnorm.h", f32); _need(weight, "rmsnorm.weight", f32); _need(out, "rmsnorm.out")
@@ -294,10 +267,6 @@ class CudaOps:
             _need(rows, "rmsnorm.rows", torch.int32)
             write_back = False
         back = 1 if (write_back and delta is not None) else 0
-        if digits is not None:
-            self._check(lib.llm_rmsnorm_digits(_at(h), _at(delta), n_part, pstride, _at(weight), _at(rows), _at(out), n_out, dim, eps, back,
-                                               1 if center else 0, *digits.args(), _stream()), lib)
-            return out
         self._check(lib.llm_rmsnorm(h.data_ptr(), None if delta is None else delta.data_ptr(), n_part, pstride, weight.data_ptr(),
                                     None if rows is None else rows.data_ptr(), out.data_ptr(), dtype_code(out.dtype), n_out, dim, eps, back,
                                     1 if center else 0, _raw_stream()), lib)
@@ -342,19 +311,6 @@ class CudaOps:
         assert gate_up.is_contiguous() and out.is_contiguous() and gate_up.shape == (n, 2 * ff)
         self._check(lib.llm_silu_mul(_at(gate_up), _at(out), dtype_code(out.dtype), n, ff, block, *self._act_args(act), _stream()), lib)
         return out
-
-    def silu_mul_digits(self, gate_up: torch.Tensor, out: torch.Tensor, ws, act="silu"):
-        """silu_mul of float32 [gate | up] rows for a product with a DigitWeight: -> `out` with its digits (DigitRows), or `out` alone where
-        the kernel does not take the sizes."""
-        n, ff = out.shape
-        if n == 0 or ff % 4 or ff > 16384:
-            return self.silu_mul(gate_up, out, act=act)
-        _need(gate_up, "silu_mul.in", torch.float32); _need(out, "silu_mul.out", torch.float32)
-        assert gate_up.is_contiguous() and out.is_contiguous() and gate_up.shape == (n, 2 * ff)
-        rows, lib = DigitRows(out, ws), self.lib()
-        self._check(lib.llm_silu_mul_digits(_ptr(gate_up), _ptr(out), c_int(n), c_int(ff), *self._act_args(act), *(c_void_p(x) for x in rows.args()),
-                                            _stream()), lib)
-        return rows
 
     EPILOGUE_ACTIVATIONS = ("silu", "gelu_tanh", "clamped_swish")  # what the gate|up product applies in its own epilogue (gemm_swiglu)
 
@@ -472,86 +428,19 @@ class CudaOps:
         self._check(lib.llm_gemm_tc(at, wt, out.data_ptr(), M, N, K, lda, ldw, ldo, dtype_code(out.dtype), swap, splits, split_stride, stages,
                                     _raw_stream()), lib)
 
-    # Float32 matrices of at least so many numbers, with rows of at least so many, are held as digits. With shorter rows a few rows of
-    # activations are faster on CUDA cores (digits, those of the activations made, against CUDA cores, us: 2,048 outputs of 512 inputs 1
-    # row 4.5 and 2.3, 16 rows 9.9 and 4.8, 300 rows 23 and 37; of 1,024 inputs 4.5 and 3.3, 11.3 and 8.0, 28 and 64; of 2,048 inputs
-    # 5.9 and 5.0, 8 rows 6.3 and 7.9, 16 rows 13 and 12, 300 rows 36 and 119), and which way a weight goes must not depend on the rows.
-    DIGITS_MIN_NUMBERS, DIGITS_MIN_K = 1 << 21, 2048
-
-    def digit_weight(self, w: torch.Tensor) -> Optional[DigitWeight]:
-        """A float32 weight [N, K] as digits (csrc/kernels/gemm_digits.cu), for gemm and gemm_partials to take in its place; None for one
-        that stays as it is: of another type, small, with a row that does not fit the form (infinities, NaN, all of it below
-        2^-90), or where memory is short. Made once, when the weight is loaded (waits for the device); the caller may let go of `w`."""
-        if w.dtype != torch.float32 or not w.is_cuda or not self.tensor_cores or w.dim() != 2 or w.stride(1) != 1:
-            return None
-        n, k = w.shape
-        if n * k < self.DIGITS_MIN_NUMBERS or k < self.DIGITS_MIN_K:
-            return None
-        lib = self.lib("tensorcore")
-        if not lib.llm_weight_digits_supported(c_int(n), c_int(k)):
-            return None
-        size = -(-n // 128) * -(-k // 64) * 32768
-        free = torch.cuda.mem_get_info(w.device)[0] + torch.cuda.memory_reserved(w.device) - torch.cuda.memory_allocated(w.device)
-        if 4 * size > free:
-            return None
-        tiles = torch.empty(size, dtype=torch.uint8, device=w.device)
-        exps = torch.empty(n, dtype=torch.int32, device=w.device)
-        self._check(lib.llm_weight_digits(_ptr(w), c_int(n), c_int(k), c_longlong(w.stride(0)), _ptr(tiles), _ptr(exps), _stream()), lib)
-        if bool((exps >= 0x7ffffffe).any()):  # (waits: products read a weight ahead of what the stream is still running)
-            return None
-        return DigitWeight(tiles, exps, n, k)
-
-    def row_digits(self, a: torch.Tensor, ws) -> DigitRows:
-        """Float32 rows as digits."""
-        rows = DigitRows(a, ws)
-        m, k = a.shape
-        lib = self.lib("tensorcore")
-        self._check(lib.llm_row_digits(a.data_ptr(), m, k, k if a.is_contiguous() else a.stride(0), *rows.args(), _stream()), lib)
-        return rows
-
-    def digit_rows(self, out: torch.Tensor, ws, weight: torch.Tensor) -> Optional[DigitRows]:
-        """Where a norm's kernel may leave its float32 rows `out` as digits too; None for rows that it does not."""
-        if out.dtype != torch.float32 or out.shape[1] % 4 or out.shape[1] > 16384 or weight.data_ptr() % 16:
-            return None
-        return DigitRows(out, ws)
-
-    DIGITS_FEW_ROWS = 8  # up to here on mma.sync, straight from memory; beyond on tcgen05
-
-    def _gemm_digits(self, a: DigitRows, w: DigitWeight, out: torch.Tensor, cuts: int = 0) -> None:
-        M, K = a.shape
-        lib = self.lib("tensorcore")
-        x = a.values
-        lda = K if x.is_contiguous() else x.stride(0)
-        common = (*a.args(), x.data_ptr(), w.tiles.data_ptr(), w.exps.data_ptr(), out.data_ptr(), M, w.shape[0], K, lda, out.stride(0))
-        if M <= self.DIGITS_FEW_ROWS and cuts == 0:
-            self._check(lib.llm_gemm_digits_few(*common, _stream()), lib)
-        else:
-            self._check(lib.llm_gemm_digits(*common, cuts, _stream()), lib)
-
-    def gemm(self, a, w, out: torch.Tensor, ws=None) -> torch.Tensor:
+    def gemm(self, a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, ws=None) -> torch.Tensor:
         """out[m,n] = sum_k a[m,k]*w[n,k]; float32 accumulation; a and w of one dtype; out float32
         or that dtype. Rows may be strided views. bfloat16 runs on the tensor cores (with a
         workspace `ws`: cut along K and reduced where the output's tiles leave multiprocessors idle,
         see _form); float32 on CUDA cores, every output element summed over k in an order that K
-        alone decides, whatever the batch, or with a DigitWeight in place of `w` (and DigitRows in place
-        of `a`, else they are made in `ws`) in exact whole numbers, whose sums no order changes.
+        alone decides, whatever the batch.
         `w` is a weight: the kernels begin to read it before the kernels launched ahead of them on the
         stream are done (`a` not). A `w` that one of this object's own kernels has just written needs a
         synchronization in between; one that torch has written does not."""
+        _need(a, "gemm.a"); _need(w, "gemm.w", a.dtype); _need(out, "gemm.out")
         M, K = a.shape
         N = w.shape[0]
         assert w.shape[1] == K and out.shape == (M, N)
-        if isinstance(w, DigitWeight):
-            _need(out, "gemm.out", torch.float32)
-            if not isinstance(a, DigitRows):
-                _need(a, "gemm.a", torch.float32)
-                if M == 0:
-                    return out
-                assert ws is not None, "a product of digits needs a workspace for its rows"
-                a = self.row_digits(a, ws)
-            self._gemm_digits(a, w, out)
-            return out
-        _need(a, "gemm.a"); _need(w, "gemm.w", a.dtype); _need(out, "gemm.out")
         operands = self._tc_operands(a, w)
         if operands is not None:
             form = self._form(M, N, K, ws is not None and out.is_contiguous(), True)
@@ -605,28 +494,25 @@ class CudaOps:
         self._gemm_tc(operands, parts, form, M * N)
         return parts
 
-    def gemm_cut_partials(self, a, w, ws, tag: str) -> Optional[torch.Tensor]:
+    def gemm_cut_partials(self, a: torch.Tensor, w: torch.Tensor, ws, tag: str) -> Optional[torch.Tensor]:
         """gemm_partials where it cuts K for these operands, so that a consumer that adds the parts saves the kernel that would; else None,
         with nothing done."""
-        if isinstance(w, DigitWeight):
-            return None
         _need(a, "gemm.a"); _need(w, "gemm.w", a.dtype)
         return self._tc_partials(a, w, ws, tag, True)
 
-    def gemm_partials(self, a, w, ws, tag: str) -> torch.Tensor:
+    def gemm_partials(self, a: torch.Tensor, w: torch.Tensor, ws, tag: str) -> torch.Tensor:
         """As gemm, for consumers that add partial sums themselves: returns float32 [parts, M, N]
         (scratch `tag` of workspace `ws`); the product is the sum over parts, to be taken in index
         order. parts is 1 in float32 and where K is not cut (_form): the rule asks how many CTAs the
-        output's tiles give, so a product of many tokens with few outputs is cut too. a, w: as in gemm."""
-        if not isinstance(w, DigitWeight):
-            _need(a, "gemm.a"); _need(w, "gemm.w", a.dtype)
+        output's tiles give, so a product of many tokens with few outputs is cut too. w: as in gemm."""
+        _need(a, "gemm.a"); _need(w, "gemm.w", a.dtype)
         parts = self._tc_partials(a, w, ws, tag, False)
         if parts is not None:
             return parts
         M, N = a.shape[0], w.shape[0]
         assert w.shape[1] == a.shape[1]
         parts = ws.get(tag, (1, M, N), torch.float32)
-        self.gemm(a, w, parts[0], ws)
+        self.gemm(a, w, parts[0])
         return parts
 
     def can_add_into(self, a: torch.Tensor, w: torch.Tensor) -> bool:

@@ -13,7 +13,7 @@ from typing import List, Optional
 
 import torch
 
-from .base import KVNeed, LayerCache, Mixer, NormalizedRows, product_weight
+from .base import KVNeed, LayerCache, Mixer, NormalizedRows
 from .registry import build_part, part_class, register_part
 from .spec import AttentionSpec, TensorNeed
 
@@ -58,9 +58,8 @@ class PagedAttention(Mixer):
 
     def load(self, tensors) -> None:
         s = self.spec
-        self.w_qkv = product_weight(self.env, torch.cat([tensors[s.q_weight], tensors[s.k_weight], tensors[s.v_weight]], dim=0).contiguous())
-        self.w_o = product_weight(self.env, tensors[s.o_weight])
-        self.takes_digit_rows = not isinstance(self.w_qkv, torch.Tensor)
+        self.w_qkv = torch.cat([tensors[s.q_weight], tensors[s.k_weight], tensors[s.v_weight]], dim=0).contiguous()
+        self.w_o = tensors[s.o_weight]
         self.position.load(tensors)
 
     def _few_tokens(self, ctx) -> bool:

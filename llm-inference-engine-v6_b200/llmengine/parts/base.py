@@ -110,18 +110,6 @@ class NormalizedRows:
         return ops.row_scale(self.sumsq, self.h.shape[1], self.eps)
 
 
-def product_weight(env: "BuildEnv", w: torch.Tensor):
-    """A weight that only products read, as the kernels take it: float32 ones of some size as digits (ops.digit_weight), others as they are."""
-    made = env.ops.digit_weight(w) if hasattr(env.ops, "digit_weight") else None
-    return w if made is None else made
-
-
-def scratch_of(ctx, w) -> tuple:
-    """The workspace, for a product whose weight is held as digits (it has scratch of its own); else nothing: with a workspace a
-    bfloat16 product may be cut along K."""
-    return () if isinstance(w, torch.Tensor) else (ctx.ws,)
-
-
 class Part:
     category = ""
     # False for a part whose forward waits for the device or sizes its work from device data (a
@@ -141,10 +129,6 @@ class Part:
     def wants_lazy_norm(self, ctx) -> bool:
         """True if, in this step, the part takes NormalizedRows in place of normalised activations."""
         return False
-
-    # True if the part's first product takes rows with their digits (ops.DigitRows) in place of normalised activations: its weight
-    # is held as digits (product_weight).
-    takes_digit_rows = False
 
     def kernel_notes(self) -> List[str]:
         """One line for each thing a user should know about how this part will run at the engine's
@@ -192,7 +176,6 @@ class Head(Part):
 class Norm(Part):
     category = "norm"
     can_defer = False  # True: forward(..., lazy=True) may return NormalizedRows
-    can_write_digits = False  # True: forward(..., digits=True) may return the rows with their digits (ops.DigitRows)
 
     def prescale_weight(self) -> Optional[torch.Tensor]:
         """For a norm of the form (weight * x) * s(x) with s a scalar per row that only needs the row's

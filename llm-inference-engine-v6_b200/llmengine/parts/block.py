@@ -61,8 +61,6 @@ class PreNormBlock(Block):
     def _norm(norm, consumer, res: Residual, ctx):
         if norm.can_defer and consumer.wants_lazy_norm(ctx):
             return norm.forward(res, ctx, lazy=True)
-        if consumer.takes_digit_rows and norm.can_write_digits:
-            return norm.forward(res, ctx, digits=True)
         return norm.forward(res, ctx)
 
 

@@ -12,7 +12,7 @@ from typing import List
 
 import torch
 
-from .base import Embedding, Head, NormalizedRows, StateNeed, product_weight, scratch_of
+from .base import Embedding, Head, NormalizedRows, StateNeed
 from .registry import build_part, part_class, register_part
 from .spec import EmbeddingSpec, HeadSpec, TensorNeed
 
@@ -132,8 +132,7 @@ class LinearHead(Head):
         return [TensorNeed(spec.weight, (spec.vocab_size, spec.dim), "compute")]
 
     def load(self, tensors) -> None:
-        self.weight = product_weight(self.env, tensors[self.spec.weight])
-        self.takes_digit_rows = not isinstance(self.weight, torch.Tensor)
+        self.weight = tensors[self.spec.weight]
 
     def wants_lazy_norm(self, ctx) -> bool:
         # every request of the step brings one token and wants its logits: the wanted rows are all rows, in order
@@ -154,7 +153,7 @@ class LinearHead(Head):
             else:
                 x = x.dense(ctx)
         if n and not done:
-            self.env.ops.gemm(x, self.weight, logits, *scratch_of(ctx, self.weight))
+            self.env.ops.gemm(x, self.weight, logits)
         if n and cap > 0.0:
             self.env.ops.softcap(logits, cap)  # logits <- cap * tanh(logits / cap), float32
         return logits

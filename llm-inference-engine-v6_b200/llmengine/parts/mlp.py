@@ -10,7 +10,7 @@ from typing import List, Optional
 import torch
 
 from .attention import add_into_stream_or_partials, res_sumsq_off
-from .base import FeedForward, NormalizedRows, product_weight, scratch_of
+from .base import FeedForward, NormalizedRows
 from .registry import register_part
 from .spec import GatedMLPSpec, TensorNeed
 
@@ -53,9 +53,8 @@ class GatedMLP(FeedForward):
         if self.blocked:
             self.w_gate_up = torch.stack([g.view(-1, 128, s.hidden), u.view(-1, 128, s.hidden)], dim=1).reshape(2 * s.intermediate, s.hidden).contiguous()
         else:
-            self.w_gate_up = product_weight(self.env, torch.cat([g, u], dim=0).contiguous())
-        self.w_down = product_weight(self.env, tensors[s.down_weight])
-        self.takes_digit_rows = not isinstance(self.w_gate_up, torch.Tensor)
+            self.w_gate_up = torch.cat([g, u], dim=0).contiguous()
+        self.w_down = tensors[s.down_weight]
 
     def _few_tokens(self, ctx) -> bool:
         s, ops, n = self.spec, self.env.ops, ctx.n_tokens
@@ -95,15 +94,11 @@ class GatedMLP(FeedForward):
             x = x[:n]
         if self.blocked:
             ops.gemm_swiglu(x, self.w_gate_up, act, ctx.ws, **extra)
-        elif not isinstance(self.w_down, torch.Tensor):  # the down product takes digits
-            gate_up = ctx.ws.get("mlp.gate_up", (n, 2 * s.intermediate), self.env.dtype)
-            ops.gemm(x, self.w_gate_up, gate_up, *scratch_of(ctx, self.w_gate_up))
-            act = ops.silu_mul_digits(gate_up, act, ctx.ws, self.act)
         elif n <= 64:  # few tokens: the products may come as partial sums, added by their consumers
             ops.silu_mul_partials(ops.gemm_partials(x, self.w_gate_up, ctx.ws, "mlp.gate_up_parts"), act, **extra)
         else:
             gate_up = ctx.ws.get("mlp.gate_up", (n, 2 * s.intermediate), self.env.dtype)
-            ops.gemm(x, self.w_gate_up, gate_up, *scratch_of(ctx, self.w_gate_up))
+            ops.gemm(x, self.w_gate_up, gate_up)
             ops.silu_mul(gate_up, act, **({"act": self.act} if s.activation != "silu" else {}))
         return add_into_stream_or_partials(ops, act, self.w_down, ctx, False, "mlp.delta")
 

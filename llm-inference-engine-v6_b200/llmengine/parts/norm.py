@@ -30,7 +30,7 @@ class RMSNorm(Norm):
 
     can_defer = True
 
-    def forward(self, res: Residual, ctx, rows=None, n_rows=None, lazy: bool = False, digits: bool = False):
+    def forward(self, res: Residual, ctx, rows=None, n_rows=None, lazy: bool = False):
         n = ctx.n_tokens if rows is None else (rows.numel() if n_rows is None else n_rows)
         if lazy and res.pending is None and res.sumsq is not None:
             # the stream is up to date and the sums of squares of its rows are known: whoever
@@ -38,18 +38,12 @@ class RMSNorm(Norm):
             pre = res.prescaled if res.prescaled_weight is self.weight else None
             return NormalizedRows(res.h, res.sumsq, self.weight, self.spec.eps, rows, n, self, pre)
         out = ctx.ws.get("norm.out" if rows is None else "norm.rows_out", (n, self.spec.dim), self.env.dtype)
-        made = self.env.ops.digit_rows(out, ctx.ws, self.weight) if digits and n > 0 else None
-        if made is None:
-            self.env.ops.rmsnorm(res.h, self.weight, self.spec.eps, out, delta=res.pending, rows=rows, n_rows=n)
-        else:
-            self.env.ops.rmsnorm(res.h, self.weight, self.spec.eps, out, delta=res.pending, rows=rows, n_rows=n, digits=made)
+        self.env.ops.rmsnorm(res.h, self.weight, self.spec.eps, out, delta=res.pending, rows=rows, n_rows=n)
         if rows is None:
             if res.pending is not None:
                 res.sumsq = res.prescaled = res.prescaled_weight = res.operand = None  # the stream has moved on
             res.pending = None
-        return out if made is None else made
-
-    can_write_digits = True
+        return out
 
     def prescale_weight(self):
         return self.weight
@@ -79,7 +73,7 @@ class LayerNorm(RMSNorm):
     """y = (x - mean) / sqrt(variance + eps) * w with the variance as the mean of the squared deviations, a weight and no bias.
     The norm kernel with its centring switched on: the fused residual sum and the row list work as for RMSNorm. It is not of the
     form weight * x * s(row), so it neither defers nor lets a producer prescale."""
-    can_defer = can_write_digits = False
+    can_defer = False
 
     def forward(self, res: Residual, ctx, rows=None, n_rows=None, lazy: bool = False):
         n = ctx.n_tokens if rows is None else (rows.numel() if n_rows is None else n_rows)
