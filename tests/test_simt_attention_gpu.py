@@ -168,3 +168,11 @@ def test_single_tokens_with_every_head_size(ops, group):
             K, V = dense[i]
             ref = _attention_ref(rows[i].view(group, hd).cpu().double(), K.double(), V.double(), n - 1, group, 1, hd, 0.2, 0)
             torch.testing.assert_close(out[i].cpu(), ref.float(), rtol=2e-5, atol=2e-5)
+
+
+@pytest.mark.parametrize("dt", [torch.float32, torch.bfloat16])
+def test_four_tiles_of_few_rows_a_multiprocessor(ops, dt):
+    """The steps of single tokens that walk their contexts, 512 CTAs say, are one round of four a multiprocessor, or two of three: what the
+    compiler gives the kernel (64 registers a thread) decides, and that changes with what else is in its file."""
+    from llmengine.ops import dtype_code
+    assert ops.lib().llm_paged_attention_simt_resident(dtype_code(dt)) >= 4
