@@ -874,9 +874,8 @@ class CudaOps:
         n_tokens = batch.n_tokens
         if dtype is torch.bfloat16 and self.tensor_cores:
             lib = self.lib("tensorcore")
-            ld_q, (out_rows, ld_out), blocks = q.stride(0), out.shape, block_table.shape[1]
-            if not out.is_contiguous():
-                ld_out = out.stride(0)
+            ld_q, out_shape, blocks = q.stride(0), out.shape, block_table.shape[1]
+            ld_out = out_shape[1] if len(out_shape) == 2 and out.is_contiguous() else out.stride(0)
             if (self.tcgen05_attention and batch.max_new_tokens >= self.TC_ATTENTION_MIN_TOKENS and blocks <= self.TC_ATTENTION_MAX_BLOCKS and
                     self._answer(lib, "llm_attention_tc_supported", nq, nkv, hd, page, ld_q, ld_out)):
                 # prompt portions: tcgen05 kernel (128 rows per CTA, scores and output in tensor memory)

@@ -351,6 +351,20 @@ def test_paged_attention(ops, dt, nq, nkv, hd, page, window):
             torch.testing.assert_close(out[i].float().cpu(), ref, **tol(dt, 2))
 
 
+@pytest.mark.parametrize("dt", DTYPES)
+@pytest.mark.parametrize("seqs", [[(0, 1), (36, 1), (63, 1)], [(0, 1), (2, 35), (0, 64)], [(0, 1), (30, 7), (60, 4)]])
+def test_paged_attention_rows_by_head(ops, dt, seqs):
+    """Queries and outputs given as [token, head, size]: the same launch."""
+    nq, nkv, hd, page = 8, 2, 64, 16
+    kc, vc, table, _ = _paged_setup(dt, nkv, hd, page, [1, 37, 64], 11)
+    b = Batch(seqs)
+    q = rnd(b.n_tokens, nq * hd, dtype=dt, seed=21)
+    flat, by_head = torch.empty_like(q), torch.empty(b.n_tokens, nq, hd, dtype=dt, device=DEV)
+    ops.paged_attention(q, kc, vc, b, table, flat, nq, nkv, hd, 0.125)
+    ops.paged_attention(q.view(b.n_tokens, nq, hd), kc, vc, b, table, by_head, nq, nkv, hd, 0.125)
+    assert torch.equal(by_head.view_as(flat), flat)
+
+
 @pytest.mark.parametrize("hd,page", [(64, 16), (128, 16), (128, 32), (64, 64)])
 @pytest.mark.parametrize("nq,nkv,window", [(32, 8, 0), (8, 2, 0), (4, 4, 0), (16, 1, 0), (8, 2, 150), (6, 2, 0), (5, 1, 70)])
 def test_paged_attention_tcgen05(ops, nq, nkv, window, hd, page):

@@ -129,10 +129,11 @@ def test_tiles_that_are_part_empty(ops, dt, nq, nkv, hd, window, seqs):
 
 
 @pytest.mark.parametrize("nq,nkv,hd,page,window", [(4, 4, 64, 16, 0), (16, 2, 128, 16, 0), (3, 1, 20, 4, 0), (10, 2, 64, 8, 700)])
-@pytest.mark.parametrize("lengths", [(1, 1023, 1024, 1025), (2048, 2049, 5, 1500), (4096, 300, 129, 3100), (4097, 64, 2000, 1)])
+@pytest.mark.parametrize("lengths", [(1, 1023, 1024, 1025), (2048, 2049, 5, 1500), (4096, 300, 129, 3100), (4097, 64, 2000, 1),
+                                     (8191, 8192, 130, 5000), (8193, 8192, 1, 300)])
 def test_single_tokens_behind_many_segments(ops, nq, nkv, hd, page, window, lengths):
-    """Single tokens of several requests, up to 4 segments of 128 keys a CTA and beyond (where segments and a merge take over), against
-    the last token of portions of five: bit-equal, whatever the other requests' lengths."""
+    """Single tokens of several requests, clusters of 8 CTAs with one to 8 segments of 128 keys each (8,192 keys) and one key beyond (where
+    segments and a merge take over), against the last token of portions of five: bit-equal, whatever the other requests' lengths."""
     kc, vc, table, dense = _paged_setup(torch.float32, nkv, hd, page, list(lengths), sum(-(-n // page) for n in lengths) + 2, seed=hd)
     q = torch.randn(len(lengths), 5, nq * hd, generator=torch.Generator().manual_seed(12)).to(DEV)
     rows = q[:, -1].contiguous()
@@ -146,6 +147,24 @@ def test_single_tokens_behind_many_segments(ops, nq, nkv, hd, page, window, leng
             assert torch.equal(portion[-1], out[i]), n
         K, V = dense[i]
         ref = _attention_ref(rows[i].view(nq, hd).cpu().double(), K.double(), V.double(), n - 1, nq, nkv, hd, 0.2, window)
+        torch.testing.assert_close(out[i].cpu(), ref.float(), rtol=2e-5, atol=2e-5)
+
+
+@pytest.mark.parametrize("n,nkv,group,hd,most", [(80, 4, 2, 64, 1024), (80, 4, 2, 64, 1025), (64, 4, 3, 32, 2048), (150, 2, 8, 128, 1024)])
+def test_single_tokens_of_many_requests(ops, n, nkv, group, hd, most):
+    """So many requests that a cluster is one CTA or two, with up to 8 segments each (and one key beyond): bit-equal to the last token of
+    portions of two."""
+    g = torch.Generator().manual_seed(n + most)
+    lengths = [most, 2] + torch.randint(2, most + 1, (n - 2,), generator=g).tolist()
+    kc, vc, table, dense = _paged_setup(torch.float32, nkv, hd, 16, lengths, sum(-(-m // 16) for m in lengths) + 2, seed=hd)
+    q = torch.randn(n, 2, nkv * group * hd, generator=g).to(DEV)
+    out, both = torch.full_like(q[:, 0].contiguous(), float("nan")), torch.empty_like(q)
+    ops.paged_attention(q[:, 1].contiguous(), kc, vc, Batch([(m - 1, 1) for m in lengths]), table, out, nkv * group, nkv, hd, 0.2)
+    ops.paged_attention(q.view(2 * n, -1), kc, vc, Batch([(m - 2, 2) for m in lengths]), table, both.view(2 * n, -1), nkv * group, nkv, hd, 0.2)
+    assert torch.equal(out, both[:, 1])
+    for i in (0, 1, n // 2):
+        K, V = dense[i]
+        ref = _attention_ref(q[i, 1].view(nkv * group, hd).cpu().double(), K.double(), V.double(), lengths[i] - 1, nkv * group, nkv, hd, 0.2, 0)
         torch.testing.assert_close(out[i].cpu(), ref.float(), rtol=2e-5, atol=2e-5)
 
 
