@@ -12,8 +12,8 @@
 // few rows: a CTA a segment is what fills the device).
 //
 // Bound by latency with few rows, by reads of shared memory and multiply-adds with many. A layer at the Llama 3.2 1B sizes:
-// 8 single tokens behind 256 to 768 keys 17 us and 7 for the merge (a warp a token and head, a lane a key: 630 us); a prompt
-// of 300 tokens 36 us and 7 (417 us).
+// 8 single tokens behind 256 to 768 keys 17 us and 7 for the merge (a warp a token and head, a lane a key: 630 us; in float32 such steps
+// run on attention_one.cu, up to some thousand keys); a prompt of 300 tokens 36 us and 7 (417 us).
 // Only keys that some row of the tile sees are fetched and scored, so a few tokens' prompt costs what it has: 5 tokens 6.1 us, a warp a
 // token and head 6.1, all 128 keys of the segment 13.9.
 //
